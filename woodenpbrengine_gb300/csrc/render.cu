@@ -582,7 +582,7 @@ wpbr_status render_pass_launch(wpbr_ctx* ctx) {
 }
 
 uint32_t persistent_full_grid() {
-  return persistent_grid((const void*)k_trace_persistent<false, 64, CameraSrc, PrimSink>);
+  return persistent_grid((const void*)k_trace_persistent<false, 64, true, CameraSrc, PrimSink>);
 }
 
 // Everything the captured pass graph bakes into its kernel arguments: the

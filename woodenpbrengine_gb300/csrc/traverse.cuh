@@ -38,12 +38,13 @@ __device__ __forceinline__ bool second_child_first(const int neg[3], uint32_t ax
   return axis == 0 ? neg[0] != 0 : (axis == 1 ? neg[1] != 0 : (axis == 2 ? neg[2] != 0 : false));
 }
 
+template <bool SPH = true>  // false: the scene has no spheres
 __device__ __forceinline__ float prim_test(const SceneView& S, const float4* prims, uint32_t pos, V3 o, V3 d,
                                            const RayTri& R, uint32_t* prim_out, float* b1, float* b2) {
   const float4* r = prims + (size_t)pos * 3;
   float4 r0 = __ldg(r), r1 = __ldg(r + 1);
   *prim_out = __float_as_uint(r0.w);
-  if (__float_as_uint(r1.w) == 1u) {
+  if (SPH && __float_as_uint(r1.w) == 1u) {
     uint32_t s = __float_as_uint(r1.x);
     V3 rlo, rld, ph;
     float t = sphere_intersect(S.sph_w2o[s], S.sph_r[s], o, d, &rlo, &rld, &ph);

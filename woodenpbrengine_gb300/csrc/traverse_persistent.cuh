@@ -62,14 +62,15 @@ __device__ __forceinline__ RayTri unpack_ray_tri(float4 s, float4 po) {
 }
 
 // prim_test for another lane's ray: the world origin and direction are read
-// on the sphere branch only.
+// on the sphere branch only. SPH = false: the scene has no spheres.
+template <bool SPH>
 __device__ __forceinline__ float prim_test_shared(const SceneView& S, const float4* prims, uint32_t pos,
                                                   const SharedRay& sr, const RayTri& R, uint32_t* prim_out,
                                                   float* b1, float* b2) {
   const float4* r = prims + (size_t)pos * 3;
   float4 r0 = __ldg(r), r1 = __ldg(r + 1);
   *prim_out = __float_as_uint(r0.w);
-  if (__float_as_uint(r1.w) == 1u) {
+  if (SPH && __float_as_uint(r1.w) == 1u) {
     uint32_t s = __float_as_uint(r1.x);
     float4 dd = sr.d;
     // (kx, ky, kz) is a permutation of (0, 1, 2): o[kx] = R.ox, o[ky] = R.oy, o[kz] = R.oz
@@ -201,7 +202,7 @@ __device__ __forceinline__ int pop_unpruned(const Stack& st, int& sp, float tb, 
   return kEnd;
 }
 
-template <bool ANY, int STACK, class Src, class Sink>
+template <bool ANY, int STACK, bool SPH, class Src, class Sink>
 __global__ void __launch_bounds__(kPersistBlock, Sink::kMinBlocks) k_trace_persistent(SceneView S, BvhView Bv,
                                                                                            Src src, Sink sink,
                                                                     uint32_t n, uint32_t* counter, uint32_t* err) {
@@ -403,7 +404,7 @@ __global__ void __launch_bounds__(kPersistBlock, Sink::kMinBlocks) k_trace_persi
           float4 s4 = sr.s;
           RayTri R = unpack_ray_tri(s4, sr.po);
           uint32_t pos = ofirst + (g - oexcl);
-          float t = prim_test_shared(S, Bv.prims, pos, sr, R, &prim, &b1, &b2);
+          float t = prim_test_shared<SPH>(S, Bv.prims, pos, sr, R, &prim, &b1, &b2);
           if (t != 0.0f && t < s4.w) {
             key = ANY ? (((unsigned long long)pos << 32) | __float_as_uint(t))
                       : (((unsigned long long)__float_as_uint(t) << 32) | pos);
@@ -457,7 +458,7 @@ __global__ void __launch_bounds__(kPersistBlock, Sink::kMinBlocks) k_trace_persi
         RayTri R = ray_tri_setup(o, d, S.quirks);
         uint32_t prim;
         float b1, b2;
-        float tt = prim_test(S, Bv.prims, hpos, o, d, R, &prim, &b1, &b2);
+        float tt = prim_test<SPH>(S, Bv.prims, hpos, o, d, R, &prim, &b1, &b2);
         h = HitRec{tt, prim, b1, b2};
       }
       sink.store(rid, h);
@@ -562,10 +563,25 @@ inline void launch_traversal(const SceneView& S, const BvhView& Bv, const Src& s
     if (B.stack_cap > stack) B.stack_cap = stack;
     kern<<<g, kPersistBlock, 0, st>>>(S, B, src, sink, n, counter, err);
   };
+  // The collide kernels are compiled without the sphere test for scenes that
+  // have no spheres: its transform and quadratic beside the traversal's state
+  // made them spill at 64 registers (44 B; 8.4 M rays on the triangle mesh,
+  // a call: 4.165 ms with the sphere test compiled in, 3.930 without; 100,003
+  // any-hit segments on 81,920 triangles 172 -> 166 us). The render passes'
+  // scenes nearly always hold a sphere (light), so those keep one variant.
+  if constexpr (Sink::kCollide) {
+    if (S.ns == 0) {
+      if (Bv.max_depth < 60)
+        go(k_trace_persistent<ANY, 64, false, Src, Sink>, 64u);
+      else
+        go(k_trace_persistent<ANY, 256, false, Src, Sink>, 256u);
+      return;
+    }
+  }
   if (Bv.max_depth < 60)
-    go(k_trace_persistent<ANY, 64, Src, Sink>, 64u);
+    go(k_trace_persistent<ANY, 64, true, Src, Sink>, 64u);
   else
-    go(k_trace_persistent<ANY, 256, Src, Sink>, 256u);
+    go(k_trace_persistent<ANY, 256, true, Src, Sink>, 256u);
 }
 
 }  // namespace wpbr
