@@ -126,7 +126,7 @@ struct EvalCtx {
   float* smem_mat;  // block accumulators (backward only)
   float* g_env;
   float* g_func;
-  double gZ;        // this thread's share of dLoss/dZ
+  double gZ;        // this thread's share of -Z dLoss/dZ
 };
 
 __device__ __forceinline__ void add_env_taps(EvalCtx& E, const EnvView& e, float s, float t, RGB3 g) {
@@ -147,7 +147,7 @@ __device__ __forceinline__ void add_env_pdf(EvalCtx& E, const EnvView& e, int ce
   if (g_pdf == 0.0f) return;
   float f = e.cond_func[cell];
   if (f != 0.0f) atomicAdd(E.g_func + cell, g_pdf * pdf / f);
-  E.gZ += (double)g_pdf * (-(double)pdf / (double)e.marg_int);
+  E.gZ += (double)g_pdf * (double)pdf;  // times -1 / Z once per block
 }
 
 __device__ __forceinline__ void add_mat(EvalCtx& E, uint32_t mid, const MatGrad& g) {
@@ -246,8 +246,8 @@ __device__ RGB3 eval_sample(EvalCtx& E, const float4* st, const uint32_t* shadow
     if (P.S.has_env) {
       V3 d{s0.x, s0.y, s0.z};
       V3 dl = xvector(A.env_e.w2l, d);
-      float s = (float)((double)sph_phi(dl) / (2.0 * kPI));
-      float t = (float)((double)sph_theta(dl) / kPI);
+      float s = div_const(sph_phi(dl), kTwoPiDiv);
+      float t = div_const(sph_theta(dl), kPiDiv);
       L = rmul(env_bilerp(A.env_e, s, t), A.env_e.le);
       if (BACK) add_env_taps(E, A.env_e, s, t, gL);
     }
@@ -315,8 +315,8 @@ __device__ RGB3 eval_sample(EvalCtx& E, const float4* st, const uint32_t* shadow
       V3 wl = xvector(A.env_e.w2l, wiw);
       float theta = sph_theta(wl);
       float phi = sph_phi(wl);
-      eu = (float)((double)phi / (2.0 * kPI));
-      ev = (float)((double)theta / kPI);
+      eu = div_const(phi, kTwoPiDiv);
+      ev = div_const(theta, kPiDiv);
       float sth = sinf_(theta);
       li = rgb1(0.0f);
       lpdf = 0.0f;
@@ -409,7 +409,7 @@ __global__ void __launch_bounds__(kTB, WPBR_ADJ_BACK_MIN_BLOCKS) k_adj_back(Pass
   if (threadIdx.x == 0) {
     double t = 0.0;
     for (int w = 0; w < kTB / 32; ++w) t += zsum[w];
-    if (t != 0.0) atomicAdd(G.g_Z, t);
+    if (t != 0.0) atomicAdd(G.g_Z, -t / (double)A.env_e.marg_int);
   }
   for (uint32_t j = threadIdx.x; j < nm; j += blockDim.x)
     if (smem[j] != 0.0f) atomicAdd(G.g_mat + j, (double)smem[j]);

@@ -14,6 +14,7 @@
 #include <float.h>
 #include <stdint.h>
 
+#include "ffround.cuh"
 #include "wpbr_fmath.h"
 
 namespace wpbr {
@@ -21,6 +22,11 @@ namespace wpbr {
 using namespace wpbr_fm;
 
 constexpr double kPI = 3.14;                 // pch.h:30
+// the double constants the reference's expressions multiply and divide by,
+// for their float-pair forms (ffround.cuh)
+constexpr FFConst kPiMul = ff_const(kPI), kTwoPiMul = ff_const(2.0 * kPI), kTwoPiSqMul = ff_const((2.0 * kPI) * kPI);
+constexpr FFConst kLog2eMul = ff_const(1.4426950408889634);  // as log2f_ (wpbr_fmath.h) writes it
+constexpr FFRecip kPiDiv = ff_recip(kPI), kTwoPiDiv = ff_recip(2.0 * kPI);
 constexpr float kMathPi = 0x1.921fb6p+1f;    // pi inside the math library
 constexpr float kSlabScale = 0x1.000006p+0f; // 1 + 2*gamma(3) in float
 constexpr uint32_t kNoHit = 0xFFFFFFFFu;

@@ -176,25 +176,6 @@ WPBR_HD float tri_intersect_pre(V3 p0, V3 p1, V3 p2, const RayTri& R, float* b0,
   return ts * inv_det;
 }
 
-// WoodenMath getRootsQuadraticEquation, restated as pbrt-v3's Quadratic
-// (double-precision discriminant and roots, rounded to float).
-WPBR_HD bool quadratic(float a, float b, float c, float* t0, float* t1) {
-  double discrim = (double)b * (double)b - 4.0 * (double)a * (double)c;
-  if (discrim < 0.0) return false;
-  double root = sqrt_d(discrim);
-  double q = (b < 0.0f) ? -0.5 * ((double)b - root) : -0.5 * ((double)b + root);
-  float r0 = (float)(q / (double)a);
-  float r1 = (float)((double)c / q);
-  if (r0 > r1) {
-    float t = r0;
-    r0 = r1;
-    r1 = t;
-  }
-  *t0 = r0;
-  *t1 = r1;
-  return true;
-}
-
 // SSphere::intersect (WoodenPBREngine/CSSphere.cpp:84-120). Returns t
 // (0 = miss) and the object-space ray and hit point.
 WPBR_HD float sphere_intersect(const Xf& w2o, float radius, V3 ro, V3 rd, V3* rlo, V3* rld, V3* phl) {

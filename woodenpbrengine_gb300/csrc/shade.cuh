@@ -23,7 +23,7 @@ struct SurfInt {
 // CTransform::operator()(CSurfaceInteraction) (CTransform.h:41-66).
 WPBR_HD SurfInt sphere_si(const Xf& o2w, const Xf& w2o, float radius, V3 rld, V3 ph) {
   float theta = acosf_(ph.z / radius);
-  float inv_zr = (float)(1.0 / (double)sqrt_(ph.x * ph.x + ph.y * ph.y));
+  float inv_zr = 1.0f / sqrt_(ph.x * ph.x + ph.y * ph.y);  // 1.0 / a double, rounded: the same float (53 >= 2*24 + 2)
   float phi_cos = ph.x * inv_zr;
   float phi_sin = ph.y * inv_zr;
   V3 dpdu = mul(V3{-ph.y, ph.x, 0.0f}, (float)(2.0 * kPI));
@@ -179,12 +179,10 @@ WPBR_HD float fresnel_dielectric(float cos_i, float eta_i, float eta_t) {
     et = t;
     cos_i = fabs_(cos_i);
   }
-  double a = 1.0 - (double)(cos_i * cos_i);
-  float sin_i = (float)sqrt_d(0.0 > a ? 0.0 : a);
+  float sin_i = sqrt_one_minus(cos_i * cos_i);
   float sin_t = ei / et * sin_i;
-  if ((double)sin_t >= 1.0) return 1.0f;
-  double b = 1.0 - (double)(sin_t * sin_t);
-  float cos_t = (float)sqrt_d(0.0 > b ? 0.0 : b);
+  if (sin_t >= 1.0f) return 1.0f;
+  float cos_t = sqrt_one_minus(sin_t * sin_t);
   float r_parl = ((et * cos_i) - (ei * cos_t)) / ((et * cos_i) + (ei * cos_t));
   float r_perp = ((ei * cos_i) - (et * cos_t)) / ((ei * cos_i) + (et * cos_t));
   return (r_parl * r_parl + r_perp * r_perp) / 2.0f;
@@ -194,7 +192,7 @@ WPBR_HD float fresnel_conductor(float cos_i, float eta_i, float eta_t, float kk)
   float eta = eta_t / eta_i;
   float etak = kk / eta_i;
   float c2 = cos_i * cos_i;
-  float s2 = (float)(1.0 - (double)c2);
+  float s2 = 1.0f - c2;  // 1.0 - (double)c2, rounded: the same float (53 >= 2*24 + 2)
   float eta2 = eta * eta;
   float etak2 = etak * etak;
   float t0 = (eta2 - etak2) - s2;
@@ -217,12 +215,11 @@ WPBR_HD float tr_d(float ax, float ay, V3 wh) {
   float c4 = cos2t(wh) * cos2t(wh);
   float cp = cosphi(wh), sp = sinphi(wh);
   float e = ((cp * cp) / (ax * ax) + (sp * sp) / (ay * ay)) * t2;
-  double den = ((((kPI * (double)ax) * (double)ay) * (double)c4) * (double)(1.0f + e)) * (double)(1.0f + e);
-  return (float)(1.0 / den);
+  return tr_rcp(kPiMul, ax, ay, c4, 1.0f + e);
 }
 WPBR_HD V3 tr_sample(float ax, float ay, V3 wo, float u0, float u1, float* d_out) {
   float cos_t;
-  float phi = (float)((2.0 * kPI) * (double)u1);
+  float phi = mul_const(u1, kTwoPiMul);
   if (ax == ay) {
     float tan2 = ((ax * ax) * u0) / (1.0f - u0);
     cos_t = 1.0f / sqrt_(1.0f + tan2);
@@ -312,12 +309,10 @@ WPBR_HD void sphere_light_sample(const Xf& o2w, float r, V3 p, float u0, float u
   V3 wcx, wcy;
   make_basis(wc, &wcx, &wcy);
   float s2 = (r * r) / len2(sub(p, pc));
-  double a = 1.0 - (double)s2;
-  float cos_max = (float)sqrt_d(0.0 > a ? 0.0 : a);
-  float cos_t = (float)((double)u0 * (1.0 - (double)cos_max) + (double)cos_max);
-  double b = 1.0 - (double)(cos_t * cos_t);
-  float sin_t = (float)sqrt_d(0.0 > b ? 0.0 : b);
-  float phi = (float)((double)(u1 * 2.0f) * kPI);
+  float cos_max = sqrt_one_minus(s2);
+  float cos_t = lerp_to_one(u0, cos_max);
+  float sin_t = sqrt_one_minus(cos_t * cos_t);
+  float phi = mul_const(u1 * 2.0f, kPiMul);
   float dc = len(sub(p, pc));
   float q = r * r - ((dc * dc) * sin_t) * sin_t;
   float ds = dc * cos_t - sqrt_(0.0f > q ? 0.0f : q);
@@ -417,8 +412,8 @@ WPBR_HD float env_pdf_uv(const EnvView& e, float u, float v) {
 // JobLightInfiniteAreaLeCompute (CLightInfiniteArea.cpp:141-160)
 WPBR_HD RGB3 env_le(const EnvView& e, V3 d) {
   V3 dl = xvector(e.w2l, d);
-  float s = (float)((double)sph_phi(dl) / (2.0 * kPI));
-  float t = (float)((double)sph_theta(dl) / kPI);
+  float s = div_const(sph_phi(dl), kTwoPiDiv);
+  float t = div_const(sph_theta(dl), kPiDiv);
   return rmul(env_bilerp(e, s, t), e.le);
 }
 // JobLightInfiniteAreaLiSample (CLightInfiniteArea.cpp:163-204): the looked-up
@@ -432,12 +427,12 @@ WPBR_HD void env_li_sample(const EnvView& e, uint32_t quirks, float u0, float u1
   *ok = false;
   float st = 0.0f;
   if (map_pdf != 0.0f) {
-    float theta = (float)((double)uv1 * kPI);
-    float phi = (float)((double)(uv0 * 2.0f) * kPI);
+    float theta = mul_const(uv1, kPiMul);
+    float phi = mul_const(uv0 * 2.0f, kPiMul);
     float ct = cosf_(theta);
     st = sinf_(theta);
     *wi = xvector(e.l2w, sph_dir(st, ct, phi));
-    *pdf = (st != 0.0f) ? (float)((double)map_pdf / (((2.0 * kPI) * kPI) * (double)st)) : 0.0f;
+    *pdf = (st != 0.0f) ? div_by_scaled(map_pdf, kTwoPiSqMul, st) : 0.0f;
     *ok = true;
   }
   if (quirks & WPBR_Q_ENV_LI_SAMPLE_FIX) *li = rmul(env_bilerp(e, uv0, uv1), e.le);
@@ -452,13 +447,13 @@ WPBR_HD void env_li_compute(const EnvView& e, V3 wi, RGB3* li, float* pdf) {
   V3 wl = xvector(e.w2l, wi);
   float theta = sph_theta(wl);
   float phi = sph_phi(wl);
-  float u = (float)((double)phi / (2.0 * kPI));
-  float v = (float)((double)theta / kPI);
+  float u = div_const(phi, kTwoPiDiv);
+  float v = div_const(theta, kPiDiv);
   float st = sinf_(theta);
   *li = rgb1(0.0f);
   *pdf = 0.0f;
   if (st != 0.0f) {
-    *pdf = (float)((double)env_pdf_uv(e, u, v) / (((2.0 * kPI) * kPI) * (double)st));
+    *pdf = div_by_scaled(env_pdf_uv(e, u, v), kTwoPiSqMul, st);
     *li = rmul(env_bilerp(e, u, v), e.le);
   }
 }

@@ -19,8 +19,7 @@ WPBR_HD float tr_d_grad(float ax, float ay, V3 wh, float* dD_dalpha) {
   float c4 = cos2t(wh) * cos2t(wh);
   float cp = cosphi(wh), sp = sinphi(wh);
   float e = ((cp * cp) / (ax * ax) + (sp * sp) / (ay * ay)) * t2;
-  double den = ((((kPI * (double)ax) * (double)ay) * (double)c4) * (double)(1.0f + e)) * (double)(1.0f + e);
-  float D = (float)(1.0 / den);
+  float D = tr_rcp(kPiMul, ax, ay, c4, 1.0f + e);
   // ln D = -ln(pi ax ay c4) - 2 ln(1 + e)
   float de_dax = -2.0f * (cp * cp) * t2 / (ax * ax * ax);
   float de_day = -2.0f * (sp * sp) * t2 / (ay * ay * ay);
@@ -36,7 +35,7 @@ WPBR_HD float fresnel_conductor_grad(float cos_i, float eta_i, float eta_t, floa
   float eta = eta_t / eta_i;
   float etak = kk / eta_i;
   float c2 = cos_i * cos_i;
-  float s2 = (float)(1.0 - (double)c2);
+  float s2 = 1.0f - c2;
   float eta2 = eta * eta;
   float etak2 = etak * etak;
   float t0 = (eta2 - etak2) - s2;
@@ -91,12 +90,10 @@ WPBR_HD float fresnel_dielectric_grad(float cos_i, float eta_i, float eta_t, flo
     cos_i = fabs_(cos_i);
     swapped = true;
   }
-  double a = 1.0 - (double)(cos_i * cos_i);
-  float sin_i = (float)sqrt_d(0.0 > a ? 0.0 : a);
+  float sin_i = sqrt_one_minus(cos_i * cos_i);
   float sin_t = ei / et * sin_i;
-  if ((double)sin_t >= 1.0) return 1.0f;
-  double b = 1.0 - (double)(sin_t * sin_t);
-  float cos_t = (float)sqrt_d(0.0 > b ? 0.0 : b);
+  if (sin_t >= 1.0f) return 1.0f;
+  float cos_t = sqrt_one_minus(sin_t * sin_t);
   float A = et * cos_i, B = ei * cos_t;
   float C = ei * cos_i, E = et * cos_t;
   float r_parl = (A - B) / (A + B);
@@ -159,7 +156,7 @@ WPBR_HD int env_cell(const EnvView& e, float u, float v) {
 // Solid-angle pdf of the environment light for map cell `cell` at sin(theta)
 // st: func[cell] / Z / (2 pi^2 st), with Z the map's integral (e.marg_int).
 WPBR_HD float env_pdf_cell(const EnvView& e, int cell, float st) {
-  return (float)((double)(e.cond_func[cell] / e.marg_int) / (((2.0 * kPI) * kPI) * (double)st));
+  return div_by_scaled(e.cond_func[cell] / e.marg_int, kTwoPiSqMul, st);
 }
 
 }  // namespace wpbr

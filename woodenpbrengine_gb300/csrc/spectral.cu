@@ -156,8 +156,8 @@ __global__ void __launch_bounds__(kTB, TEX ? WPBR_SPAWN_TEX_MIN_BLOCKS : WPBR_SP
       for (uint32_t i = 0; i < nl; ++i)
         if (P.S.lights[i].type == WPBR_LIGHT_ENV) env_light = i;
       V3 dl = xvector(P.S.env.w2l, r.d);
-      float s = (float)((double)sph_phi(dl) / (2.0 * kPI));
-      float t = (float)((double)sph_theta(dl) / kPI);
+      float s = div_const(sph_phi(dl), kTwoPiDiv);
+      float t = div_const(sph_theta(dl), kPiDiv);
       st[3] = make_float4(s, t, 0.0f, 0.0f);
     }
     st[0] = make_float4(__uint_as_float(flags), __uint_as_float(env_light), 0.0f, 0.0f);
@@ -249,11 +249,11 @@ __global__ void __launch_bounds__(kTB, TEX ? WPBR_SPAWN_TEX_MIN_BLOCKS : WPBR_SP
       V3 wl = xvector(P.S.env.w2l, wi_w);
       float theta = sph_theta(wl);
       float phi = sph_phi(wl);
-      float uu = (float)((double)phi / (2.0 * kPI));
-      float vv = (float)((double)theta / kPI);
+      float uu = div_const(phi, kTwoPiDiv);
+      float vv = div_const(theta, kPiDiv);
       float stt = sinf_(theta);
       contributes = stt != 0.0f;  // else Li stays black
-      if (contributes) blpdf = (float)((double)env_pdf_uv(P.S.env, uu, vv) / (((2.0 * kPI) * kPI) * (double)stt));
+      if (contributes) blpdf = div_by_scaled(env_pdf_uv(P.S.env, uu, vv), kTwoPiSqMul, stt);
       s3.z = uu;
       s3.w = vv;
     }

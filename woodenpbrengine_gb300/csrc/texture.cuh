@@ -115,6 +115,9 @@ WPBR_HD RGB3 rlerp(float t, RGB3 a, RGB3 b) {
   return RGB3{(1.0f - t) * a.r + t * b.r, (1.0f - t) * a.g + t * b.g, (1.0f - t) * a.b + t * b.b};
 }
 
+// log2f_ (wpbr_fmath.h) without its double product.
+WPBR_HD float log2_(float x) { return mul_const(logf_(x), kLog2eMul); }
+
 // STexture2DSamplerAnisotropic::eval. The reference compares dstdx with itself
 // when picking the major axis (never swaps) and hands ewa the unclamped
 // derivatives; the clamped minor axis only chooses the level.
@@ -129,7 +132,7 @@ WPBR_HD RGB3 tex_aniso(const TexView& T, uint32_t texid, const TexFootprint& fp)
   }
   if (minor == 0.0f) return tex_triangle(T, ti, fp.p, 0);
   uint32_t n = ti.n_levels;
-  float lod = (float)(n - 1) + log2f_(minor > 0.0f ? minor : 0.0f);
+  float lod = (float)(n - 1) + log2_(minor > 0.0f ? minor : 0.0f);
   lod = lod > 0.0f ? lod : 0.0f;
   int ilod = (int)floorf(lod);
   if (ilod >= (int)n - 1) return tex_ewa(T, ti, fp, n - 1);
@@ -148,7 +151,7 @@ WPBR_HD RGB3 tex_iso(const TexView& T, uint32_t texid, const TexFootprint& fp) {
   float width = 2.0f * (a < b ? b : a);
   if (!(width > 0.0f)) return tex_triangle(T, ti, fp.p, 0);
   uint32_t n = ti.n_levels;
-  float level = (float)(n - 1) + log2f_(width);
+  float level = (float)(n - 1) + log2_(width);
   if (level < 0.0f) return tex_triangle(T, ti, fp.p, 0);
   if (level >= (float)(n - 1)) return tex_texel(T, T.levels[ti.first_level + n - 1], 0, 0);
   int il = (int)floorf(level);
@@ -204,11 +207,11 @@ WPBR_HD SurfDiff surf_differentials(const SurfInt& s, const RayD& r) {
 WPBR_HD V2 sphere_st(const Xf& w2o, V3 p) {
   V3 v = normalize(xpoint(w2o, p));
   float theta = sph_theta(v), phi = sph_phi(v);
-  return V2{(float)((double)theta * 1.0 / kPI), (float)((double)phi / (2.0 * kPI))};
+  return V2{div_const(theta, kPiDiv), div_const(phi, kTwoPiDiv)};
 }
 
 WPBR_HD float sphere_wrap(float x) {
-  if ((double)x > 0.5) return 1.0f - x;
+  if (x > 0.5f) return 1.0f - x;
   if (x < -0.5f) return -x + 1.0f;
   return x;
 }
