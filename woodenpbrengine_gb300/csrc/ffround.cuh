@@ -5,10 +5,11 @@
 // sphere quadratic, the square roots of 1 - x^2) and rounds the result to
 // float. GB300 issues one FP64 instruction per 16 cycles and SM where it
 // issues four FP32 ones per cycle, and those expressions kept the FP64 pipe
-// 73 % busy in the spawn kernel and 75 % in the shadow traversal of a sphere
-// scene. Here each expression is evaluated as an unevaluated sum hi + lo of
-// two floats (error-free products by fused multiply-add, error-free sums by
-// Knuth's TwoSum; T. J. Dekker, "A floating-point technique for extending the
+// 73 % busy in the spawn kernel of a 1080p frame, 75 % in the shadow traversal
+// of a sphere scene and 41 to 49 % in the differentiable estimator's. Here
+// each one is evaluated as an unevaluated sum hi + lo of two floats
+// (error-free products by fused multiply-add, error-free sums by Knuth's
+// TwoSum; T. J. Dekker, "A floating-point technique for extending the
 // available precision", Numer. Math. 18, 1971) with a relative error below
 // 2^-43, and the float result is taken only if every number within 2^-42 of
 // hi + lo rounds to the same float (Ziv's rounding test). The double
@@ -18,8 +19,9 @@
 // that an error term could leave the float range) takes the double expression
 // itself, out of line.
 //
-// Measured on GB300 (per-pass times of the kernels that lost their doubles):
-// see the figures at each user.
+// Per pass, before -> after: 1080p full frame, spawn 171 -> 143 us, finish 70
+// -> 57 us; textured spheres at 1080p, shadow rays 144 -> 112 us; 512 x 512
+// differentiable pass, spawn 47 -> 42 us, shadow rays 46 -> 33 us.
 #pragma once
 
 #include <stdint.h>
