@@ -225,8 +225,8 @@ WPBR_API void wpbr_destroy(wpbr_ctx* ctx) {
   bvh_release(ctx, false);
   if (ctx->bvh.h_info) cudaFreeHost(ctx->bvh.h_info);
   RenderState& R = ctx->rs;
-  if (R.ggraph) cudaGraphExecDestroy(R.ggraph);
-  if (R.sgraph) cudaGraphExecDestroy(R.sgraph);
+  for (RenderState::GroupGraph& g : R.groups)
+    if (g.exec) cudaGraphExecDestroy(g.exec);
   for (uint32_t g = 0; g < RenderState::kMaxGroup; ++g) {
     if (R.gstream[g]) cudaStreamDestroy(R.gstream[g]);
     if (R.gjoin[g]) cudaEventDestroy(R.gjoin[g]);
@@ -234,7 +234,7 @@ WPBR_API void wpbr_destroy(wpbr_ctx* ctx) {
   if (R.gfork) cudaEventDestroy(R.gfork);
   R.acc.release(); R.hit_prim.release(); R.shadow_rays.release(); R.shadow_hit.release(); R.shadow_map.release();
   R.pstate.release();
-  R.Lbuf.release(); R.pfilm.release(); R.pass_dev.release(); R.counters.release();
+  R.Lbuf.release(); R.pfilm.release(); R.pass_dev.release(); R.counters.release(); R.order.release(); R.slices.release();
   R.spec_mats.release(); R.spec_le.release(); R.spec_L.release(); R.spec_acc.release();
   ctx->io_rays.release(); ctx->io_hits.release(); ctx->io_stats.release();
   ctx->tscr[0].release(); ctx->tscr[1].release();

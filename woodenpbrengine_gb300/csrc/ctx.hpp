@@ -129,17 +129,17 @@ struct RenderState {
   bool spec_dirty = false;  // Sampled64 passes ran since the last toRGB of the film
   const uint32_t* pass_ptr = nullptr;  // shared pass index (batches); null: pass_dev
   uint32_t trace_grid = 0;             // persistent traversal grid cap (0: full)
-  // pass groups (render_frame, small RGB films): kMaxGroup branches of one
-  // fork/join graph, each on its own stream, state slice and pass index word
+  // pass groups (render_frame): up to kMaxGroup branches of one fork/join
+  // graph, each on its own stream, state slice and pass index word. Slice 0
+  // is the buffers above, the others lie in `slices`; a frame has at most two
+  // graphs, one for its whole groups and one for the passes left over.
   static constexpr uint32_t kMaxGroup = 8;
-  uint32_t group = 0;  // passes per group of the captured group graph
-  cudaGraphExec_t ggraph = nullptr;
-  uint64_t ggraph_key = 0;
-  // Sampled64 frames: one graph of `sgroup` sequential passes (sample slots
-  // 0 .. sgroup - 1) and one film gather over them
-  cudaGraphExec_t sgraph = nullptr;
-  uint64_t sgraph_key = 0;
-  uint32_t sgroup = 0;
+  struct GroupGraph {
+    cudaGraphExec_t exec = nullptr;
+    uint64_t key = 0;
+  };
+  GroupGraph groups[2];
+  DevBuf<unsigned char> slices;
   cudaStream_t gstream[kMaxGroup] = {};
   cudaEvent_t gfork = nullptr, gjoin[kMaxGroup] = {};
 };
@@ -295,19 +295,33 @@ wpbr_status render_pass_fused(wpbr_ctx* ctx, uint32_t pass);
 wpbr_status render_pass_launch(wpbr_ctx* ctx);
 wpbr_status render_frame(wpbr_ctx* ctx);
 wpbr_status spectral_setup(wpbr_ctx* ctx);
+// The per-pixel buffers one sample pass works in (slice g of a pass group).
+struct PassBufs {
+  uint32_t* hit_prim;
+  float4* pstate;
+  float4* Lbuf;
+  float2* pfilm;
+  float4* shadow_rays;
+  uint32_t* shadow_map;
+  uint32_t* shadow_hit;
+  uint32_t* order;
+  uint32_t* counters;
+};
 // Sampled64 pieces of render_pass_launch: the scalar spawn (replaces the
 // RGB spawn) and the per-bin finish + film (replace the RGB finish + film).
 // `order`: the material-sorted pixel order (null: film order).
 // Sample slots: a Sampled64 frame writes `slots` passes' film positions and
 // spectra side by side and gathers them into the film at once.
 cudaError_t spectral_slots(wpbr_ctx* ctx, uint32_t slots);
-cudaError_t spectral_spawn_launch(wpbr_ctx* ctx, const uint32_t* pass_ptr, const uint32_t* order, uint32_t slot);
-cudaError_t spectral_finish_launch(wpbr_ctx* ctx, const uint32_t* order, uint32_t slot, uint32_t film_slots);
+cudaError_t spectral_spawn_launch(wpbr_ctx* ctx, const PassBufs& B, const uint32_t* pass_ptr, const uint32_t* order,
+                                  uint32_t slot, cudaStream_t st);
+cudaError_t spectral_finish_launch(wpbr_ctx* ctx, const PassBufs& B, const uint32_t* order, uint32_t slot,
+                                   cudaStream_t st);
+cudaError_t spectral_film_launch(wpbr_ctx* ctx, uint32_t film_slots, cudaStream_t st);
 wpbr_status spectral_resolve(wpbr_ctx* ctx);
 // float4 per pixel of the fused pass's state buffer (RenderState::pstate);
 // the RGB and the Sampled64 spawn records both fit in it.
 constexpr int kPassStateF4 = 7;
-uint32_t persistent_full_grid();
 void bvh_release(wpbr_ctx* ctx, bool keep_traversal);
 wpbr_status job_run(wpbr_ctx* ctx, uint32_t job, uint32_t pass);
 wpbr_status job_record(wpbr_ctx* ctx, uint32_t x0, uint32_t y0, uint32_t x1, uint32_t y1, wpbr_pass_record* rec);

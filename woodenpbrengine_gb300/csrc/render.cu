@@ -508,61 +508,87 @@ wpbr_status render_setup(wpbr_ctx* ctx, uint32_t spp, uint32_t seed, uint32_t st
 
 
 namespace {
-// The kernels of one sample pass on stream `st` over state slice g of a pass
-// group (per-pixel arrays offset by g films, counters by g sets), reading the
-// pass index at pass_ptr; with_film appends the film gather. Sampled64
-// passes write sample slot spec_slot and, when spec_film > 0, gather slots
-// 0 .. spec_film - 1 into the film.
-wpbr_status pass_kernels(wpbr_ctx* ctx, uint32_t g, const uint32_t* pass_ptr, cudaStream_t st, uint32_t grid,
-                         bool with_film, uint32_t spec_slot = 0, uint32_t spec_film = 1) {
+// Bytes of one state slice: the per-pixel arrays, then the counters, each
+// part 256-byte aligned.
+constexpr size_t kSliceAlign = 256;
+size_t slice_part(size_t bytes) { return (bytes + kSliceAlign - 1) / kSliceAlign * kSliceAlign; }
+template <class F>
+size_t slice_layout(size_t n, F&& part) {
+  size_t at = 0;
+  for (size_t bytes : {n * 4, n * kStateF4 * 16, n * 16, n * 8, n * 64, n * 8, n * 8, n * 4,
+                       (size_t)kPassCounters * 4}) {
+    part(at);
+    at += slice_part(bytes);
+  }
+  return at;
+}
+size_t slice_bytes(size_t n) {
+  return slice_layout(n, [](size_t) {});
+}
+
+// State slice g of a pass group: the context's own buffers for g = 0.
+PassBufs pass_bufs(const wpbr_ctx* ctx, uint32_t g) {
+  const RenderState& R = ctx->rs;
+  if (g == 0)
+    return PassBufs{R.hit_prim.p,   R.pstate.p,     R.Lbuf.p,  R.pfilm.p,   R.shadow_rays.p,
+                    R.shadow_map.p, R.shadow_hit.p, R.order.p, R.counters.p};
+  const size_t n = (size_t)R.W * R.H;
+  unsigned char* at[9];
+  int k = 0;
+  unsigned char* base = R.slices.p + (size_t)(g - 1) * slice_bytes(n);
+  slice_layout(n, [&](size_t off) { at[k++] = base + off; });
+  return PassBufs{(uint32_t*)at[0], (float4*)at[1],   (float4*)at[2],   (float2*)at[3],  (float4*)at[4],
+                  (uint32_t*)at[5], (uint32_t*)at[6], (uint32_t*)at[7], (uint32_t*)at[8]};
+}
+
+void film_launch(const wpbr_ctx* ctx, const PassBufs& B, cudaStream_t st) {
+  const RenderState& R = ctx->rs;
+  k_film_tiles<<<dim3(div_up(R.W, kFilmTile), div_up(R.H, kFilmTile)), kFilmThreadsRGB, 0, st>>>(
+      R.W, R.H, B.pfilm, B.Lbuf, (float4*)R.acc.p);
+}
+
+// The kernels of one sample pass up to its samples (the film gather follows),
+// on stream `st` in state slice B, reading the pass index at pass_ptr. A
+// Sampled64 pass writes sample slot spec_slot.
+wpbr_status pass_kernels(wpbr_ctx* ctx, const PassBufs& B, const uint32_t* pass_ptr, cudaStream_t st, uint32_t grid,
+                         uint32_t spec_slot = 0) {
   RenderState& R = ctx->rs;
   PassCtx P = make_pass_ctx(ctx);
   const uint32_t n = R.W * R.H;
-  const size_t o = (size_t)g * n;
-  uint32_t* counters = R.counters.p + (size_t)g * kPassCounters;
-  uint32_t* hit_prim = R.hit_prim.p + o;
-  float4* pstate = R.pstate.p + o * kStateF4;
-  float4* Lbuf = R.Lbuf.p + o;
-  float2* pfilm = R.pfilm.p + o;
-  uint32_t* shadow_hit = R.shadow_hit.p + 2 * o;
-  uint32_t* order_buf = R.order.p + o;
+  uint32_t* counters = B.counters;
   WPBR_CUDA(cudaMemsetAsync(counters, 0, kPassCounters * sizeof(uint32_t), st));
-  const ShadowQueue sq{R.shadow_rays.p + 4 * o, R.shadow_map.p + 2 * o, counters + kQueueCounter};
+  const ShadowQueue sq{B.shadow_rays, B.shadow_map, counters + kQueueCounter};
   bool spectral = ctx->spectrum == WPBR_SPECTRUM_SAMPLED64;
-  launch_traversal<false>(P.S, P.Bv, CameraSrc{P, pass_ptr}, PrimSink{hit_prim}, n, counters, P.err, st, grid);
+  launch_traversal<false>(P.S, P.Bv, CameraSrc{P, pass_ptr}, PrimSink{B.hit_prim}, n, counters, P.err, st, grid);
   // the pixels in material-sorted order for the spawn and finish kernels
   const uint32_t* order = nullptr;
   if (n >= kSortMinPixels) {
     uint32_t* cat_counts = counters + 2;
-    k_cat_count<<<div_up(n, kCatBlock), kCatBlock, 0, st>>>(P.S, n, hit_prim, cat_counts);
-    k_cat_scatter<<<div_up(n, kCatBlock), kCatBlock, 0, st>>>(P.S, n, hit_prim, cat_counts, cat_counts + kPixCats,
-                                                              order_buf, P.err);
-    order = order_buf;
+    k_cat_count<<<div_up(n, kCatBlock), kCatBlock, 0, st>>>(P.S, n, B.hit_prim, cat_counts);
+    k_cat_scatter<<<div_up(n, kCatBlock), kCatBlock, 0, st>>>(P.S, n, B.hit_prim, cat_counts, cat_counts + kPixCats,
+                                                              B.order, P.err);
+    order = B.order;
   }
   if (spectral)
-    WPBR_CUDA(spectral_spawn_launch(ctx, pass_ptr, order, spec_slot));
+    WPBR_CUDA(spectral_spawn_launch(ctx, B, pass_ptr, order, spec_slot, st));
   else
-    (ctx->has_metal ? k_spawn<true> : k_spawn<false>)<<<div_up(n, kTB), kTB, 0, st>>>(P, pass_ptr, hit_prim, pstate,
-                                                                                      sq, Lbuf, pfilm, order);
+    (ctx->has_metal ? k_spawn<true> : k_spawn<false>)<<<div_up(n, kTB), kTB, 0, st>>>(
+        P, pass_ptr, B.hit_prim, B.pstate, sq, B.Lbuf, B.pfilm, order);
   // shadow rays: unoccluded iff no hit or the closest hit is the sampled
   // light's primitive; with environment lights only that is "no hit", which
   // the any-hit traversal decides with the same primitive tests, stopping at
   // the first hit (the stored id is then some hit, never a light's)
   // (the spawn queued only the rays it traces; the traversal walks the queue)
   const QueueSrc qsrc{sq.rays, sq.count};
-  const MapSink qsink{shadow_hit, sq.map};
+  const MapSink qsink{B.shadow_hit, sq.map};
   if (ctx->env_lights_only)
     launch_traversal<true>(P.S, P.Bv, qsrc, qsink, 2 * n, counters + 1, P.err, st, grid);
   else
     launch_traversal<false>(P.S, P.Bv, qsrc, qsink, 2 * n, counters + 1, P.err, st, grid);
-  if (spectral) {
-    WPBR_CUDA(spectral_finish_launch(ctx, order, spec_slot, spec_film));
-  } else {
-    k_finish<<<div_up(n, kTB), kTB, 0, st>>>(P, pstate, shadow_hit, Lbuf, order);
-    if (with_film)
-      k_film_tiles<<<dim3(div_up(R.W, kFilmTile), div_up(R.H, kFilmTile)), kFilmThreadsRGB, 0, st>>>(
-          R.W, R.H, pfilm, Lbuf, (float4*)R.acc.p);
-  }
+  if (spectral)
+    WPBR_CUDA(spectral_finish_launch(ctx, B, order, spec_slot, st));
+  else
+    k_finish<<<div_up(n, kTB), kTB, 0, st>>>(P, B.pstate, B.shadow_hit, B.Lbuf, order);
   WPBR_CUDA(cudaGetLastError());
   return WPBR_OK;
 }
@@ -578,11 +604,16 @@ wpbr_status render_pass_launch(wpbr_ctx* ctx) {
   WPBR_CUDA(R.counters.ensure(kPassCounters));
   WPBR_CUDA(R.shadow_map.ensure((size_t)2 * n));
   WPBR_CUDA(R.order.ensure(n));
-  return pass_kernels(ctx, 0, R.pass_ptr ? R.pass_ptr : R.pass_dev.p, ctx->stream, R.trace_grid, true);
-}
-
-uint32_t persistent_full_grid() {
-  return persistent_grid((const void*)k_trace_persistent<false, 64, true, CameraSrc, PrimSink>);
+  const PassBufs B = pass_bufs(ctx, 0);
+  wpbr_status s = pass_kernels(ctx, B, R.pass_ptr ? R.pass_ptr : R.pass_dev.p, ctx->stream, R.trace_grid);
+  if (s != WPBR_OK) return s;
+  if (ctx->spectrum == WPBR_SPECTRUM_SAMPLED64) {
+    WPBR_CUDA(spectral_film_launch(ctx, 1, ctx->stream));
+  } else {
+    film_launch(ctx, B, ctx->stream);
+    WPBR_CUDA(cudaGetLastError());
+  }
+  return WPBR_OK;
 }
 
 // Everything the captured pass graph bakes into its kernel arguments: the
@@ -606,7 +637,7 @@ static uint64_t pass_graph_key(const wpbr_ctx* ctx) {
   mix((uint64_t)ctx->spectrum | ((uint64_t)ctx->quirks << 8));
   const void* ptrs[] = {R.acc.p,    R.hit_prim.p, R.shadow_rays.p,     R.shadow_hit.p,      R.shadow_map.p, R.pstate.p,
                         R.Lbuf.p,   R.pfilm.p,    R.pass_dev.p,        R.counters.p,        R.pass_ptr, R.order.p,
-                        ctx->d_err.p, ctx->bvh.view.nodes,
+                        R.slices.p, ctx->d_err.p, ctx->bvh.view.nodes,
                         ctx->bvh.view.prims, R.spec_mats.p, R.spec_le.p, R.spec_L.p, R.spec_acc.p};
   for (const void* q : ptrs) mix((uint64_t)(uintptr_t)q);
   return h;
@@ -646,152 +677,119 @@ wpbr_status render_pass_fused(wpbr_ctx* ctx, uint32_t pass) {
   return WPBR_OK;
 }
 
-// Passes per group for a frame: small films leave most of the GPU idle in one
-// pass (its traversals hold a few tens of thousands of rays), so the passes
-// of a group run as concurrent branches until a group holds about 2^18 rays;
-// the size divides spp, so every group is whole.
-uint32_t group_size(uint32_t n, uint32_t spp) {
-  uint32_t k = (uint32_t)std::min<uint64_t>(RenderState::kMaxGroup, ((1ull << 18) + n - 1) / n);
-  k = std::min(k, spp);
-  while (k > 1 && spp % k) --k;
-  return std::max(k, 1u);
+// Passes per group of a frame. A traversal launch ends with a tail in which
+// most of its warps have no ray left (1080p full frame: 31 to 41 % of the warp
+// slots active over the launch), and a small film never fills the GPU at all,
+// so the passes of a group run as concurrent branches and fill one another's
+// tails. 1080p x 16 spp, full frame / textured, groups of 1: 19.9 / 14.6 ms;
+// 2: 16.0 / 14.1; 4: 15.2 / 13.8; 8: 14.8 / 13.6. A Sampled64 pass also keeps a
+// slot of 64-bin samples per pixel until the group's film gather, so those
+// groups stop at 4. Groups are bounded to 2^24 pixels of state (3.8 GB);
+// larger films render fewer passes at a time.
+uint32_t group_size(const RenderState& R, bool spectral) {
+  const uint64_t n = (uint64_t)R.W * R.H;
+  const uint64_t k = std::max<uint64_t>(1u, (1ull << 24) / n);
+  return (uint32_t)std::min<uint64_t>({k, R.spp, spectral ? 4u : RenderState::kMaxGroup});
 }
 
-// A Sampled64 frame in groups of J sequential passes: one graph runs the J
-// passes, each writing its film positions and spectra to its own sample
-// slot, then one film gather adds the J slots in pass order (each pass's
-// neighbours in row-major order), so the film is identical to J one-pass
-// gathers while the 64-bin accumulator is read and written once per group.
-static wpbr_status spectral_frame(wpbr_ctx* ctx, uint32_t J) {
+// Captures (or reuses) the graph of a group of K passes. RGB: K branches, each
+// pass in its own state slice, and the film gathers in pass order on the
+// context's stream, each as soon as its branch is done. Sampled64: K branches
+// writing sample slots 0 .. K - 1, then one film gather over the slots. Every
+// pass computes what it computes alone and the film adds the passes in order,
+// so the film is the one that K single passes make. Returns WPBR_OK with
+// G.exec null when the stream cannot be captured (the legacy default stream).
+static wpbr_status group_graph(wpbr_ctx* ctx, RenderState::GroupGraph& G, uint32_t K) {
   RenderState& R = ctx->rs;
   cudaStream_t st = ctx->stream;
-  const uint32_t n = R.W * R.H;
-  WPBR_CUDA(spectral_slots(ctx, J));
-  WPBR_CUDA(R.pass_dev.ensure(J));
-  WPBR_CUDA(R.counters.ensure(kPassCounters));
-  WPBR_CUDA(R.shadow_map.ensure((size_t)2 * n));
-  WPBR_CUDA(R.order.ensure(n));
-  const uint64_t key = pass_graph_key(ctx) * 0x100000001B3ull + 0x5300u + J;
-  if (R.sgraph && (R.sgraph_key != key || R.sgroup != J)) {
-    cudaGraphExecDestroy(R.sgraph);
-    R.sgraph = nullptr;
-  }
-  if (!R.sgraph) {
-    cudaGraph_t gr = nullptr;
-    WPBR_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    wpbr_status s = WPBR_OK;
-    for (uint32_t j = 0; j < J && s == WPBR_OK; ++j)
-      s = pass_kernels(ctx, 0, R.pass_dev.p + j, st, R.trace_grid, false, j, j + 1 == J ? J : 0);
-    cudaError_t e2 = cudaStreamEndCapture(st, &gr);
-    cudaError_t e = cudaSuccess;
-    if (s == WPBR_OK && e2 == cudaSuccess && gr) e = cudaGraphInstantiate(&R.sgraph, gr, 0);
-    if (gr) cudaGraphDestroy(gr);
-    if (s != WPBR_OK) {
-      cudaGetLastError();
-      return s;
-    }
-    if (e != cudaSuccess || e2 != cudaSuccess || !R.sgraph) {
-      cudaGetLastError();
-      R.sgraph = nullptr;
-      return set_err(ctx, WPBR_ERR_CUDA, "render: Sampled64 pass-group graph capture failed");
-    }
-    R.sgraph_key = key;
-    R.sgroup = J;
-  }
-  R.spec_dirty = true;
-  uint32_t passes[4];
-  for (uint32_t base = 0; base < R.spp; base += J) {
-    for (uint32_t j = 0; j < J; ++j) passes[j] = base + j;
-    WPBR_CUDA(cudaMemcpyAsync(R.pass_dev.p, passes, sizeof(uint32_t) * J, cudaMemcpyHostToDevice, st));
-    WPBR_CUDA(cudaGraphLaunch(R.sgraph, st));
-  }
-  return WPBR_OK;
-}
-
-// A whole frame (every pass of render_setup's spp) through the fused pass.
-// Films of RGB frames that fit a group of several passes render a group at a
-// time: one fork/join graph whose K branches run the pass kernels of passes
-// base .. base + K - 1 on their own streams, state slices and pass index
-// words (each traversal capped at a K-th of the resident grid), then the K
-// film gathers in pass order on the context's stream. Every pass computes
-// what it computes alone, and the film adds the passes in the same order, so
-// the film is identical to spp calls of render_pass_fused.
-wpbr_status render_frame(wpbr_ctx* ctx) {
-  RenderState& R = ctx->rs;
-  if (!R.ready) return set_err(ctx, WPBR_ERR_NOT_BUILT, "render: render_setup not called");
-  const uint32_t n = R.W * R.H;
-  if (ctx->spectrum == WPBR_SPECTRUM_SAMPLED64 && !R.pass_ptr) {
-    const uint32_t J = R.spp % 4 == 0 ? 4u : (R.spp % 2 == 0 ? 2u : 1u);
-    if (J > 1) return spectral_frame(ctx, J);
-  }
-  const uint32_t K = (ctx->spectrum == WPBR_SPECTRUM_RGB && !R.pass_ptr) ? group_size(n, R.spp) : 1u;
-  if (K <= 1) {
-    for (uint32_t p = 0; p < R.spp; ++p) {
-      wpbr_status s = render_pass_fused(ctx, p);
-      if (s != WPBR_OK) return s;
-    }
-    return WPBR_OK;
-  }
-  cudaStream_t st = ctx->stream;
-  const size_t kn = (size_t)K * n;
-  WPBR_CUDA(R.hit_prim.ensure(kn));
-  WPBR_CUDA(R.pstate.ensure(kn * kStateF4));
-  WPBR_CUDA(R.Lbuf.ensure(kn));
-  WPBR_CUDA(R.pfilm.ensure(kn));
-  WPBR_CUDA(R.shadow_rays.ensure(4 * kn));
-  WPBR_CUDA(R.shadow_map.ensure(2 * kn));
-  WPBR_CUDA(R.shadow_hit.ensure(2 * kn));
-  WPBR_CUDA(R.order.ensure(kn));
-  WPBR_CUDA(R.counters.ensure((size_t)K * kPassCounters));
-  WPBR_CUDA(R.pass_dev.ensure(K));
+  const bool spectral = ctx->spectrum == WPBR_SPECTRUM_SAMPLED64;
+  const uint64_t key = pass_graph_key(ctx) * 0x100000001B3ull + K;
+  if (G.exec && G.key == key) return WPBR_OK;
+  if (G.exec) cudaGraphExecDestroy(G.exec);
+  G.exec = nullptr;
   for (uint32_t g = 0; g < K; ++g)
     if (!R.gstream[g]) WPBR_CUDA(cudaStreamCreateWithFlags(&R.gstream[g], cudaStreamNonBlocking));
   if (!R.gfork) WPBR_CUDA(cudaEventCreateWithFlags(&R.gfork, cudaEventDisableTiming));
   for (uint32_t g = 0; g < K; ++g)
     if (!R.gjoin[g]) WPBR_CUDA(cudaEventCreateWithFlags(&R.gjoin[g], cudaEventDisableTiming));
-  const uint64_t key = pass_graph_key(ctx) * 0x100000001B3ull + K;
-  if (R.ggraph && (R.ggraph_key != key || R.group != K)) {
-    cudaGraphExecDestroy(R.ggraph);
-    R.ggraph = nullptr;
+  if (cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
+    cudaGetLastError();
+    return WPBR_OK;
   }
-  if (!R.ggraph) {
-    const uint32_t full = persistent_full_grid();
-    const uint32_t grid = std::max(1u, full / K);
-    cudaGraph_t gr = nullptr;
-    WPBR_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    wpbr_status s = WPBR_OK;
-    cudaError_t e = cudaEventRecord(R.gfork, st);
-    for (uint32_t g = 0; g < K && e == cudaSuccess && s == WPBR_OK; ++g) {
-      e = cudaStreamWaitEvent(R.gstream[g], R.gfork, 0);
-      if (e != cudaSuccess) break;
-      s = pass_kernels(ctx, g, R.pass_dev.p + g, R.gstream[g], grid, false);
-      if (s != WPBR_OK) break;
-      e = cudaEventRecord(R.gjoin[g], R.gstream[g]);
-      if (e == cudaSuccess) e = cudaStreamWaitEvent(st, R.gjoin[g], 0);
-    }
-    for (uint32_t g = 0; g < K && e == cudaSuccess && s == WPBR_OK; ++g)
-      k_film_tiles<<<dim3(div_up(R.W, kFilmTile), div_up(R.H, kFilmTile)), kFilmThreadsRGB, 0, st>>>(
-          R.W, R.H, R.pfilm.p + (size_t)g * n, R.Lbuf.p + (size_t)g * n, (float4*)R.acc.p);
-    cudaError_t e2 = cudaStreamEndCapture(st, &gr);
-    if (s == WPBR_OK && e == cudaSuccess && e2 == cudaSuccess && gr) e = cudaGraphInstantiate(&R.ggraph, gr, 0);
-    if (gr) cudaGraphDestroy(gr);
-    if (s != WPBR_OK) {
-      cudaGetLastError();
-      return s;
-    }
-    if (e != cudaSuccess || e2 != cudaSuccess || !R.ggraph) {
-      cudaGetLastError();
-      R.ggraph = nullptr;
-      return set_err(ctx, WPBR_ERR_CUDA, "render: pass-group graph capture failed");
-    }
-    R.ggraph_key = key;
-    R.group = K;
+  wpbr_status s = WPBR_OK;
+  cudaError_t e = cudaEventRecord(R.gfork, st);
+  for (uint32_t g = 0; g < K && e == cudaSuccess && s == WPBR_OK; ++g) {
+    e = cudaStreamWaitEvent(R.gstream[g], R.gfork, 0);
+    if (e != cudaSuccess) break;
+    s = pass_kernels(ctx, pass_bufs(ctx, g), R.pass_dev.p + g, R.gstream[g], R.trace_grid, g);
+    if (s != WPBR_OK) break;
+    e = cudaEventRecord(R.gjoin[g], R.gstream[g]);
   }
-  uint32_t passes[RenderState::kMaxGroup];
-  for (uint32_t base = 0; base < R.spp; base += K) {
-    for (uint32_t g = 0; g < K; ++g) passes[g] = base + g;
-    WPBR_CUDA(cudaMemcpyAsync(R.pass_dev.p, passes, sizeof(uint32_t) * K, cudaMemcpyHostToDevice, st));
-    WPBR_CUDA(cudaGraphLaunch(R.ggraph, st));
+  for (uint32_t g = 0; g < K && e == cudaSuccess && s == WPBR_OK; ++g) {
+    e = cudaStreamWaitEvent(st, R.gjoin[g], 0);
+    if (e == cudaSuccess && !spectral) film_launch(ctx, pass_bufs(ctx, g), st);
+  }
+  if (e == cudaSuccess && s == WPBR_OK && spectral) e = spectral_film_launch(ctx, K, st);
+  cudaGraph_t gr = nullptr;
+  const cudaError_t e2 = cudaStreamEndCapture(st, &gr);
+  if (s == WPBR_OK && e == cudaSuccess && e2 == cudaSuccess && gr) e = cudaGraphInstantiate(&G.exec, gr, 0);
+  if (gr) cudaGraphDestroy(gr);
+  if (s != WPBR_OK) {
+    cudaGetLastError();
+    return s;
+  }
+  if (e != cudaSuccess || e2 != cudaSuccess || !G.exec) {
+    cudaGetLastError();
+    G.exec = nullptr;
+    return set_err(ctx, WPBR_ERR_CUDA, "render: pass-group graph capture failed");
+  }
+  G.key = key;
+  return WPBR_OK;
+}
+
+// A whole frame (every pass of render_setup's spp) through the fused pass, in
+// pass groups; spp that the group size does not divide ends with a smaller
+// group (a graph of its own).
+wpbr_status render_frame(wpbr_ctx* ctx) {
+  RenderState& R = ctx->rs;
+  if (!R.ready) return set_err(ctx, WPBR_ERR_NOT_BUILT, "render: render_setup not called");
+  const size_t n = (size_t)R.W * R.H;
+  const bool spectral = ctx->spectrum == WPBR_SPECTRUM_SAMPLED64;
+  uint32_t K = R.pass_ptr ? 1u : group_size(R, spectral);
+  if (K > 1) {
+    // the group's buffers; a device without room for them renders one pass at
+    // a time, in the buffers render_setup made
+    cudaError_t e = R.slices.ensure((K - 1) * slice_bytes(n));
+    if (e == cudaSuccess) e = R.pass_dev.ensure(RenderState::kMaxGroup);
+    if (e == cudaSuccess && spectral) e = spectral_slots(ctx, K);
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      R.slices.release();
+      K = 1;
+      WPBR_CUDA(R.pass_dev.ensure(1));
+      if (spectral) WPBR_CUDA(spectral_slots(ctx, 1));
+    } else {
+      WPBR_CUDA(e);
+    }
+  }
+  uint32_t base = 0;
+  cudaStream_t st = ctx->stream;
+  while (K > 1 && base < R.spp) {
+    const uint32_t k = std::min(K, R.spp - base);
+    RenderState::GroupGraph& G = R.groups[k == K ? 0 : 1];
+    wpbr_status s = group_graph(ctx, G, k);
+    if (s != WPBR_OK) return s;
+    if (!G.exec) break;
+    if (spectral) R.spec_dirty = true;
+    uint32_t passes[RenderState::kMaxGroup];
+    for (uint32_t g = 0; g < k; ++g) passes[g] = base + g;
+    WPBR_CUDA(cudaMemcpyAsync(R.pass_dev.p, passes, sizeof(uint32_t) * k, cudaMemcpyHostToDevice, st));
+    WPBR_CUDA(cudaGraphLaunch(G.exec, st));
+    base += k;
+  }
+  for (; base < R.spp; ++base) {
+    wpbr_status s = render_pass_fused(ctx, base);
+    if (s != WPBR_OK) return s;
   }
   return WPBR_OK;
 }

@@ -641,29 +641,33 @@ cudaError_t spectral_slots(wpbr_ctx* ctx, uint32_t slots) {
 // The scalar spawn of the Sampled64 pass, between the camera traversal and
 // the shadow-ray traversal (render_pass_launch); the pass's film positions go
 // to sample slot `slot`.
-cudaError_t spectral_spawn_launch(wpbr_ctx* ctx, const uint32_t* pass_ptr, const uint32_t* order, uint32_t slot) {
+cudaError_t spectral_spawn_launch(wpbr_ctx* ctx, const PassBufs& B, const uint32_t* pass_ptr, const uint32_t* order,
+                                  uint32_t slot, cudaStream_t st) {
   RenderState& R = ctx->rs;
   uint32_t n = R.W * R.H;
-  const ShadowQueue sq{R.shadow_rays.p, R.shadow_map.p, R.counters.p + kQueueCounter};
-  (ctx->has_metal ? k_sspawn<true> : k_sspawn<false>)<<<div_up(n, kTB), kTB, 0, ctx->stream>>>(
-      spec_pass_ctx(ctx), pass_ptr, R.hit_prim.p, R.pstate.p, sq, R.pfilm.p + (size_t)slot * n, order);
+  const ShadowQueue sq{B.shadow_rays, B.shadow_map, B.counters + kQueueCounter};
+  (ctx->has_metal ? k_sspawn<true> : k_sspawn<false>)<<<div_up(n, kTB), kTB, 0, st>>>(
+      spec_pass_ctx(ctx), pass_ptr, B.hit_prim, B.pstate, sq, R.pfilm.p + (size_t)slot * n, order);
   return cudaGetLastError();
 }
 
-// The per-bin finish after the shadow-ray traversal (the pass's spectra to
-// sample slot `slot`), then, when film_slots > 0, the film gather of slots
-// 0 .. film_slots - 1 in slot order.
-cudaError_t spectral_finish_launch(wpbr_ctx* ctx, const uint32_t* order, uint32_t slot, uint32_t film_slots) {
+// The per-bin finish after the shadow-ray traversal: the pass's spectra to
+// sample slot `slot`.
+cudaError_t spectral_finish_launch(wpbr_ctx* ctx, const PassBufs& B, const uint32_t* order, uint32_t slot,
+                                   cudaStream_t st) {
   RenderState& R = ctx->rs;
   uint32_t n = R.W * R.H;
   SpecCtx C{(const SpecMat*)R.spec_mats.p, (const S64*)R.spec_le.p, R.spec_L.p + (size_t)slot * n * kSpecN};
-  k_sfinish<<<div_up((uint64_t)n * kBinLanes, 128), 128, 0, ctx->stream>>>(spec_pass_ctx(ctx), C, R.pstate.p,
-                                                                            R.shadow_hit.p, order);
-  if (film_slots) {
-    dim3 fg(div_up(R.W, kFT), div_up(R.H, kFT));
-    k_sfilm<<<fg, kFilmThreads, 0, ctx->stream>>>(R.W, R.H, R.pfilm.p, R.spec_L.p, film_slots, R.spec_acc.p,
-                                                   (float4*)R.acc.p);
-  }
+  k_sfinish<<<div_up((uint64_t)n * kBinLanes, 128), 128, 0, st>>>(spec_pass_ctx(ctx), C, B.pstate, B.shadow_hit,
+                                                                   order);
+  return cudaGetLastError();
+}
+
+// The film gather of sample slots 0 .. film_slots - 1 in slot order.
+cudaError_t spectral_film_launch(wpbr_ctx* ctx, uint32_t film_slots, cudaStream_t st) {
+  RenderState& R = ctx->rs;
+  dim3 fg(div_up(R.W, kFT), div_up(R.H, kFT));
+  k_sfilm<<<fg, kFilmThreads, 0, st>>>(R.W, R.H, R.pfilm.p, R.spec_L.p, film_slots, R.spec_acc.p, (float4*)R.acc.p);
   return cudaGetLastError();
 }
 
