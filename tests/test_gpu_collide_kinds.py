@@ -1,6 +1,7 @@
 """Collide batches against the oracle over the kernels a batch can take: scenes
-of triangles only, of spheres and a quad, and of both; batches in input order
-and (2^18 rays and more) in ray order; bounded and unbounded rays."""
+of triangles only, of spheres and a quad, and of both; batches of one ray a warp
+up to full warps, with and without rays left for the warps to fetch, in input
+order and (2^19 rays and more) in ray order; bounded and unbounded rays."""
 import numpy as np
 import pytest
 
@@ -18,7 +19,7 @@ def random_rays(n, extent, seed):
 
 
 @pytest.mark.parametrize("config,level,extent", [(1, 3, 1.2), (0, 0, 12.0), (2, 4, 12.0)])
-@pytest.mark.parametrize("n", [1, 33, 5000, (1 << 18) + 7])
+@pytest.mark.parametrize("n", [1, 33, 2433, 5000, 77825, 155649, (1 << 19) + 7])
 def test_scene_kinds(W, O, ctx, config, level, extent, n):
     g = W.SceneGen(config, 11, (64, 64), level=level)
     ctx.set_quirks(0)

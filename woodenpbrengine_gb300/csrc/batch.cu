@@ -350,6 +350,7 @@ WPBR_API wpbr_status wpbr_batch_render_setup(wpbr_batch* b, uint32_t spp, uint32
     wpbr_status st = render_setup(c, spp, seed, first_stream + (uint32_t)k);
     if (st != WPBR_OK) return from_scene(b, k, st);
     c->rs.pass_ptr = b->pass_dev.p;
+    c->rs.trace_share = (uint32_t)b->scenes.size();
     BATCH_CUDA(cudaStreamSynchronize(c->stream));  // film clears done before the graph runs
   }
   b->spp = spp;

@@ -129,6 +129,7 @@ struct RenderState {
   bool spec_dirty = false;  // Sampled64 passes ran since the last toRGB of the film
   const uint32_t* pass_ptr = nullptr;  // shared pass index (batches); null: pass_dev
   uint32_t trace_grid = 0;             // persistent traversal grid cap (0: full)
+  uint32_t trace_share = 1;            // passes of this size that run at the same time (the scenes of a batch)
   // pass groups (render_frame): up to kMaxGroup branches of one fork/join
   // graph, each on its own stream, state slice and pass index word. Slice 0
   // is the buffers above, the others lie in `slices`; a frame has at most two

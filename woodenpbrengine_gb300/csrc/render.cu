@@ -548,18 +548,19 @@ void film_launch(const wpbr_ctx* ctx, const PassBufs& B, cudaStream_t st) {
 }
 
 // The kernels of one sample pass up to its samples (the film gather follows),
-// on stream `st` in state slice B, reading the pass index at pass_ptr. A
-// Sampled64 pass writes sample slot spec_slot.
-wpbr_status pass_kernels(wpbr_ctx* ctx, const PassBufs& B, const uint32_t* pass_ptr, cudaStream_t st, uint32_t grid,
-                         uint32_t spec_slot = 0) {
+// on stream `st` in state slice B, reading the pass index at pass_ptr; `share`
+// passes run at the same time. A Sampled64 pass writes sample slot spec_slot.
+wpbr_status pass_kernels(wpbr_ctx* ctx, const PassBufs& B, const uint32_t* pass_ptr, cudaStream_t st,
+                         uint32_t share, uint32_t spec_slot = 0) {
   RenderState& R = ctx->rs;
   PassCtx P = make_pass_ctx(ctx);
-  const uint32_t n = R.W * R.H;
+  const uint32_t n = R.W * R.H, grid = R.trace_grid;
   uint32_t* counters = B.counters;
   WPBR_CUDA(cudaMemsetAsync(counters, 0, kPassCounters * sizeof(uint32_t), st));
   const ShadowQueue sq{B.shadow_rays, B.shadow_map, counters + kQueueCounter};
   bool spectral = ctx->spectrum == WPBR_SPECTRUM_SAMPLED64;
-  launch_traversal<false>(P.S, P.Bv, CameraSrc{P, pass_ptr}, PrimSink{B.hit_prim}, n, counters, P.err, st, grid);
+  launch_traversal<false>(P.S, P.Bv, CameraSrc{P, pass_ptr}, PrimSink{B.hit_prim}, n, counters, P.err, st, grid,
+                          share);
   // the pixels in material-sorted order for the spawn and finish kernels
   const uint32_t* order = nullptr;
   if (n >= kSortMinPixels) {
@@ -582,9 +583,9 @@ wpbr_status pass_kernels(wpbr_ctx* ctx, const PassBufs& B, const uint32_t* pass_
   const QueueSrc qsrc{sq.rays, sq.count};
   const MapSink qsink{B.shadow_hit, sq.map};
   if (ctx->env_lights_only)
-    launch_traversal<true>(P.S, P.Bv, qsrc, qsink, 2 * n, counters + 1, P.err, st, grid);
+    launch_traversal<true>(P.S, P.Bv, qsrc, qsink, 2 * n, counters + 1, P.err, st, grid, share);
   else
-    launch_traversal<false>(P.S, P.Bv, qsrc, qsink, 2 * n, counters + 1, P.err, st, grid);
+    launch_traversal<false>(P.S, P.Bv, qsrc, qsink, 2 * n, counters + 1, P.err, st, grid, share);
   if (spectral)
     WPBR_CUDA(spectral_finish_launch(ctx, B, order, spec_slot, st));
   else
@@ -605,7 +606,7 @@ wpbr_status render_pass_launch(wpbr_ctx* ctx) {
   WPBR_CUDA(R.shadow_map.ensure((size_t)2 * n));
   WPBR_CUDA(R.order.ensure(n));
   const PassBufs B = pass_bufs(ctx, 0);
-  wpbr_status s = pass_kernels(ctx, B, R.pass_ptr ? R.pass_ptr : R.pass_dev.p, ctx->stream, R.trace_grid);
+  wpbr_status s = pass_kernels(ctx, B, R.pass_ptr ? R.pass_ptr : R.pass_dev.p, ctx->stream, R.trace_share);
   if (s != WPBR_OK) return s;
   if (ctx->spectrum == WPBR_SPECTRUM_SAMPLED64) {
     WPBR_CUDA(spectral_film_launch(ctx, 1, ctx->stream));
@@ -721,7 +722,7 @@ static wpbr_status group_graph(wpbr_ctx* ctx, RenderState::GroupGraph& G, uint32
   for (uint32_t g = 0; g < K && e == cudaSuccess && s == WPBR_OK; ++g) {
     e = cudaStreamWaitEvent(R.gstream[g], R.gfork, 0);
     if (e != cudaSuccess) break;
-    s = pass_kernels(ctx, pass_bufs(ctx, g), R.pass_dev.p + g, R.gstream[g], R.trace_grid, g);
+    s = pass_kernels(ctx, pass_bufs(ctx, g), R.pass_dev.p + g, R.gstream[g], K, g);
     if (s != WPBR_OK) break;
     e = cudaEventRecord(R.gjoin[g], R.gstream[g]);
   }

@@ -161,9 +161,8 @@ wpbr_status trace_rays(wpbr_ctx* ctx, const float4* d_rays, uint64_t n, float4* 
     e = X.counter.ensure(1);
     if (e == cudaSuccess) {
       uint32_t* c = X.counter.p;
-      e = cudaMemsetAsync(c, 0, sizeof(uint32_t), st);
       const uint32_t* perm = nullptr;
-      if (e == cudaSuccess && sorted) e = ray_order(ctx, X, Bv, d_rays, (uint32_t)n, st, &perm, nullptr);
+      if (sorted) e = ray_order(ctx, X, Bv, d_rays, (uint32_t)n, st, &perm, nullptr);
       // optional CUDA events around the traversal launch (wpbr_set_kernel_timing)
       int slot = -1;
       if (e == cudaSuccess && ctx->kernel_timing && ctx->timed < wpbr_ctx::kTimedMax) {
@@ -177,16 +176,16 @@ wpbr_status trace_rays(wpbr_ctx* ctx, const float4* d_rays, uint64_t n, float4* 
           PermSrc src{d_rays, perm};
           PermHitSink4 sink{d_hits, perm};
           if (mode == WPBR_TRACE_ANY)
-            launch_traversal<true>(S, Bv, src, sink, (uint32_t)n, c, ctx->d_err.p, st);
+            launch_traversal<true>(S, Bv, src, sink, (uint32_t)n, c, ctx->d_err.p, st, 0, 1, true);
           else
-            launch_traversal<false>(S, Bv, src, sink, (uint32_t)n, c, ctx->d_err.p, st);
+            launch_traversal<false>(S, Bv, src, sink, (uint32_t)n, c, ctx->d_err.p, st, 0, 1, true);
         } else {
           BufferSrc src{d_rays};
           HitSink4 sink{d_hits};
           if (mode == WPBR_TRACE_ANY)
-            launch_traversal<true>(S, Bv, src, sink, (uint32_t)n, c, ctx->d_err.p, st);
+            launch_traversal<true>(S, Bv, src, sink, (uint32_t)n, c, ctx->d_err.p, st, 0, 1, true);
           else
-            launch_traversal<false>(S, Bv, src, sink, (uint32_t)n, c, ctx->d_err.p, st);
+            launch_traversal<false>(S, Bv, src, sink, (uint32_t)n, c, ctx->d_err.p, st, 0, 1, true);
         }
         e = cudaGetLastError();
       }

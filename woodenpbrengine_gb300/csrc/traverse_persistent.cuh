@@ -12,6 +12,9 @@
 // makes pruning more conservative — the hit is the one trace_ray returns.
 #pragma once
 
+#include <algorithm>
+#include <atomic>
+
 #include "common.cuh"
 #include "traverse.cuh"
 
@@ -205,7 +208,8 @@ __device__ __forceinline__ int pop_unpruned(const Stack& st, int& sp, float tb, 
 template <bool ANY, int STACK, bool SPH, class Src, class Sink>
 __global__ void __launch_bounds__(kPersistBlock, Sink::kMinBlocks) k_trace_persistent(SceneView S, BvhView Bv,
                                                                                            Src src, Sink sink,
-                                                                    uint32_t n, uint32_t* counter, uint32_t* err) {
+                                                                    uint32_t n, uint32_t width, uint32_t* counter,
+                                                                    uint32_t* err) {
   __shared__ SharedRay s_ray[kPersistBlock / 32][32];
   __shared__ unsigned long long s_key[kPersistBlock / 32][32];
   __shared__ uint32_t s_hprim[kPersistBlock / 32][32];  // primitive and barycentrics of s_key's hit
@@ -235,19 +239,30 @@ __global__ void __launch_bounds__(kPersistBlock, Sink::kMinBlocks) k_trace_persi
   stack_bind(stk, &s_stk_tr[0][threadIdx.x], &s_stk_c[0][threadIdx.x]);
   uint32_t rid = 0;
   bool active = false;
-  bool exhausted = false;
+  bool exhausted = lane >= width;  // a narrow warp's other lanes only help with leaf tests
   uint32_t guard = 0;
   n = src.limit(n);  // a queue source reads its length from device memory
+  // A warp's first rays follow from its place in the grid; only a batch that
+  // outlasts them fetches from the counter.
+  const uint32_t placed = gridDim.x * (kPersistBlock / 32) * width;
+  uint32_t first = (blockIdx.x * (kPersistBlock / 32) + wid) * width;
+  bool fetch = false;
 
   while (true) {
     // ---- refill idle lanes ------------------------------------------------
     __syncwarp();
     uint32_t idle = __ballot_sync(0xFFFFFFFFu, !active && !exhausted);
     if (idle && (__popc(idle) >= WPBR_REFILL_MIN || !__any_sync(0xFFFFFFFFu, active))) {
-      uint32_t leader = __ffs(idle) - 1;
-      uint32_t base = 0;
-      if (lane == leader) base = atomicAdd(counter, (uint32_t)__popc(idle));
-      base = __shfl_sync(0xFFFFFFFFu, base, leader);
+      uint32_t base = first;
+      if (fetch) {
+        base = n;  // past the end: nothing to fetch
+        if (placed < n) {
+          const uint32_t leader = __ffs(idle) - 1;
+          if (lane == leader) base = placed + atomicAdd(counter, (uint32_t)__popc(idle));
+          base = __shfl_sync(0xFFFFFFFFu, base, leader);
+        }
+      }
+      fetch = true;
       if (!active && !exhausted) {
         uint32_t r = base + __popc(idle & lt_mask);
         if (r >= n) {
@@ -547,41 +562,87 @@ struct MapSink {
 };
 
 
+// Resident blocks of one traversal kernel on the current device: the
+// occupancy query costs more than a small launch, so it is asked once per
+// kernel and device.
+template <bool ANY, int STACK, bool SPH, class Src, class Sink>
+inline unsigned resident_grid() {
+  constexpr int kDevices = 64;
+  static std::atomic<unsigned> known[kDevices];
+  const void* kern = (const void*)k_trace_persistent<ANY, STACK, SPH, Src, Sink>;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevices) return persistent_grid(kern, kPersistBlock);
+  unsigned g = known[dev].load(std::memory_order_relaxed);
+  if (!g) {
+    g = persistent_grid(kern, kPersistBlock);
+    known[dev].store(g, std::memory_order_relaxed);
+  }
+  return g;
+}
+
+// Without a cap, batches that would not give half of the resident warps 32
+// rays each are spread over them, fewer rays to a warp (the other lanes still
+// help with leaf tests): a launch of few rays lasts as long as its slowest
+// warp, which walks the union of its rays' paths. us a launch, 32 rays a warp
+// -> spread: spheres and a quad, 64 / 1,000 / 10,000 rays 27 / 35 / 35 -> 16 /
+// 17 / 24; any-hit segments on 81,920 triangles 56 / 78 / 105 -> 33 / 51 / 80;
+// benchmark rays on 1.31 M triangles 82 / 124 / 184 -> 43 / 93 / 165. Spread
+// over a quarter of the warps those are 3 to 12 % slower at 10,000 rays, over
+// all of them 65,536 rays on the spheres take 39 instead of 31 us: from there
+// on the divergent paths cost more issue slots than the shorter ones save.
+template <bool ANY, int STACK, bool SPH, class Src, class Sink>
+inline void launch_traversal_kernel(const SceneView& S, BvhView Bv, const Src& src, const Sink& sink, uint32_t n,
+                                    uint32_t* counter, uint32_t* err, cudaStream_t st, uint32_t grid_cap,
+                                    uint32_t share, bool zero_counter) {
+  constexpr uint32_t kWarps = kPersistBlock / 32;
+  const unsigned full = resident_grid<ANY, STACK, SPH, Src, Sink>();
+  unsigned g = full;
+  uint32_t width = 32;
+  if (grid_cap) {
+    g = std::min(grid_cap, full);
+  } else {
+    width = (uint32_t)std::min<uint64_t>(32u, div_up((uint64_t)n * share, (uint64_t)full * kWarps / 2));
+    g = std::min(full, div_up(n, (uint64_t)width * kWarps));
+  }
+  if (zero_counter && n > (uint64_t)g * kWarps * width) cudaMemsetAsync(counter, 0, sizeof(uint32_t), st);
+  if (Bv.stack_cap > STACK) Bv.stack_cap = STACK;
+  k_trace_persistent<ANY, STACK, SPH, Src, Sink><<<g, kPersistBlock, 0, st>>>(S, Bv, src, sink, n, width, counter, err);
+}
+
 // Launches the traversal whose stack fits the tree: a lane's stack never
 // holds more entries than the tree is deep, so trees shallower than 60
 // levels take the 64-entry kernel and deeper ones (the callers refuse depths
 // of 250 and more) the 256-entry kernel of the reference's nodesToVisit[256]
 // (SLBVH.cpp:101); grid_cap limits the persistent grid (0: one full wave of
-// resident blocks).
+// resident blocks), share is the number of launches of this size that run at
+// the same time (the branches of a pass group or a batch). n > 0. The counter must be zero when the kernel starts and
+// is used by batches larger than the grid's first rays only; zero_counter
+// clears it here when it is.
+//
+// The collide kernels are compiled without the sphere test for scenes that
+// have no spheres: its transform and quadratic beside the traversal's state
+// made them spill at 64 registers (44 B; 8.4 M rays on the triangle mesh,
+// a call: 4.162 ms with the sphere test compiled in, 3.960 without; 100,003
+// any-hit segments on 81,920 triangles 173 -> 166 us). The render passes'
+// scenes nearly always hold a sphere (light), so those keep one variant.
 template <bool ANY, class Src, class Sink>
 inline void launch_traversal(const SceneView& S, const BvhView& Bv, const Src& src, const Sink& sink, uint32_t n,
-                             uint32_t* counter, uint32_t* err, cudaStream_t st, uint32_t grid_cap = 0) {
-  auto go = [&](auto kern, uint32_t stack) {
-    unsigned full = persistent_grid((const void*)kern, kPersistBlock);
-    unsigned g = (grid_cap && grid_cap < full) ? grid_cap : full;
-    BvhView B = Bv;
-    if (B.stack_cap > stack) B.stack_cap = stack;
-    kern<<<g, kPersistBlock, 0, st>>>(S, B, src, sink, n, counter, err);
-  };
-  // The collide kernels are compiled without the sphere test for scenes that
-  // have no spheres: its transform and quadratic beside the traversal's state
-  // made them spill at 64 registers (44 B; 8.4 M rays on the triangle mesh,
-  // a call: 4.165 ms with the sphere test compiled in, 3.930 without; 100,003
-  // any-hit segments on 81,920 triangles 172 -> 166 us). The render passes'
-  // scenes nearly always hold a sphere (light), so those keep one variant.
+                             uint32_t* counter, uint32_t* err, cudaStream_t st, uint32_t grid_cap = 0,
+                             uint32_t share = 1, bool zero_counter = false) {
+  const bool shallow = Bv.max_depth < 60;
   if constexpr (Sink::kCollide) {
     if (S.ns == 0) {
-      if (Bv.max_depth < 60)
-        go(k_trace_persistent<ANY, 64, false, Src, Sink>, 64u);
+      if (shallow)
+        launch_traversal_kernel<ANY, 64, false>(S, Bv, src, sink, n, counter, err, st, grid_cap, share, zero_counter);
       else
-        go(k_trace_persistent<ANY, 256, false, Src, Sink>, 256u);
+        launch_traversal_kernel<ANY, 256, false>(S, Bv, src, sink, n, counter, err, st, grid_cap, share, zero_counter);
       return;
     }
   }
-  if (Bv.max_depth < 60)
-    go(k_trace_persistent<ANY, 64, true, Src, Sink>, 64u);
+  if (shallow)
+    launch_traversal_kernel<ANY, 64, true>(S, Bv, src, sink, n, counter, err, st, grid_cap, share, zero_counter);
   else
-    go(k_trace_persistent<ANY, 256, true, Src, Sink>, 256u);
+    launch_traversal_kernel<ANY, 256, true>(S, Bv, src, sink, n, counter, err, st, grid_cap, share, zero_counter);
 }
 
 }  // namespace wpbr
