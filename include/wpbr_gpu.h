@@ -132,7 +132,7 @@ enum wpbr_trace_mode { WPBR_TRACE_CLOSEST = 0, WPBR_TRACE_ANY = 1 };
 WPBR_API wpbr_status wpbr_collide(wpbr_ctx* ctx, const float* rays, uint64_t n, float* hits, uint32_t mode);
 WPBR_API wpbr_status wpbr_collide_device(wpbr_ctx* ctx, const void* d_rays, uint64_t n, void* d_hits,
                                          uint32_t mode);
-/* Large batches (256k rays and more) are traced in the order of their
+/* Large batches (512k rays and more) are traced in the order of their
  * origins' Morton cells on a 2^b per axis grid over the scene bounds
  * (b = bits_per_axis, default 8, at most 10) and written back at their input
  * positions; the hits do not depend on the order. 0 traces in input order. */
@@ -331,7 +331,7 @@ WPBR_API wpbr_status wpbr_adjoint_backward_device(wpbr_ctx* ctx, float* d_grad_m
  * Applies to later launches (pass graphs are recaptured). */
 WPBR_API wpbr_status wpbr_set_traversal_limits(wpbr_ctx* ctx, uint32_t max_stack_entries, uint32_t max_loop_steps);
 /* The order wpbr_collide traces a batch of n rays in when it sorts them
- * (batches of 2^18 rays and more, wpbr_set_ray_sort > 0): keys[i] is the
+ * (batches of 2^19 rays and more, wpbr_set_ray_sort > 0): keys[i] is the
  * Morton code of ray i's origin cell (3 x bits-per-axis bits over the scene
  * bounds) and perm[j] the input index of the j-th ray traced, a stable sort of
  * the keys. rays as for wpbr_collide (host); any n below 2^32 - 1. */

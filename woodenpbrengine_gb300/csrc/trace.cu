@@ -9,7 +9,13 @@ namespace wpbr {
 
 namespace {
 
-constexpr uint64_t kRaySortMin = 1u << 18;  // batches below this are traced in input order
+// Batches below this are traced in input order: the sort (13 launches) costs
+// more than the order saves. us a call sorted / in input order, 262,144 rays:
+// benchmark rays on 1.31 M triangles 395 / 359, any-hit segments 390 / 354,
+// rays aimed from outside 385 / 318. At 524,288 it is still 6 to 15 % behind, at
+// 4 M even, and at 8.4 M ahead for rays off the surface (segments 4.11 / 4.40
+// ms, benchmark rays 3.93 / 4.00).
+constexpr uint64_t kRaySortMin = 1u << 19;
 
 template <bool ANY, bool STATS, int STACK>
 __global__ void __launch_bounds__(128) k_trace(SceneView S, BvhView Bv, const float4* __restrict__ rays, uint64_t n,
