@@ -450,7 +450,7 @@ __global__ void k_adj_loss(uint32_t n, const float4* acc, const float* target, f
   }
 }
 
-// Map function cells -> texel green channel, through k_env_lum's lookups:
+// Map function cells -> texel green channel, through k_env_rows' lookups:
 // func[i] = green(bilerp(x/W, y/H)) * sin(theta_y); every cell also carries
 // dLoss/dZ * dZ/dfunc = g_Z / (W H).
 __global__ void k_adj_env_finish(EnvView e, uint32_t quirks, const float* g_func, const double* g_Z, float* g_env) {
@@ -492,12 +492,6 @@ __global__ void k_apply_mat_params(const float* prm, uint32_t nmat, wpbr_materia
     d.eta_t[c] = p[4 + c];
     d.k[c] = p[7 + c];
   }
-}
-
-__global__ void k_env_to_rgb4(const float* prm, uint32_t n, float4* rgb) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  rgb[i] = make_float4(prm[3 * (size_t)i], prm[3 * (size_t)i + 1], prm[3 * (size_t)i + 2], 0.0f);
 }
 
 __global__ void k_mat_grad_out(const double* g, uint32_t n, float* out) {
@@ -694,8 +688,7 @@ wpbr_status adjoint_set_params(wpbr_ctx* ctx, const float* mat, const float* env
       WPBR_CUDA(cudaMemcpyAsync(J.env_prm.p, env, sizeof(float) * 3 * J.n_texels, cudaMemcpyHostToDevice, st));
       src = J.env_prm.p;
     }
-    k_env_to_rgb4<<<div_up(J.n_texels, 256), 256, 0, st>>>(src, (uint32_t)J.n_texels, J.rgb_e.p);
-    WPBR_CUDA(cudaGetLastError());
+    WPBR_CUDA(rgb_to_texels(src, J.n_texels, J.rgb_e.p, st));
     wpbr_status s = rebuild_eval_distribution(ctx);
     if (s != WPBR_OK) return s;
   }

@@ -212,7 +212,8 @@ struct wpbr_ctx {
   bool env_lights_only = false;
   int envW = 0, envH = 0;
   wpbr::DevBuf<float4> env_rgb;
-  wpbr::DevBuf<float> cond_func, cond_cdf, cond_int, marg_func, marg_cdf, marg_int, env_lum;
+  wpbr::DevBuf<float> cond_func, cond_cdf, cond_int, marg_func, marg_cdf, marg_int;
+  wpbr::DevBuf<float> env_raw;  // the uploaded RGB texels, three floats each
   wpbr::Xf env_l2w, env_w2l;
   wpbr::RGB3 env_le{1, 1, 1};
   float env_marg_int = 0.0f;
@@ -285,6 +286,8 @@ cudaError_t radix_sort_pairs(uint32_t* k0, uint32_t* v0, uint32_t* k1, uint32_t*
 wpbr_status trace_rays(wpbr_ctx* ctx, const float4* d_rays, uint64_t n, float4* d_hits, uint32_t mode,
                        uint32_t* d_stats, int scratch = 0, cudaStream_t stream = nullptr);
 wpbr_status env_preprocess(wpbr_ctx* ctx);
+// n RGB texels (three floats each, device memory) as float4 texels.
+cudaError_t rgb_to_texels(const float* d_rgb, uint64_t n, float4* d_out, cudaStream_t st);
 // Distribution2D of an environment image (JobLightInfiniteAreaPreprocessSampling)
 // into caller-owned arrays: cond_func/cond_cdf/cond_int of H rows of W, marg_* of H.
 struct EnvDist {
