@@ -1,6 +1,7 @@
 // context.cu — the C ABI (include/wpbr_gpu.h): context lifetime, scene
 // upload, BVH build/export, collision, rendering entry points.
 #include <cuda_runtime.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <cmath>
@@ -118,6 +119,27 @@ void gauss_table(float* w) {
   }
 }
 
+}  // namespace
+
+namespace wpbr {
+void touch_pages(void* host, size_t bytes) {
+  if (!host || !bytes) return;
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, host) != cudaSuccess || at.type != cudaMemoryTypeUnregistered) {
+    cudaGetLastError();  // page-locked or managed memory (or no host memory: the copy will say)
+    return;
+  }
+  static const size_t page = [] {
+    const long v = sysconf(_SC_PAGESIZE);
+    return v > 0 ? (size_t)v : (size_t)4096;
+  }();
+  volatile unsigned char* p = (volatile unsigned char*)host;
+  for (size_t i = 0; i < bytes; i += page) p[i] = p[i];
+  p[bytes - 1] = p[bytes - 1];
+}
+}  // namespace wpbr
+
+namespace {
 template <typename T>
 cudaError_t upload(DevBuf<T>& d, const T* h, size_t n, cudaStream_t s) {
   cudaError_t e = d.ensure(n);
@@ -633,6 +655,7 @@ static wpbr_status collide_pipelined(wpbr_ctx* ctx, const float* rays, uint64_t 
   // copies already queued read `rays` and write `hits`, so all four streams
   // are drained before the call returns, whatever happened.
   wpbr_status s = WPBR_OK;
+  bool touched = false;
   cudaError_t ce = cudaSuccess;
   const char* what = "collide";
   for (int i = 0; i < 4; ++i) {
@@ -650,6 +673,8 @@ static wpbr_status collide_pipelined(wpbr_ctx* ctx, const float* rays, uint64_t 
     if (s != WPBR_OK) break;
     ce = cudaEventRecord(ctx->io_ev[1], cs);
     if (ce == cudaSuccess) ce = cudaStreamWaitEvent(ctx->io_d2h, ctx->io_ev[1], 0);
+    if (!touched) touch_pages(hits, 16 * n);  // while the first chunk is traced
+    touched = true;
     if (ce == cudaSuccess)
       ce = cudaMemcpyAsync(hits + 4 * off, ctx->io_hits.p + off, 16 * c, cudaMemcpyDeviceToHost, ctx->io_d2h);
     if (ce != cudaSuccess) {
@@ -681,6 +706,7 @@ static wpbr_status collide_host(wpbr_ctx* ctx, const float* rays, uint64_t n, fl
   WPBR_CUDA(cudaMemcpyAsync(ctx->io_rays.p, rays, 32 * n, cudaMemcpyHostToDevice, st));
   wpbr_status s = trace_rays(ctx, ctx->io_rays.p, n, ctx->io_hits.p, mode, stats ? ctx->io_stats.p : nullptr);
   if (s != WPBR_OK) return s;
+  touch_pages(hits, 16 * n);  // while the rays are traced
   WPBR_CUDA(cudaMemcpyAsync(hits, ctx->io_hits.p, 16 * n, cudaMemcpyDeviceToHost, st));
   if (stats) WPBR_CUDA(cudaMemcpyAsync(stats, ctx->io_stats.p, 8 * n, cudaMemcpyDeviceToHost, st));
   WPBR_CUDA(cudaStreamSynchronize(st));
@@ -746,23 +772,7 @@ WPBR_API wpbr_status wpbr_render(wpbr_ctx* ctx) {
 
 WPBR_API wpbr_status wpbr_film_read(wpbr_ctx* ctx, float* acc_L, float* acc_w) {
   if (!ctx) return WPBR_ERR_INVALID_ARG;
-  RenderState& R = ctx->rs;
-  if (!R.ready) return set_err(ctx, WPBR_ERR_NOT_BUILT, "film_read: render_setup not called");
-  wpbr_status rs = spectral_resolve(ctx);
-  if (rs != WPBR_OK) return rs;
-  size_t n = (size_t)R.W * R.H;
-  std::vector<float> a(n * 4);
-  WPBR_CUDA(cudaMemcpyAsync(a.data(), R.acc.p, sizeof(float) * 4 * n, cudaMemcpyDeviceToHost, ctx->stream));
-  WPBR_CUDA(cudaStreamSynchronize(ctx->stream));
-  for (size_t i = 0; i < n; ++i) {
-    if (acc_L) {
-      acc_L[3 * i] = a[4 * i];
-      acc_L[3 * i + 1] = a[4 * i + 1];
-      acc_L[3 * i + 2] = a[4 * i + 2];
-    }
-    if (acc_w) acc_w[i] = a[4 * i + 3];
-  }
-  return WPBR_OK;
+  return film_read(ctx, acc_L, acc_w);
 }
 
 WPBR_API wpbr_status wpbr_film_tonemap(wpbr_ctx* ctx, uint8_t* rgb8) {
