@@ -2420,9 +2420,7 @@ __global__ void k_node2(const uint32_t* info, const uint32_t* lin_node, const fl
     }
   }
   Node2 nd;
-  nd.b0 = make_float4(b[0][0], b[0][3], b[0][1], b[0][4]);
-  nd.b1 = make_float4(b[1][0], b[1][3], b[1][1], b[1][4]);
-  nd.bz = make_float4(b[0][2], b[0][5], b[1][2], b[1][5]);
+  node2_set_boxes(nd, b[0], b[1]);
   nd.meta = make_int4(ref[0], ref[1], (int)cnt[0], (int)((lin_node[(size_t)i * 3 + 2] << 30) | (cnt[1] & 0x3FFFFFFFu)));
   const uint32_t at = slot[int_index[i]];
   out[at] = nd;
@@ -2586,9 +2584,7 @@ __global__ void k_split_emit(const uint32_t* info, const uint32_t* is_int, const
       }
     }
     Node2 nd;
-    nd.b0 = make_float4(b[0][0], b[0][3], b[0][1], b[0][4]);
-    nd.b1 = make_float4(b[1][0], b[1][3], b[1][1], b[1][4]);
-    nd.bz = make_float4(b[0][2], b[0][5], b[1][2], b[1][5]);
+    node2_set_boxes(nd, b[0], b[1]);
     nd.meta = make_int4(cref[0], cref[1], (int)ccnt[0], (int)((3u << 30) | ccnt[1]));
     out[base + h] = nd;
   }

@@ -97,12 +97,12 @@ __device__ HitRec trace_ray(const SceneView& S, const BvhView& Bv, V3 o, V3 d, f
         break;
       }
       const Node2* np_ = Bv.nodes + ref;
-      float4 b0 = __ldg(&np_->b0), b1 = __ldg(&np_->b1), bz = __ldg(&np_->bz);
+      float4 bx = __ldg(&np_->bx), by = __ldg(&np_->by), bz = __ldg(&np_->bz);
       int4 m = __ldg(&np_->meta);
       nv += 2;
       float t0, t1;
-      bool h0 = slab_test(V3{b0.x, b0.z, bz.x}, V3{b0.y, b0.w, bz.y}, o, inv, neg, tmax, &t0) && !(t0 > tb * kPruneScale);
-      bool h1 = slab_test(V3{b1.x, b1.z, bz.z}, V3{b1.y, b1.w, bz.w}, o, inv, neg, tmax, &t1) && !(t1 > tb * kPruneScale);
+      bool h0 = slab_test(V3{bx.x, by.x, bz.x}, V3{bx.z, by.z, bz.z}, o, inv, neg, tmax, &t0) && !(t0 > tb * kPruneScale);
+      bool h1 = slab_test(V3{bx.y, by.y, bz.y}, V3{bx.w, by.w, bz.w}, o, inv, neg, tmax, &t1) && !(t1 > tb * kPruneScale);
       uint32_t axis = ((uint32_t)m.w) >> 30;
       uint32_t c0n = (uint32_t)m.z, c1n = ((uint32_t)m.w) & 0x3FFFFFFFu;
       if (h0 && h1) {

@@ -93,6 +93,92 @@ __device__ __forceinline__ float prim_test_shared(const SceneView& S, const floa
   return t;
 }
 
+// ---- box tests of one node ---------------------------------------------------
+// slab_test's decision for both children with fewer instructions, for rays
+// whose plane distances cannot be NaN (origin and reciprocal direction finite,
+// |origin| <= 2^100, no reciprocal zero). Then, per axis, the smaller product
+// is the one slab_test selects by the direction's sign; slab_test's comparisons
+// amount to max(entries) <= min(exits), because an axis's own entry and exit
+// are in order wherever the scaled exit is positive; scaling the smallest exit
+// is scaling each (rounding is monotonic); and the ray's own tmax and the
+// best hit so far are one limit L: entry < tmax is entry <= the float below
+// tmax. The subtractions and products are the same IEEE operations, two lanes
+// (the two children) to an instruction; no multiply-add can form, as each
+// product follows a subtraction. Every decision and every entry distance equals
+// slab_test's, except that an entry of zero may carry either sign.
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(uint64_t v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ float2 plane2(uint64_t planes, uint64_t o2, uint64_t inv2) {
+  uint64_t d, t;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(planes), "l"(o2));
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(t) : "l"(d), "l"(inv2));
+  return unpack2(t);
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ float min3(float a, float b, float c) {
+  float r;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+constexpr float kLeastPositive = 0x1p-149f;
+struct RayBox {
+  uint64_t ox, oy, oz, ix, iy, iz;  // origin and reciprocal direction, each twice
+};
+struct BoxPair {
+  float t0, t1;  // entry distances
+  bool h0, h1;
+};
+__device__ __forceinline__ BoxPair box_pair_test(const float4& bx, const float4& by, const float4& bz,
+                                                 const RayBox& R, float L) {
+  const float2 ax = plane2(pack2(bx.x, bx.y), R.ox, R.ix), cx = plane2(pack2(bx.z, bx.w), R.ox, R.ix);
+  const float2 ay = plane2(pack2(by.x, by.y), R.oy, R.iy), cy = plane2(pack2(by.z, by.w), R.oy, R.iy);
+  const float2 az = plane2(pack2(bz.x, bz.y), R.oz, R.iz), cz = plane2(pack2(bz.z, bz.w), R.oz, R.iz);
+  BoxPair r;
+  r.t0 = max3(fminf(ax.x, cx.x), fminf(ay.x, cy.x), fminf(az.x, cz.x));
+  r.t1 = max3(fminf(ax.y, cx.y), fminf(ay.y, cy.y), fminf(az.y, cz.y));
+  const float e0 = min3(fmaxf(ax.x, cx.x), fmaxf(ay.x, cy.x), fmaxf(az.x, cz.x)) * kSlabScale;
+  const float e1 = min3(fmaxf(ax.y, cx.y), fmaxf(ay.y, cy.y), fmaxf(az.y, cz.y)) * kSlabScale;
+  // entry <= exit, entry <= L and exit > 0 (with L > 0)
+  r.h0 = fmaxf(r.t0, kLeastPositive) <= fminf(e0, L);
+  r.h1 = fmaxf(r.t1, kLeastPositive) <= fminf(e1, L);
+  return r;
+}
+// The same for any ray, by slab_test_flat itself, out of line.
+static __device__ __noinline__ BoxPair box_pair_any(const Node2* np, float ox, float oy, float oz, float ix, float iy,
+                                                    float iz, float L) {
+  const float4 bx = __ldg(&np->bx), by = __ldg(&np->by), bz = __ldg(&np->bz);
+  const V3 o{ox, oy, oz}, inv{ix, iy, iz};
+  const int neg[3] = {inv.x < 0.0f, inv.y < 0.0f, inv.z < 0.0f};
+  BoxPair r;
+  r.h0 = slab_test_flat(V3{bx.x, by.x, bz.x}, V3{bx.z, by.z, bz.z}, o, inv, neg, inf_(), &r.t0) && r.t0 <= L;
+  r.h1 = slab_test_flat(V3{bx.y, by.y, bz.y}, V3{bx.w, by.w, bz.w}, o, inv, neg, inf_(), &r.t1) && r.t1 <= L;
+  return r;
+}
+// Whether box_pair_test takes this ray.
+__device__ __forceinline__ bool box_pair_ok(V3 o, V3 inv) {
+  auto in = [](float v, float lo, float hi) { return fabsf(v) >= lo && fabsf(v) <= hi; };
+  return in(o.x, 0.0f, 0x1p100f) && in(o.y, 0.0f, 0x1p100f) && in(o.z, 0.0f, 0x1p100f) &&
+         in(inv.x, kLeastPositive, FLT_MAX) && in(inv.y, kLeastPositive, FLT_MAX) &&
+         in(inv.z, kLeastPositive, FLT_MAX);
+}
+// The limit on entry distances of an unbounded or bounded ray before its
+// first hit; a tmax that no hit can lie below admits no box.
+__device__ __forceinline__ float entry_limit(float tmax) {
+  return tmax > 0.0f ? __uint_as_float(__float_as_uint(tmax) - 1u) : -1.0f;
+}
+
 // Traversal stack of one lane: the far children pushed on the way down, with
 // their leaf counts and entry distances. The collide kernels (Sink::kCollide)
 // keep (entry distance, ref) in one 8-byte word, so testing a popped entry
@@ -196,11 +282,11 @@ __device__ __forceinline__ void stack_bind(TravStack<STACK, PACKED>&, unsigned l
 // Pops until an entry whose entry distance does not exceed the best hit by
 // more than the pruning margin; kEnd when the stack runs out.
 template <class Stack>
-__device__ __forceinline__ int pop_unpruned(const Stack& st, int& sp, float tb, uint32_t* cnt) {
+__device__ __forceinline__ int pop_unpruned(const Stack& st, int& sp, float limit, uint32_t* cnt) {
   int r = kEnd;
   while (sp > 0) {
     --sp;
-    if (st.take(sp, tb * kPruneScale, &r, cnt)) return r;
+    if (st.take(sp, limit, &r, cnt)) return r;
   }
   return kEnd;
 }
@@ -220,9 +306,10 @@ __global__ void __launch_bounds__(kPersistBlock, Sink::kMinBlocks) k_trace_persi
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t wid = threadIdx.x >> 5;
   const uint32_t lt_mask = (1u << lane) - 1u;
-  V3 o{0, 0, 0}, inv{0, 0, 0};
-  int neg[3] = {0, 0, 0};
-  float tmax = 0.0f, tb = 0.0f;
+  RayBox rb{0, 0, 0, 0, 0, 0};
+  uint32_t near1 = 0;   // bit a: the second child of a split along axis a comes first (bit 3 clear: axis code 3)
+  bool plain = true;    // box_pair_test takes the ray
+  float tb = 0.0f, L = 0.0f;  // best hit; largest entry distance of a box worth visiting
   // The render passes' kernels keep the hit record the cooperative leaf
   // tests leave in shared memory; the collide kernels keep only the winning
   // primitive's sorted position and test it once more when the ray is done
@@ -271,13 +358,16 @@ __global__ void __launch_bounds__(kPersistBlock, Sink::kMinBlocks) k_trace_persi
           rid = r;
           float4 ro, rd;
           src.load(r, &ro, &rd);
-          o = V3{ro.x, ro.y, ro.z};
+          const V3 o{ro.x, ro.y, ro.z};
           const V3 d{rd.x, rd.y, rd.z};
-          tmax = rd.w;
-          inv = V3{1.0f / d.x, 1.0f / d.y, 1.0f / d.z};
-          neg[0] = inv.x < 0.0f;
-          neg[1] = inv.y < 0.0f;
-          neg[2] = inv.z < 0.0f;
+          const float tmax = rd.w;
+          const V3 inv{1.0f / d.x, 1.0f / d.y, 1.0f / d.z};
+          const int neg[3] = {inv.x < 0.0f, inv.y < 0.0f, inv.z < 0.0f};
+          near1 = (neg[0] ? 1u : 0u) | (neg[1] ? 2u : 0u) | (neg[2] ? 4u : 0u);
+          plain = box_pair_ok(o, inv);
+          rb = RayBox{pack2(o.x, o.x),     pack2(o.y, o.y),     pack2(o.z, o.z),
+                      pack2(inv.x, inv.x), pack2(inv.y, inv.y), pack2(inv.z, inv.z)};
+          L = entry_limit(tmax);
           RayTri R = ray_tri_setup(o, d, S.quirks);
           SharedRay& sr = s_ray[wid][lane];
           uint32_t kpack =
@@ -317,16 +407,16 @@ __global__ void __launch_bounds__(kPersistBlock, Sink::kMinBlocks) k_trace_persi
           break;
         }
         const Node2* np_ = Bv.nodes + ref;
-        float4 b0 = __ldg(&np_->b0), b1 = __ldg(&np_->b1), bz = __ldg(&np_->bz);
-        int4 m = __ldg(&np_->meta);
-        float t0, t1;
-        float tbs = tb * kPruneScale;
-        bool h0 = slab_test_flat(V3{b0.x, b0.z, bz.x}, V3{b0.y, b0.w, bz.y}, o, inv, neg, tmax, &t0) && !(t0 > tbs);
-        bool h1 = slab_test_flat(V3{b1.x, b1.z, bz.z}, V3{b1.y, b1.w, bz.w}, o, inv, neg, tmax, &t1) && !(t1 > tbs);
+        const int4 m = __ldg(&np_->meta);
+        const BoxPair bp = plain ? box_pair_test(__ldg(&np_->bx), __ldg(&np_->by), __ldg(&np_->bz), rb, L)
+                                 : box_pair_any(np_, unpack2(rb.ox).x, unpack2(rb.oy).x, unpack2(rb.oz).x,
+                                                unpack2(rb.ix).x, unpack2(rb.iy).x, unpack2(rb.iz).x, L);
+        const float t0 = bp.t0, t1 = bp.t1;
+        const bool h0 = bp.h0, h1 = bp.h1;
         uint32_t axis = ((uint32_t)m.w) >> 30;
         uint32_t c0n = (uint32_t)m.z, c1n = ((uint32_t)m.w) & 0x3FFFFFFFu;
         if (h0 && h1) {
-          bool first1 = second_child_first(neg, axis);
+          const bool first1 = (near1 >> axis) & 1u;
           if ((uint32_t)sp >= Bv.stack_cap) {  // stack_cap <= STACK (launch_traversal clamps it)
             atomicOr(err, kErrStackOverflow);
             ref = kEnd;
@@ -345,13 +435,13 @@ __global__ void __launch_bounds__(kPersistBlock, Sink::kMinBlocks) k_trace_persi
           ref = m.y;
           cnt = c1n;
         } else {
-          ref = pop_unpruned(stk, sp, tb, &cnt);
+          ref = pop_unpruned(stk, sp, L, &cnt);
         }
         // postpone the first leaf found, keep descending for the next one
         if (ref < 0 && ref != kEnd && lref == kEnd) {
           lref = ref;
           lcnt = cnt;
-          ref = pop_unpruned(stk, sp, tb, &cnt);
+          ref = pop_unpruned(stk, sp, L, &cnt);
         }
         if (!__any_sync(__activemask(), lref == kEnd)) break;
       }
@@ -359,7 +449,7 @@ __global__ void __launch_bounds__(kPersistBlock, Sink::kMinBlocks) k_trace_persi
       if (lref == kEnd && ref < 0 && ref != kEnd) {
         lref = ref;
         lcnt = cnt;
-        ref = pop_unpruned(stk, sp, tb, &cnt);
+        ref = pop_unpruned(stk, sp, L, &cnt);
       }
     }
 
@@ -449,6 +539,7 @@ __global__ void __launch_bounds__(kPersistBlock, Sink::kMinBlocks) k_trace_persi
               h = HitRec{t, s_hprim[wid][lane], bb.x, bb.y};
             }
             tb = t;
+            L = fminf(L, t * kPruneScale);
             if (ANY) done_any = true;
           }
         }
@@ -462,14 +553,14 @@ __global__ void __launch_bounds__(kPersistBlock, Sink::kMinBlocks) k_trace_persi
         } else if (ref < 0 && ref != kEnd) {  // next node is a leaf too: test it in the next round
           lref = ref;
           lcnt = cnt;
-          ref = pop_unpruned(stk, sp, tb, &cnt);
+          ref = pop_unpruned(stk, sp, L, &cnt);
         }
       }
     }
     if (active && ref == kEnd && lref == kEnd) {
       if (Sink::kCollide && hpos != kNoHit) {
         const float4 dd = s_ray[wid][lane].d;
-        const V3 d{dd.x, dd.y, dd.z};
+        const V3 o{unpack2(rb.ox).x, unpack2(rb.oy).x, unpack2(rb.oz).x}, d{dd.x, dd.y, dd.z};
         RayTri R = ray_tri_setup(o, d, S.quirks);
         uint32_t prim;
         float b1, b2;

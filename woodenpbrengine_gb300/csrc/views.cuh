@@ -42,12 +42,20 @@ struct SceneView {
 // top two bits of cnt1 (the parent's split axis, for near-first order);
 // axis code 3 marks the records of the leaf-split layout that subdivide one
 // large leaf of the reference's tree: child 0 (the lower positions) first.
+// Axis by axis, the two children's planes side by side, so that one 16-byte
+// load gives the operands of the two-lane FP32 instructions (box_pair_test).
 struct __align__(16) Node2 {
-  float4 b0;   // c0 lo.x hi.x lo.y hi.y
-  float4 b1;   // c1 lo.x hi.x lo.y hi.y
-  float4 bz;   // c0 lo.z hi.z, c1 lo.z hi.z
+  float4 bx;   // lo.x of c0, c1; hi.x of c0, c1
+  float4 by;
+  float4 bz;
   int4 meta;   // ref0, ref1, cnt0, (axis<<30)|cnt1
 };
+// Boxes of the children as {lo.xyz, hi.xyz}.
+WPBR_HD void node2_set_boxes(Node2& nd, const float c0[6], const float c1[6]) {
+  nd.bx = make_float4(c0[0], c1[0], c0[3], c1[3]);
+  nd.by = make_float4(c0[1], c1[1], c0[4], c1[4]);
+  nd.bz = make_float4(c0[2], c1[2], c0[5], c1[5]);
+}
 
 struct BvhView {
   const Node2* nodes;    // the layout traversed (leaf-split by default)
