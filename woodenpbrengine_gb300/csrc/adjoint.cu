@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(kTB, WPBR_ADJ_SPAWN_MIN_BLOCKS) k_adj_spawn(Pa
   uint32_t li_idx = pick_light(P, pix, pass);
   const wpbr_light& lt = P.S.lights[li_idx];
   float u0, u1;
-  wpbr_rng::sample2d(P.rs, pix, pass, wpbr_rng::DIM_LIGHT, &u0, &u1);
+  sample2d(P.rs, pix, pass, wpbr_rng::DIM_LIGHT, &u0, &u1);
   V3 wi{0, 0, 0};
   RGB3 li = rgb1(0.0f);
   float lpdf = 0.0f;
@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(kTB, WPBR_ADJ_SPAWN_MIN_BLOCKS) k_adj_spawn(Pa
   const bool trace_l = ok && !rblack(li);
   if (trace_l) flags |= AF_TRACE_L;
   sq.push(trace_l, 2 * pix, add(s.p, mul(wi, (float)0.1)), wi);
-  wpbr_rng::sample2d(P.rs, pix, pass, wpbr_rng::DIM_BSDF, &u0, &u1);
+  sample2d(P.rs, pix, pass, wpbr_rng::DIM_BSDF, &u0, &u1);
   V3 bwi_l;
   float bpdf;
   bool valid;
@@ -529,14 +529,9 @@ AdjView adj_view(const wpbr_ctx* ctx) {
 }
 
 PassCtx adj_pass_ctx(wpbr_ctx* ctx) {
-  PassCtx P;
-  P.S = scene_view(ctx);
-  P.Bv = render_traversal_view(ctx);
-  P.rs = wpbr_rng::Stream{ctx->adj.seed, ctx->adj.stream, ctx->adj.spp, (ctx->quirks & WPBR_Q_REF_SAMPLER_ARRAYS) ? 1u : 0u};
-  P.W = ctx->adj.W;
-  P.H = ctx->adj.H;
-  P.err = ctx->d_err.p;
-  return P;
+  return pass_ctx(scene_view(ctx), render_traversal_view(ctx),
+                  wpbr_rng::Stream{ctx->adj.seed, ctx->adj.stream, ctx->adj.spp, (ctx->quirks & WPBR_Q_REF_SAMPLER_ARRAYS) ? 1u : 0u},
+                  ctx->adj.W, ctx->adj.H, ctx->d_err.p);
 }
 
 wpbr_status rebuild_eval_distribution(wpbr_ctx* ctx) {

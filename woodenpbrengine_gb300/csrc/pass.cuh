@@ -6,6 +6,7 @@
 
 #include "camera.cuh"
 #include "common.cuh"
+#include "sampler.cuh"
 #include "shade.cuh"
 #include "views.cuh"
 #include "wpbr_sampling.h"
@@ -43,10 +44,15 @@ constexpr int kTB = 128;
 struct PassCtx {
   SceneView S;
   BvhView Bv;
-  wpbr_rng::Stream rs;
+  Sampler rs;
   uint32_t W, H;
+  FastDiv row;  // by W
   uint32_t* err;
 };
+inline PassCtx pass_ctx(const SceneView& S, const BvhView& Bv, wpbr_rng::Stream rs, uint32_t W, uint32_t H,
+                        uint32_t* err) {
+  return PassCtx{S, Bv, make_sampler(rs), W, H, fast_div(W), err};
+}
 
 __device__ __forceinline__ V3 ld3(const float* f, uint32_t i) { return V3{f[3 * i], f[3 * i + 1], f[3 * i + 2]}; }
 __device__ __forceinline__ void st3(float* f, uint32_t i, V3 v) {
@@ -198,17 +204,12 @@ __device__ __forceinline__ wpbr_material metal_unpack(float4 v) {
   return e;
 }
 
-__device__ __forceinline__ void pixel_xy(uint32_t pix, uint32_t W, uint32_t* x, uint32_t* y) {
-  *x = pix % W;
-  *y = pix / W;
-}
-
 // JobSamplerUpdateCameraSamples (CSSampler.cpp:7-23): pFilm = pixel + u2
 __device__ __forceinline__ void camera_sample(const PassCtx& P, uint32_t pix, uint32_t pass, float* fx, float* fy) {
-  uint32_t x, y;
-  pixel_xy(pix, P.W, &x, &y);
+  uint32_t x;
+  const uint32_t y = div_mod(pix, P.row, &x);
   float u0, u1;
-  wpbr_rng::sample2d(P.rs, pix, pass, wpbr_rng::DIM_CAMERA, &u0, &u1);
+  sample2d(P.rs, pix, pass, wpbr_rng::DIM_CAMERA, &u0, &u1);
   *fx = (float)x + u0;
   *fy = (float)y + u1;
 }
@@ -216,7 +217,8 @@ __device__ __forceinline__ void camera_sample(const PassCtx& P, uint32_t pix, ui
 // JobScatteringSampleLight (SScattering.cpp:82-88), index clamped
 __device__ __forceinline__ uint32_t pick_light(const PassCtx& P, uint32_t pix, uint32_t pass) {
   uint32_t nl = P.S.nlights;
-  float ul = wpbr_rng::sample1d(P.rs, pix, pass, wpbr_rng::DIM_LIGHT_PICK);
+  if (nl == 1) return 0;  // whatever the sample
+  float ul = sample1d(P.rs, pix, pass, wpbr_rng::DIM_LIGHT_PICK);
   float fl = (ul + 0.5f) * (float)(nl - 1);
   uint32_t li = (uint32_t)fl;
   return li > nl - 1 ? nl - 1 : li;
@@ -230,7 +232,7 @@ struct LightSample {
 };
 __device__ LightSample sample_light(const PassCtx& P, const wpbr_light& lt, V3 p, uint32_t pix, uint32_t pass) {
   float u0, u1;
-  wpbr_rng::sample2d(P.rs, pix, pass, wpbr_rng::DIM_LIGHT, &u0, &u1);
+  sample2d(P.rs, pix, pass, wpbr_rng::DIM_LIGHT, &u0, &u1);
   LightSample s;
   s.wi = V3{0, 0, 0};
   s.li = rgb1(0.0f);

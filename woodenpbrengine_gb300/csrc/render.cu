@@ -188,7 +188,7 @@ __global__ void kj_sample_bsdf(PassCtx P, uint32_t pass, Staged G) {
   Frame fr = load_frame(G.f[F_FRAME], pix);
   wpbr_material m = staged_material(P, G, pix);
   float u0, u1;
-  wpbr_rng::sample2d(P.rs, pix, pass, wpbr_rng::DIM_BSDF, &u0, &u1);
+  sample2d(P.rs, pix, pass, wpbr_rng::DIM_BSDF, &u0, &u1);
   V3 wi_l;
   float pdf;
   bool valid;
@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(kTB, TEX ? WPBR_SPAWN_TEX_MIN_BLOCKS : WPBR_SP
   if (trace_l) flags |= SF_TRACE_L;
   sq.push(trace_l, 2 * pix, add(s.p, mul(ls.wi, (float)0.1)), ls.wi);
   float u0, u1;
-  wpbr_rng::sample2d(P.rs, pix, pass, wpbr_rng::DIM_BSDF, &u0, &u1);
+  sample2d(P.rs, pix, pass, wpbr_rng::DIM_BSDF, &u0, &u1);
   V3 bwi_l;
   float bpdf;
   bool valid;
@@ -491,14 +491,9 @@ __global__ void k_film_split(uint32_t n, const float4* acc, float* L, float* w) 
 }
 
 PassCtx make_pass_ctx(wpbr_ctx* ctx) {
-  PassCtx P;
-  P.S = scene_view(ctx);
-  P.Bv = render_traversal_view(ctx);
-  P.rs = wpbr_rng::Stream{ctx->rs.seed, ctx->rs.stream, ctx->rs.spp, (ctx->quirks & WPBR_Q_REF_SAMPLER_ARRAYS) ? 1u : 0u};
-  P.W = ctx->rs.W;
-  P.H = ctx->rs.H;
-  P.err = ctx->d_err.p;
-  return P;
+  return pass_ctx(scene_view(ctx), render_traversal_view(ctx),
+                  wpbr_rng::Stream{ctx->rs.seed, ctx->rs.stream, ctx->rs.spp, (ctx->quirks & WPBR_Q_REF_SAMPLER_ARRAYS) ? 1u : 0u},
+                  ctx->rs.W, ctx->rs.H, ctx->d_err.p);
 }
 
 Staged staged_view(wpbr_ctx* ctx) {

@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(kTB, TEX ? WPBR_SPAWN_TEX_MIN_BLOCKS : WPBR_SP
   // the environment lookup at the sampled (s, t); without the fix the
   // environment branch's Li is black and nothing is traced
   float u0, u1;
-  wpbr_rng::sample2d(P.rs, pix, pass, wpbr_rng::DIM_LIGHT, &u0, &u1);
+  sample2d(P.rs, pix, pass, wpbr_rng::DIM_LIGHT, &u0, &u1);
   V3 wi{0, 0, 0};
   float lpdf = 0.0f;
   bool ok = true, li_possible = true;
@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(kTB, TEX ? WPBR_SPAWN_TEX_MIN_BLOCKS : WPBR_SP
     }
   }
   // ---- BSDF-sampling branch
-  wpbr_rng::sample2d(P.rs, pix, pass, wpbr_rng::DIM_BSDF, &u0, &u1);
+  sample2d(P.rs, pix, pass, wpbr_rng::DIM_BSDF, &u0, &u1);
   V3 wi_l;
   float bpdf = 0.0f;
   bool valid;
@@ -619,14 +619,9 @@ wpbr_status spectral_setup(wpbr_ctx* ctx) {
 }
 
 static PassCtx spec_pass_ctx(wpbr_ctx* ctx) {
-  PassCtx P;
-  P.S = scene_view(ctx);
-  P.Bv = render_traversal_view(ctx);
-  P.rs = wpbr_rng::Stream{ctx->rs.seed, ctx->rs.stream, ctx->rs.spp, (ctx->quirks & WPBR_Q_REF_SAMPLER_ARRAYS) ? 1u : 0u};
-  P.W = ctx->rs.W;
-  P.H = ctx->rs.H;
-  P.err = ctx->d_err.p;
-  return P;
+  return pass_ctx(scene_view(ctx), render_traversal_view(ctx),
+                  wpbr_rng::Stream{ctx->rs.seed, ctx->rs.stream, ctx->rs.spp, (ctx->quirks & WPBR_Q_REF_SAMPLER_ARRAYS) ? 1u : 0u},
+                  ctx->rs.W, ctx->rs.H, ctx->d_err.p);
 }
 
 // Room for `slots` passes' film positions and sample spectra.
