@@ -27,9 +27,12 @@ constexpr int kTB = 128;
 #endif
 // The same kernels compiled with the texture path (scenes with textured
 // metal): the EWA loops need registers, and bounding them lost (textured
-// scene at 1080p: 1535 Msamples/s unbounded, 1487 at 8 blocks, 1439 at 12).
+// scene at 1080p: 1535 Msamples/s unbounded, 1487 at 8 blocks, 1439 at 12)
+// while their shading waited on FP64. Without it, 16 spp, ms: unbounded (95
+// registers, 5 blocks) 10.75, 6 blocks 10.75, 7 10.53, 8 10.53. (The other
+// spawn kernel again: 6 blocks 12.06, 8 11.84, 10 11.67, 12 11.68, 14 11.80.)
 #ifndef WPBR_SPAWN_TEX_MIN_BLOCKS
-#define WPBR_SPAWN_TEX_MIN_BLOCKS 1
+#define WPBR_SPAWN_TEX_MIN_BLOCKS 7
 #endif
 // The differentiable estimator's spawn: forward 4.06 -> 3.84 ms at 12 blocks
 // (512x512 x 16 spp).
