@@ -727,8 +727,7 @@ wpbr_status adjoint_forward(wpbr_ctx* ctx, const float* target, float* image, do
     wpbr_status s = replay_pass(ctx, P, A, p);
     if (s != WPBR_OK) return s;
     k_adj_eval<<<div_up(n, kTB), kTB, 0, st>>>(P, A, J.state.p, J.shadow_hit.p, J.Lb.p);
-    k_film_tiles<<<dim3(div_up(J.W, kFilmTile), div_up(J.H, kFilmTile)), kFilmThreadsRGB, 0, st>>>(
-        J.W, J.H, J.pf.p, J.Lb.p, J.acc.p);
+    film_tiles_launch(J.W, J.H, J.pf.p, J.Lb.p, J.acc.p, st);
   }
   const float* d_target = nullptr;
   if (target) {

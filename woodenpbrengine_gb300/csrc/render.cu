@@ -615,8 +615,7 @@ PassBufs pass_bufs(const wpbr_ctx* ctx, uint32_t g) {
 
 void film_launch(const wpbr_ctx* ctx, const PassBufs& B, cudaStream_t st) {
   const RenderState& R = ctx->rs;
-  k_film_tiles<<<dim3(div_up(R.W, kFilmTile), div_up(R.H, kFilmTile)), kFilmThreadsRGB, 0, st>>>(
-      R.W, R.H, B.pfilm, B.Lbuf, (float4*)R.acc.p);
+  film_tiles_launch(R.W, R.H, B.pfilm, B.Lbuf, (float4*)R.acc.p, st);
 }
 
 // The kernels of one sample pass up to its samples (the film gather follows),
@@ -896,8 +895,7 @@ wpbr_status job_run(wpbr_ctx* ctx, uint32_t job, uint32_t pass) {
     case WPBR_JOB_INTEGRATE_BSDF: kj_integrate_bsdf<<<g, kTB, 0, st>>>(P, G); break;
     case WPBR_JOB_FILM_ACCUMULATE:
       kj_film_pack<<<g, kTB, 0, st>>>(P, G, R.pfilm.p, R.Lbuf.p);
-      k_film_tiles<<<dim3(div_up(R.W, kFilmTile), div_up(R.H, kFilmTile)), kFilmThreadsRGB, 0, st>>>(
-          R.W, R.H, R.pfilm.p, R.Lbuf.p, (float4*)R.acc.p);
+      film_tiles_launch(R.W, R.H, R.pfilm.p, R.Lbuf.p, (float4*)R.acc.p, st);
       break;
   }
   WPBR_CUDA(cudaGetLastError());
