@@ -162,7 +162,13 @@ struct AdjState {
   DevBuf<double> g_mat, g_scalar;
   DevBuf<float4> state, rays, Lb, acc, gpix;
   DevBuf<float2> pf;
-  DevBuf<uint32_t> hit_prim, shadow_hit, shadow_map, pass_dev, counters;  // counters: 2 ray fetches, queued shadow rays
+  DevBuf<uint32_t> hit_prim, shadow_hit, shadow_map;
+  DevBuf<uint32_t> pass_dev, counters;  // per pass: its index; 2 ray fetches and the queued shadow rays
+  // passes in flight: lane 0 works in the buffers above, the others in slices
+  static constexpr uint32_t kLanes = 8;
+  DevBuf<unsigned char> slices;
+  cudaStream_t lane[kLanes] = {};
+  cudaEvent_t fork_ev = nullptr, ready_ev[kLanes] = {}, free_ev[kLanes] = {};
   void release() {
     mats_s.release(); mats_e.release(); rgb_s.release(); rgb_e.release();
     s_func.release(); s_cdf.release(); s_int.release(); s_mfunc.release(); s_mcdf.release(); s_mint.release();
@@ -170,7 +176,16 @@ struct AdjState {
     mat_prm.release(); env_prm.release(); target.release(); image.release(); g_env.release(); g_func.release();
     g_mat.release(); g_scalar.release(); state.release(); rays.release(); Lb.release(); acc.release();
     gpix.release(); pf.release(); hit_prim.release(); shadow_hit.release(); shadow_map.release(); pass_dev.release();
-    counters.release();
+    counters.release(); slices.release();
+    for (uint32_t k = 0; k < kLanes; ++k) {
+      if (lane[k]) cudaStreamDestroy(lane[k]);
+      if (ready_ev[k]) cudaEventDestroy(ready_ev[k]);
+      if (free_ev[k]) cudaEventDestroy(free_ev[k]);
+      lane[k] = nullptr;
+      ready_ev[k] = free_ev[k] = nullptr;
+    }
+    if (fork_ev) cudaEventDestroy(fork_ev);
+    fork_ev = nullptr;
     ready = false;
   }
 };
