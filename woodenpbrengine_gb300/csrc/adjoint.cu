@@ -128,6 +128,11 @@ struct EvalCtx {
   float* g_env;
   float* g_func;
   double gZ;        // this thread's share of -Z dLoss/dZ
+  // the sums that many lanes of a warp share (backward): a hit's material
+  // partials under the material's index, or a camera miss's texel partials
+  // under kTexelKey | first texel
+  uint32_t key;
+  float part[12];
 };
 
 __device__ __forceinline__ void add_env_taps(EvalCtx& E, const EnvView& e, float s, float t, RGB3 g) {
@@ -151,13 +156,66 @@ __device__ __forceinline__ void add_env_pdf(EvalCtx& E, const EnvView& e, int ce
   E.gZ += (double)g_pdf * (double)pdf;  // times -1 / Z once per block
 }
 
+constexpr uint32_t kNoKey = 0xFFFFFFFFu, kTexelKey = 0x80000000u;
 __device__ __forceinline__ void add_mat(EvalCtx& E, uint32_t mid, const MatGrad& g) {
-  float* m = E.smem_mat + 10 * mid;
-  if (g.a != 0.0f) atomicAdd(m, g.a);
+  E.key = mid;
+  E.part[0] = g.a;
   for (int c = 0; c < 3; ++c) {
-    if (g.R[c] != 0.0f) atomicAdd(m + 1 + c, g.R[c]);
-    if (g.eta[c] != 0.0f) atomicAdd(m + 4 + c, g.eta[c]);
-    if (g.k[c] != 0.0f) atomicAdd(m + 7 + c, g.k[c]);
+    E.part[1 + c] = g.R[c];
+    E.part[4 + c] = g.eta[c];
+    E.part[7 + c] = g.k[c];
+  }
+  E.part[10] = E.part[11] = 0.0f;
+}
+// A camera miss's texels: add_env_taps for lanes whose neighbours mostly see
+// the same four texels.
+__device__ __forceinline__ void share_env_taps(EvalCtx& E, const EnvView& e, float s, float t, RGB3 g) {
+  int idx[4];
+  float w[4];
+  env_taps(e, s, t, idx, w);
+  E.key = kTexelKey | (uint32_t)idx[0];
+  for (int k = 0; k < 4; ++k) {
+    E.part[3 * k] = g.r * e.le.r * w[k];
+    E.part[3 * k + 1] = g.g * e.le.g * w[k];
+    E.part[3 * k + 2] = g.b * e.le.b * w[k];
+  }
+}
+// Adds each lane's 12 parts to their targets, one addition per target and
+// distinct key of the warp instead of one per lane. Halving exchanges leave the sum
+// of part 8 b4 + 4 b3 + 2 b2 + b1 in the lanes with those index bits. A warp's
+// neighbouring pixels mostly share a material or four texels of the map: with
+// one addition per lane the backward kernel took 118 us a pass of 512 x 512,
+// most of it in the shared-memory compare-and-swap loops and the atomics'
+// queues; 76 us with one per key.
+__device__ __forceinline__ void add_shared(const EvalCtx& E, const EnvView& e) {
+  const uint32_t lane = threadIdx.x & 31u;
+  uint32_t todo = __ballot_sync(0xFFFFFFFFu, E.key != kNoKey);
+  while (todo) {
+    const uint32_t key = __shfl_sync(0xFFFFFFFFu, E.key, __ffs(todo) - 1);
+    const bool mine = E.key == key;
+    todo &= ~__ballot_sync(0xFFFFFFFFu, mine);
+    float v[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = mine && i < 12 ? E.part[i < 12 ? i : 0] : 0.0f;
+#pragma unroll
+    for (int half = 8; half >= 1; half >>= 1) {
+      const bool upper = lane & (2 * half);
+#pragma unroll
+      for (int i = 0; i < half; ++i) {
+        const float keep = upper ? v[i + half] : v[i], send = upper ? v[i] : v[i + half];
+        v[i] = keep + __shfl_xor_sync(0xFFFFFFFFu, send, 2 * half);
+      }
+    }
+    const float sum = v[0] + __shfl_xor_sync(0xFFFFFFFFu, v[0], 1);
+    const uint32_t k = lane >> 1;
+    if ((lane & 1u) || k >= 12 || sum == 0.0f) continue;
+    if (key & kTexelKey) {
+      const int i0 = (int)(key & ~kTexelKey), s0 = i0 % e.W, t0 = i0 / e.W;
+      const int tap = (int)k / 3, s = min(s0 + (tap >> 1), e.W - 1), t = min(t0 + (tap & 1), e.H - 1);
+      atomicAdd(E.g_env + 3 * ((size_t)t * e.W + s) + k % 3, sum);
+    } else if (k < 10) {
+      atomicAdd(E.smem_mat + 10 * key + k, sum);
+    }
   }
 }
 
@@ -234,124 +292,159 @@ __device__ RGB3 bsdf_branch_f(const wpbr_material& m, V3 wo, V3 wi, float* pdf, 
   return RGB3{m.R[0] * fr, m.R[1] * fr, m.R[2] * fr};
 }
 
-// One sample at theta. With BACK, gL is dLoss/dL of this sample and the
-// partials are accumulated; the return value is L either way.
-template <bool BACK>
-__device__ RGB3 eval_sample(EvalCtx& E, const float4* st, const uint32_t* shadow, uint32_t pix, RGB3 gL) {
+// One branch of a sample at theta: what its value li f w / pdf and its
+// derivatives are made of. pdf is the sampling density of the branch's
+// direction (lpdf for the light branch, bpdf for the BSDF one), opdf the
+// other strategy's.
+struct AdjBranch {
+  RGB3 li, f;
+  float pdf, opdf, w, dw, dwo;  // weight and its derivatives with respect to pdf and opdf
+  int cell;                     // environment map cell, -1: no environment light
+  float eu, ev;                 // its map coordinates
+  bool on;                      // contributes
+};
+__device__ __forceinline__ RGB3 branch_value(const AdjBranch& b) { return rmuls(rmul(b.li, b.f), b.w / b.pdf); }
+
+// The light-sampling branch: L += li f w / lpdf.
+__device__ __forceinline__ AdjBranch light_branch(const PassCtx& P, const AdjView& A, const wpbr_light& lt,
+                                                  const wpbr_material& m, V3 wo, V3 wi, float lpdf, float es, float et,
+                                                  float sin_theta) {
+  AdjBranch b;
+  b.cell = -1;
+  b.eu = es;
+  b.ev = et;
+  if (lt.type == WPBR_LIGHT_SPHERE) {
+    b.li = RGB3{lt.Le[0], lt.Le[1], lt.Le[2]};
+    b.pdf = lpdf;
+  } else {
+    b.li = (P.S.quirks & WPBR_Q_ENV_LI_SAMPLE_FIX) ? rmul(env_bilerp(A.env_e, es, et), A.env_e.le) : rgb1(0.0f);
+    b.cell = env_cell(A.env_e, es, et);
+    b.pdf = (sin_theta != 0.0f) ? env_pdf_cell(A.env_e, b.cell, sin_theta) : 0.0f;
+  }
+  b.f = bsdf_eval_ad<false>(m, wo, wi, &b.opdf, rgb1(0.0f), 0.0f, nullptr);
+  b.on = b.opdf != 0.0f;
+  b.w = power_heuristic_grad(b.pdf, b.opdf, &b.dw, &b.dwo);
+  return b;
+}
+// The BSDF-sampling branch: L += li f w / bpdf.
+__device__ __forceinline__ AdjBranch bsdf_branch(const PassCtx& P, const AdjView& A, const wpbr_light& lt,
+                                                 const wpbr_material& m, V3 wo, V3 wi, V3 wiw, V3 p) {
+  AdjBranch b;
+  b.cell = -1;
+  b.eu = b.ev = 0.0f;
+  b.on = false;
+  b.f = rgb1(0.0f);
+  b.pdf = b.w = b.dw = b.dwo = 0.0f;
+  if (lt.type == WPBR_LIGHT_SPHERE) {
+    b.opdf = sphere_light_pdf(P.S.sph_o2w[lt.sphere_index], P.S.sph_r[lt.sphere_index], p, P.S.quirks);
+    b.li = RGB3{lt.Le[0], lt.Le[1], lt.Le[2]};
+  } else {
+    V3 wl = xvector(A.env_e.w2l, wiw);
+    float theta = sph_theta(wl);
+    float phi = sph_phi(wl);
+    b.eu = div_const(phi, kTwoPiDiv);
+    b.ev = div_const(theta, kPiDiv);
+    float sth = sinf_(theta);
+    b.li = rgb1(0.0f);
+    b.opdf = 0.0f;
+    if (sth != 0.0f) {
+      b.cell = env_cell(A.env_e, b.eu, b.ev);
+      b.opdf = env_pdf_cell(A.env_e, b.cell, sth);
+      b.li = rmul(env_bilerp(A.env_e, b.eu, b.ev), A.env_e.le);
+    }
+  }
+  if (rblack(b.li)) return b;
+  b.f = bsdf_branch_f<false>(m, wo, wi, &b.pdf, rgb1(0.0f), 0.0f, nullptr);
+  if (b.pdf == 0.0f) return b;
+  b.on = true;
+  b.w = (b.pdf == 1.0f) ? 1.0f : power_heuristic_grad(b.pdf, b.opdf, &b.dw, &b.dwo);
+  return b;
+}
+// Upstream gradients of a branch's parts.
+struct BranchGrad {
+  RGB3 li, f;
+  float pdf, opdf;
+};
+__device__ __forceinline__ BranchGrad branch_grad(const AdjBranch& b, RGB3 gL) {
+  const float T = b.w / b.pdf;
+  BranchGrad g;
+  g.li = RGB3{gL.r * b.f.r * T, gL.g * b.f.g * T, gL.b * b.f.b * T};
+  g.f = RGB3{gL.r * b.li.r * T, gL.g * b.li.g * T, gL.b * b.li.b * T};
+  const float gT = gL.r * b.li.r * b.f.r + gL.g * b.li.g * b.f.g + gL.b * b.li.b * b.f.b;
+  const float gw = gT / b.pdf;
+  g.pdf = -gT * b.w / (b.pdf * b.pdf) + gw * b.dw;
+  g.opdf = gw * b.dwo;
+  return g;
+}
+
+// One sample at theta: the return value is L. BACK: gL(L) gives dLoss/dL of
+// this sample (zero: nothing to propagate), and the partials are accumulated.
+// Each branch is evaluated once and its value's parts are kept for the
+// reverse sweep. (The backward kernel evaluated every sample first for its
+// value, a second time for its parts and in the reverse sweep a third time:
+// 47 M instructions and 134 us a pass of 512 x 512; once, 34 M and 118 us.)
+template <bool BACK, class GL>
+__device__ __forceinline__ RGB3 eval_sample(EvalCtx& E, const float4* st, const uint32_t* shadow, uint32_t pix, GL gL) {
   const PassCtx& P = *E.P;
   const AdjView& A = *E.A;
-  float4 s0 = st[0];
-  uint32_t flags = __float_as_uint(s0.w);
-  RGB3 L = rgb1(0.0f);
+  const float4 s0 = st[0];
+  const uint32_t flags = __float_as_uint(s0.w);
   if (!(flags & AF_HIT)) {
-    if (P.S.has_env) {
-      V3 d{s0.x, s0.y, s0.z};
-      V3 dl = xvector(A.env_e.w2l, d);
-      float s = div_const(sph_phi(dl), kTwoPiDiv);
-      float t = div_const(sph_theta(dl), kPiDiv);
-      L = rmul(env_bilerp(A.env_e, s, t), A.env_e.le);
-      if (BACK) add_env_taps(E, A.env_e, s, t, gL);
+    if (!P.S.has_env) return rgb1(0.0f);
+    const V3 dl = xvector(A.env_e.w2l, V3{s0.x, s0.y, s0.z});
+    const float s = div_const(sph_phi(dl), kTwoPiDiv);
+    const float t = div_const(sph_theta(dl), kPiDiv);
+    const RGB3 L = rmul(env_bilerp(A.env_e, s, t), A.env_e.le);
+    if (BACK) {
+      const RGB3 g = gL(L);
+      if (!rblack(g)) share_env_taps(E, A.env_e, s, t, g);
     }
     return L;
   }
-  float4 s1 = st[1];
-  uint32_t li_idx = __float_as_uint(s1.w);
+  RGB3 L = rgb1(0.0f);
+  const float4 s1 = st[1];
+  const uint32_t li_idx = __float_as_uint(s1.w);
   if (li_idx == 0xFFFFFFFFu) return L;
-  float4 s2 = st[2], s3 = st[3], s4 = st[4], s5 = st[5];
-  uint32_t mid = __float_as_uint(s2.w);
+  const float4 s2 = st[2], s3 = st[3], s4 = st[4], s5 = st[5];
+  const uint32_t mid = __float_as_uint(s2.w);
   const wpbr_material& m = A.mats_e[mid];
   const wpbr_light& lt = P.S.lights[li_idx];
-  uint32_t lp = light_prim(lt);
-  V3 wo{s0.x, s0.y, s0.z};
-  MatGrad g{};
-  // ---- light-sampling branch: L += li f w / lpdf
+  const uint32_t lp = light_prim(lt);
+  const V3 wo{s0.x, s0.y, s0.z}, wl{s1.x, s1.y, s1.z}, wb{s2.x, s2.y, s2.z};
+  AdjBranch bl, bb;
+  bl.on = bb.on = false;
   if ((flags & AF_TRACE_L) && (shadow[2 * pix] == kNoHit || shadow[2 * pix] == lp)) {
-    V3 wi{s1.x, s1.y, s1.z};
-    RGB3 li;
-    float lpdf;
-    int cell = -1;
-    if (lt.type == WPBR_LIGHT_SPHERE) {
-      li = RGB3{lt.Le[0], lt.Le[1], lt.Le[2]};
-      lpdf = s3.w;
-    } else {
-      li = (P.S.quirks & WPBR_Q_ENV_LI_SAMPLE_FIX) ? rmul(env_bilerp(A.env_e, s4.w, s5.x), A.env_e.le) : rgb1(0.0f);
-      cell = env_cell(A.env_e, s4.w, s5.x);
-      lpdf = (s5.y != 0.0f) ? env_pdf_cell(A.env_e, cell, s5.y) : 0.0f;
-    }
-    float bpdf;
-    RGB3 f = bsdf_eval_ad<false>(m, wo, wi, &bpdf, rgb1(0.0f), 0.0f, nullptr);
-    if (bpdf != 0.0f) {
-      float dw_da, dw_db;
-      float w = power_heuristic_grad(lpdf, bpdf, &dw_da, &dw_db);
-      float T = w / lpdf;
-      L = radd(L, rmuls(rmul(li, f), T));
-      if (BACK) {
-        RGB3 gli{gL.r * f.r * T, gL.g * f.g * T, gL.b * f.b * T};
-        RGB3 gf{gL.r * li.r * T, gL.g * li.g * T, gL.b * li.b * T};
-        float gT = gL.r * li.r * f.r + gL.g * li.g * f.g + gL.b * li.b * f.b;
-        float gw = gT / lpdf;
-        float glpdf = -gT * w / (lpdf * lpdf) + gw * dw_da;
-        float gbpdf = gw * dw_db;
-        bsdf_eval_ad<true>(m, wo, wi, &bpdf, gf, gbpdf, &g);
-        if (cell >= 0) {
-          if (P.S.quirks & WPBR_Q_ENV_LI_SAMPLE_FIX) add_env_taps(E, A.env_e, s4.w, s5.x, gli);
-          add_env_pdf(E, A.env_e, cell, lpdf, glpdf);
-        }
-      }
-    }
+    bl = light_branch(P, A, lt, m, wo, wl, s3.w, s4.w, s5.x, s5.y);
+    if (bl.on) L = radd(L, branch_value(bl));
   }
-  // ---- BSDF-sampling branch: L += li f w / bpdf
   if ((flags & AF_TRACE_B) && (shadow[2 * pix + 1] == kNoHit || shadow[2 * pix + 1] == lp)) {
-    V3 wi{s2.x, s2.y, s2.z};
-    V3 wiw{s3.x, s3.y, s3.z};
-    RGB3 li;
-    float lpdf;
-    int cell = -1;
-    float eu = 0.0f, ev = 0.0f;
-    if (lt.type == WPBR_LIGHT_SPHERE) {
-      lpdf = sphere_light_pdf(P.S.sph_o2w[lt.sphere_index], P.S.sph_r[lt.sphere_index], V3{s4.x, s4.y, s4.z},
-                              P.S.quirks);
-      li = RGB3{lt.Le[0], lt.Le[1], lt.Le[2]};
-    } else {
-      V3 wl = xvector(A.env_e.w2l, wiw);
-      float theta = sph_theta(wl);
-      float phi = sph_phi(wl);
-      eu = div_const(phi, kTwoPiDiv);
-      ev = div_const(theta, kPiDiv);
-      float sth = sinf_(theta);
-      li = rgb1(0.0f);
-      lpdf = 0.0f;
-      if (sth != 0.0f) {
-        cell = env_cell(A.env_e, eu, ev);
-        lpdf = env_pdf_cell(A.env_e, cell, sth);
-        li = rmul(env_bilerp(A.env_e, eu, ev), A.env_e.le);
-      }
-    }
-    if (!rblack(li)) {
-      float bpdf;
-      RGB3 f = bsdf_branch_f<false>(m, wo, wi, &bpdf, rgb1(0.0f), 0.0f, nullptr);
-      if (bpdf != 0.0f) {
-        float dw_da = 0.0f, dw_db = 0.0f;
-        float w = (bpdf == 1.0f) ? 1.0f : power_heuristic_grad(bpdf, lpdf, &dw_da, &dw_db);
-        float T = w / bpdf;
-        L = radd(L, rmuls(rmul(li, f), T));
-        if (BACK) {
-          RGB3 gli{gL.r * f.r * T, gL.g * f.g * T, gL.b * f.b * T};
-          RGB3 gf{gL.r * li.r * T, gL.g * li.g * T, gL.b * li.b * T};
-          float gT = gL.r * li.r * f.r + gL.g * li.g * f.g + gL.b * li.b * f.b;
-          float gw = gT / bpdf;
-          float gbpdf = -gT * w / (bpdf * bpdf) + gw * dw_da;
-          float glpdf = gw * dw_db;
-          bsdf_branch_f<true>(m, wo, wi, &bpdf, gf, gbpdf, &g);
-          if (cell >= 0) {
-            add_env_taps(E, A.env_e, eu, ev, gli);
-            add_env_pdf(E, A.env_e, cell, lpdf, glpdf);
-          }
+    bb = bsdf_branch(P, A, lt, m, wo, wb, V3{s3.x, s3.y, s3.z}, V3{s4.x, s4.y, s4.z});
+    if (bb.on) L = radd(L, branch_value(bb));
+  }
+  if (BACK && (bl.on || bb.on)) {
+    const RGB3 up = gL(L);
+    if (!rblack(up)) {
+      MatGrad g{};
+      float pdf;
+      if (bl.on) {
+        const BranchGrad q = branch_grad(bl, up);
+        bsdf_eval_ad<true>(m, wo, wl, &pdf, q.f, q.opdf, &g);
+        if (bl.cell >= 0) {
+          if (P.S.quirks & WPBR_Q_ENV_LI_SAMPLE_FIX) add_env_taps(E, A.env_e, bl.eu, bl.ev, q.li);
+          add_env_pdf(E, A.env_e, bl.cell, bl.pdf, q.pdf);
         }
       }
+      if (bb.on) {
+        const BranchGrad q = branch_grad(bb, up);
+        bsdf_branch_f<true>(m, wo, wb, &pdf, q.f, q.pdf, &g);
+        if (bb.cell >= 0) {
+          add_env_taps(E, A.env_e, bb.eu, bb.ev, q.li);
+          add_env_pdf(E, A.env_e, bb.cell, bb.opdf, q.opdf);
+        }
+      }
+      add_mat(E, mid, g);
     }
   }
-  if (BACK) add_mat(E, mid, g);
   return L;
 }
 
@@ -360,28 +453,38 @@ __global__ void __launch_bounds__(kTB) k_adj_eval(PassCtx P, AdjView A, const fl
                                                   float4* Lb) {
   uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x;
   if (pix >= P.W * P.H) return;
-  EvalCtx E{&P, &A, nullptr, nullptr, nullptr, 0.0};
-  RGB3 L = eval_sample<false>(E, state + (size_t)pix * kAdjF4, shadow, pix, rgb1(0.0f));
+  EvalCtx E{&P, &A, nullptr, nullptr, nullptr, 0.0, kNoKey};
+  RGB3 L = eval_sample<false>(E, state + (size_t)pix * kAdjF4, shadow, pix, [](RGB3) { return rgb1(0.0f); });
   if (!finite3(L)) L = rgb1(0.0f);
   Lb[pix] = make_float4(L.r, L.g, L.b, 0.0f);
 }
 
 
-// dLoss/dL of a sample: the transpose of the tile-clipped film gather.
-__device__ RGB3 film_adjoint(uint32_t W, uint32_t H, uint32_t pix, float2 f, const float4* gpix) {
-  uint32_t sx = pix % W, sy = pix / W;
-  int tx0 = (int)((sx / 32) * 32), ty0 = (int)((sy / 32) * 32);
-  int tx1 = min(tx0 + 31, (int)W - 1), ty1 = min(ty0 + 31, (int)H - 1);
-  float dx0 = f.x - 0.5f, dy0 = f.y - 0.5f;
-  int pminx = max((int)ceilf(dx0 - 2.0f), tx0), pmaxx = min((int)floorf(dx0 + 2.0f), tx1);
-  int pminy = max((int)ceilf(dy0 - 2.0f), ty0), pmaxy = min((int)floorf(dy0 + 2.0f), ty1);
+// dLoss/dL of a sample: the transpose of the tile-clipped film gather (the
+// factors of k_film_tiles over the sample's own footprint).
+__device__ __forceinline__ RGB3 film_adjoint(uint32_t W, uint32_t H, int sx, int sy, float2 f, const float4* gpix) {
+  const int tx0 = sx / 32 * 32, ty0 = sy / 32 * 32;
+  const int tx1 = min(tx0 + 31, (int)W - 1), ty1 = min(ty0 + 31, (int)H - 1);
+  const float dx0 = f.x - 0.5f, dy0 = f.y - 0.5f;
+  const int pminx = max((int)ceilf(dx0 - 2.0f), tx0), pmaxx = min((int)floorf(dx0 + 2.0f), tx1);
+  const int pminy = max((int)ceilf(dy0 - 2.0f), ty0), pmaxy = min((int)floorf(dy0 + 2.0f), ty1);
+  float mx[5], my[5];
+  film_factors(f.x, sx, tx0, tx1, mx);
+  film_factors(f.y, sy, ty0, ty1, my);
   RGB3 g = rgb1(0.0f);
-  for (int y = pminy; y <= pmaxy; ++y)
-    for (int x = pminx; x <= pmaxx; ++x) {
-      float w = mitchell1(((float)x - f.x) / 2.0f) * mitchell1(((float)y - f.y) / 2.0f);
-      float4 gp = gpix[(size_t)y * W + x];
+#pragma unroll
+  for (int j = 0; j < 5; ++j) {
+    const int y = sy - 2 + j;
+    if (y < pminy || y > pmaxy) continue;
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+      const int x = sx - 2 + i;
+      if (x < pminx || x > pmaxx) continue;
+      const float w = mx[i] * my[j];
+      const float4 gp = gpix[(size_t)y * W + x];
       g = radd(g, RGB3{gp.x * w, gp.y * w, gp.z * w});
     }
+  }
   return g;
 }
 
@@ -394,15 +497,17 @@ __global__ void __launch_bounds__(kTB, WPBR_ADJ_BACK_MIN_BLOCKS) k_adj_back(Pass
   for (uint32_t j = threadIdx.x; j < nm; j += blockDim.x) smem[j] = 0.0f;
   __syncthreads();
   uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x;
-  EvalCtx E{&P, &A, smem, G.g_env, G.g_func, 0.0};
+  EvalCtx E{&P, &A, smem, G.g_env, G.g_func, 0.0, kNoKey};
   if (pix < P.W * P.H) {
-    const float4* st = state + (size_t)pix * kAdjF4;
-    RGB3 L = eval_sample<false>(E, st, shadow, pix, rgb1(0.0f));
-    if (finite3(L)) {
-      RGB3 gL = film_adjoint(P.W, P.H, pix, pf[pix], G.gpix);
-      if (!rblack(gL)) eval_sample<true>(E, st, shadow, pix, gL);
-    }
+    eval_sample<true>(E, state + (size_t)pix * kAdjF4, shadow, pix, [&](RGB3 L) {
+      if (!finite3(L)) return rgb1(0.0f);
+      uint32_t x;
+      const uint32_t y = div_mod(pix, P.row, &x);
+      return film_adjoint(P.W, P.H, (int)x, (int)y, pf[pix], G.gpix);
+    });
   }
+  __syncwarp();
+  add_shared(E, A.env_e);
   double z = E.gZ;
   for (int o = 16; o > 0; o >>= 1) z += __shfl_down_sync(0xFFFFFFFFu, z, o);
   if ((threadIdx.x & 31) == 0) zsum[threadIdx.x >> 5] = z;

@@ -39,7 +39,8 @@ constexpr int kTB = 128;
 #ifndef WPBR_ADJ_SPAWN_MIN_BLOCKS
 #define WPBR_ADJ_SPAWN_MIN_BLOCKS 12
 #endif
-// ... and its reverse sweep: backward 5.63 -> 5.19 ms at 12 blocks (8: 5.43).
+// ... and its reverse sweep: a 512 x 512 x 16 spp step 3.85 ms at 12 blocks, 10
+// 3.91, 8 3.92, 6 3.96.
 #ifndef WPBR_ADJ_BACK_MIN_BLOCKS
 #define WPBR_ADJ_BACK_MIN_BLOCKS 12
 #endif
