@@ -31,6 +31,7 @@
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 
 #include "common.cuh"
 #include "ctx.hpp"
@@ -127,6 +128,56 @@ __global__ void k_scan_tile(In in, V* out, uint32_t n, V* bsum) {
   if (threadIdx.x == kScanBlock - 1 && bsum) bsum[blockIdx.x] = total_before + sum;
 }
 
+// A scan of at most kScanOne values in one launch: one block takes them
+// kScanOneTile at a time with a running carry. The tile scan and the add of a
+// short scan cost a launch each and next to no work (10 K values: 3.4 + 6.9
+// us, 6 us in one block).
+constexpr int kScanOneBlock = 1024;
+constexpr uint32_t kScanOneTile = kScanOneBlock * kScanItems;
+constexpr uint32_t kScanOne = 2 * kScanOneTile;
+template <class V, class In>
+__global__ void __launch_bounds__(kScanOneBlock) k_scan_one(In in, V* out, uint32_t n) {
+  __shared__ V sh[kScanOneTile];
+  __shared__ V wsum[kScanOneBlock / 32];
+  const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
+  V carry = 0;
+  for (uint32_t base = 0; base < n; base += kScanOneTile) {
+    const uint32_t m = min(kScanOneTile, n - base);
+    for (uint32_t i = threadIdx.x; i < kScanOneTile; i += kScanOneBlock) sh[i] = i < m ? in(base + i) : V(0);
+    __syncthreads();
+    V v[kScanItems], sum = 0;
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k) {
+      v[k] = sh[threadIdx.x * kScanItems + k];
+      sum += v[k];
+    }
+    V x = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const V y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+      if (lane >= (uint32_t)o) x += y;
+    }
+    if (lane == 31) wsum[w] = x;
+    __syncthreads();
+    V before = 0, total = 0;
+    for (uint32_t q = 0; q < kScanOneBlock / 32; ++q) {
+      const V t = wsum[q];
+      before += q < w ? t : V(0);
+      total += t;
+    }
+    V run = carry + before + (x - sum);
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k) {
+      sh[threadIdx.x * kScanItems + k] = run;
+      run += v[k];
+    }
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < m; i += kScanOneBlock) out[base + i] = sh[i];
+    carry += total;
+    __syncthreads();
+  }
+}
+
 template <class V>
 __global__ void k_scan_add(V* out, uint32_t n, const V* boff) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -160,6 +211,10 @@ __global__ void __launch_bounds__(kScanBlock) k_scan_add_tiles(V* out, uint32_t 
 
 template <class V, class In>
 cudaError_t scan_exclusive_t(In in, V* out, uint32_t n, V* tmp, size_t tmp_n, cudaStream_t s) {
+  if (n <= kScanOne) {
+    k_scan_one<V, In><<<1, kScanOneBlock, 0, s>>>(in, out, n);
+    return cudaGetLastError();
+  }
   struct Lvl {
     const V* in;  // levels above the first: the sums below
     V* out;
@@ -208,10 +263,11 @@ size_t scan_tmp_need(uint32_t n) {
 
 }  // namespace
 
-// Kernel launches of scan_exclusive over n elements: one tile scan per
-// level, one add per level but the last.
+// Kernel launches of scan_exclusive over n elements: one for at most kScanOne,
+// else one tile scan per level, one add per level but the last.
 uint32_t scan_launches(uint32_t n) {
   if (n == 0) return 0;
+  if (n <= kScanOne) return 1;
   uint32_t levels = 1;
   for (uint32_t m = n; m > (uint32_t)kScanTile; m = div_up(m, kScanTile)) ++levels;
   return levels == 2 ? 2 : 2 * levels - 1;
@@ -296,16 +352,18 @@ __device__ __forceinline__ uint32_t left_shift3(uint32_t x) {
 }
 __device__ __forceinline__ uint32_t f2u_trunc(float v) { return (v >= 0.0f) ? (uint32_t)v : 0u; }
 
+__device__ __forceinline__ uint32_t morton_code(float4 c, const uint32_t* cb_enc) {
+  float lx = fdec(cb_enc[0]), ly = fdec(cb_enc[1]), lz = fdec(cb_enc[2]);
+  float hx = fdec(cb_enc[3]), hy = fdec(cb_enc[4]), hz = fdec(cb_enc[5]);
+  float nx = (c.x - lx) / (hx - lx), ny = (c.y - ly) / (hy - ly), nz = (c.z - lz) / (hz - lz);
+  return (left_shift3(f2u_trunc(nz * 1024.0f)) << 2) | (left_shift3(f2u_trunc(ny * 1024.0f)) << 1) |
+         left_shift3(f2u_trunc(nx * 1024.0f));
+}
 __global__ void k_morton(uint32_t N, const float4* cen, const uint32_t* cb_enc, uint32_t* codes, uint32_t* keys,
                          uint32_t* vals) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
-  float lx = fdec(cb_enc[0]), ly = fdec(cb_enc[1]), lz = fdec(cb_enc[2]);
-  float hx = fdec(cb_enc[3]), hy = fdec(cb_enc[4]), hz = fdec(cb_enc[5]);
-  float4 c = cen[i];
-  float nx = (c.x - lx) / (hx - lx), ny = (c.y - ly) / (hy - ly), nz = (c.z - lz) / (hz - lz);
-  uint32_t code = (left_shift3(f2u_trunc(nz * 1024.0f)) << 2) | (left_shift3(f2u_trunc(ny * 1024.0f)) << 1) |
-                  left_shift3(f2u_trunc(nx * 1024.0f));
+  const uint32_t code = morton_code(cen[i], cb_enc);
   codes[i] = code;
   keys[i] = code;
   vals[i] = i;
@@ -465,6 +523,152 @@ __global__ void k_treelet_ids(const uint32_t* skey, uint32_t* tid, uint32_t* tst
   if (f) tstart[t] = i;
   if (i == N - 1) info[kInfoT] = t + 1u;
 }
+// A5, A6 and the treelets of at most kOrderMax primitives in one block: codes,
+// the stable LSD sort (k_radix_scatter's ranking, the whole array in shared
+// memory between the passes) and the treelet scan. A build of a few thousand
+// primitives is bound by its launches, and these stages took 16 of 38 (and
+// nine memsets, now k_build_init): 67 primitives 213 -> 167 us a build, 1,280
+// 296 -> 223, 5,376 352 -> 290, 20,480 505 -> 474 (the one-launch scans).
+constexpr int kOrderThreads = 1024;
+constexpr int kOrderItems = 8;
+constexpr uint32_t kOrderMax = kOrderThreads * kOrderItems;
+constexpr int kOrderWarps = kOrderThreads / 32;
+constexpr size_t kOrderSmem = 4 * kOrderMax + 2 * kOrderMax + 2 * kOrderWarps * 256;
+__global__ void __launch_bounds__(kOrderThreads) k_small_order(uint32_t N, const float4* cen, const uint32_t* cb_enc,
+                                                               int passes, uint32_t* codes, uint32_t* skey,
+                                                               uint32_t* sprim, uint32_t* tid, uint32_t* tstart,
+                                                               uint32_t* info) {
+  extern __shared__ __align__(16) unsigned char order_smem[];
+  uint32_t* s_key = (uint32_t*)order_smem;
+  uint16_t* s_val = (uint16_t*)(s_key + kOrderMax);
+  uint16_t(*s_wc)[256] = (uint16_t(*)[256])(s_val + kOrderMax);  // per warp and digit: keys, then the warp's offset
+  __shared__ uint32_t s_lst[256], s_wsum[kOrderWarps];
+  const uint32_t FULL = 0xFFFFFFFFu;
+  const uint32_t lane = lane_id(), w = threadIdx.x >> 5, lt = (1u << lane) - 1u;
+  const uint32_t base = w * (32 * kOrderItems);
+  uint32_t key[kOrderItems], val[kOrderItems], rk[kOrderItems];
+#pragma unroll
+  for (int k = 0; k < kOrderItems; ++k) {
+    const uint32_t i = base + k * 32 + lane;
+    val[k] = i;
+    key[k] = i < N ? morton_code(cen[i], cb_enc) : 0u;
+    if (i < N) codes[i] = key[k];
+  }
+  for (int ps = 0; ps < passes; ++ps) {
+    const int shift = 8 * ps;
+    const uint32_t dmask = ps == 3 ? 0x3Fu : 0xFFu;
+    for (uint32_t j = threadIdx.x; j < kOrderWarps * 128; j += kOrderThreads) ((uint32_t*)s_wc)[j] = 0;
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kOrderItems; ++k) {
+      if (base + k * 32 >= N) break;  // warp-uniform
+      const bool valid = base + k * 32 + lane < N;
+      const uint32_t d = valid ? (key[k] >> shift) & dmask : 256u + lane;
+      const uint32_t peers = __match_any_sync(FULL, d);
+      const uint32_t leader = __ffs(peers) - 1;
+      uint32_t before = 0;
+      if (valid && lane == leader) {
+        before = s_wc[w][d];
+        s_wc[w][d] = (uint16_t)(before + __popc(peers));
+      }
+      before = __shfl_sync(FULL, before, leader);
+      rk[k] = before + __popc(peers & lt);
+      __syncwarp();
+    }
+    __syncthreads();
+    uint32_t acc = 0, x = 0;
+    if (threadIdx.x < 256) {  // per digit: the warps' offsets, then the digit's start
+      for (int q = 0; q < kOrderWarps; ++q) {
+        const uint32_t c = s_wc[q][threadIdx.x];
+        s_wc[q][threadIdx.x] = (uint16_t)acc;
+        acc += c;
+      }
+      x = acc;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(FULL, x, o);
+        if (lane >= (uint32_t)o) x += y;
+      }
+      if (lane == 31) s_wsum[w] = x;
+    }
+    __syncthreads();
+    if (threadIdx.x < 256) {
+      uint32_t wb = 0;
+      for (uint32_t q = 0; q < w; ++q) wb += s_wsum[q];
+      s_lst[threadIdx.x] = wb + x - acc;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kOrderItems; ++k)
+      if (base + k * 32 + lane < N) {
+        const uint32_t d = (key[k] >> shift) & dmask;
+        const uint32_t pos = s_lst[d] + s_wc[w][d] + rk[k];
+        s_key[pos] = key[k];
+        s_val[pos] = (uint16_t)val[k];
+      }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kOrderItems; ++k) {
+      const uint32_t i = base + k * 32 + lane;
+      if (i < N) {
+        key[k] = s_key[i];
+        val[k] = s_val[i];
+      }
+    }
+    __syncthreads();
+  }
+  // treelets: a flag where the top 12 bits change, counted warp by warp
+  uint32_t flags[kOrderItems], mine = 0;
+#pragma unroll
+  for (int k = 0; k < kOrderItems; ++k) {
+    const uint32_t i = base + k * 32 + lane;
+    const bool f = i < N && (i == 0 || ((key[k] ^ s_key[i - 1]) & kTreeletMask) != 0);
+    flags[k] = __ballot_sync(FULL, f);
+    mine += __popc(flags[k]);
+  }
+  if (lane == 0) s_wsum[w] = mine;
+  __syncthreads();
+  uint32_t run = 0, total = 0;
+  for (uint32_t q = 0; q < kOrderWarps; ++q) {
+    run += q < w ? s_wsum[q] : 0u;
+    total += s_wsum[q];
+  }
+#pragma unroll
+  for (int k = 0; k < kOrderItems; ++k) {
+    const uint32_t i = base + k * 32 + lane;
+    const uint32_t t = run + __popc(flags[k] & (lt | (1u << lane))) - 1u;
+    if (i < N) {
+      skey[i] = key[k];
+      sprim[i] = val[k];
+      tid[i] = t;
+      if ((flags[k] >> lane) & 1u) tstart[t] = i;
+    }
+    run += __popc(flags[k]);
+  }
+  if (threadIdx.x == 0) info[kInfoT] = total;
+}
+
+// Every buffer that a build's kernels expect cleared.
+struct BuildInit {
+  uint32_t NU, N2, N;
+  uint32_t *visits, *parent, *is_int, *int_kids, *cb_enc, *bar, *depth_max, *split_depth;
+};
+__global__ void k_build_init(BuildInit B) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < B.NU) {
+    B.visits[i] = 0u;
+    B.parent[i] = 0xFFFFFFFFu;
+  }
+  if (i < B.N2) B.is_int[i] = 0u;
+  if (i < B.N) B.int_kids[i] = 0u;
+  if (i < 6) B.cb_enc[i] = i < 3 ? 0xFFFFFFFFu : 0u;  // centroid bounds start empty
+  if (i < 4) B.bar[i] = 0u;
+  if (i == 0) {
+    *B.depth_max = 0u;
+    *B.split_depth = 0u;
+  }
+}
+
 // Primitives of treelet t: from its start to the next treelet's (T treelets).
 __device__ __forceinline__ uint32_t treelet_size(uint32_t t, const uint32_t* tstart, const uint32_t* info, uint32_t N) {
   const uint32_t T = info[kInfoT];
@@ -953,6 +1157,35 @@ __device__ __forceinline__ void batch_segments(const uint32_t* seg_of, uint32_t 
   __syncthreads();
 }
 
+// The SAH's root: true when at most kMedSeg roots leave the cooperative levels
+// nothing to do (a build of at most kMedSeg primitives launches only this).
+__device__ __forceinline__ bool sah_start(const CoopSah& C, uint32_t T) {
+  const bool first = blockIdx.x == 0 && threadIdx.x == 0;
+  if (first) *C.root_out = T == 1 ? C.troot[0] : (T == 0 ? kNone : C.N2);  // N2: SAH node 0
+  if (T > kMedSeg) return false;
+  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < T && T > 1; p += gridDim.x * blockDim.x)
+    C.item[0][p] = p;
+  if (first) {
+    const bool small = T > 1 && T <= kSmallSeg, medium = T > kSmallSeg;
+    if (T == 1) C.t_ld[0] = 0u;
+    if (T > 1) {
+      (small ? C.small_start : C.med_start)[0] = 0u;
+      (small ? C.small_end : C.med_end)[0] = T - 1;
+      (small ? C.small_node : C.med_node)[0] = 0u;
+      (small ? C.small_ld : C.med_ld)[0] = 0u;
+    }
+    C.counters[0] = T > 1 ? 1u : 0u;
+    C.counters[2] = small ? 1u : 0u;
+    C.counters[3] = medium ? 1u : 0u;
+    C.counters[4] = 0u;
+    C.counters[5] = 0u;
+    C.counters[1] = 0u;
+    C.counters[7] = 0u;
+  }
+  return true;
+}
+__global__ void k_sah_start(CoopSah C) { sah_start(C, *C.T_p); }
+
 __global__ void __launch_bounds__(kCoopBlock, kCoopPerSM) k_sah_levels(CoopSah C) {
   __shared__ SlotSeg sl[kSlots];
   __shared__ uint32_t s_acc[kSlots * kSegWords];
@@ -968,41 +1201,7 @@ __global__ void __launch_bounds__(kCoopBlock, kCoopPerSM) k_sah_levels(CoopSah C
   const uint32_t lane = lane_id(), wid = threadIdx.x >> 5;
 
   // ---- set-up: one treelet, a small segment, or level 0 over every root ----
-  if (T <= 1) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-      *C.root_out = T == 1 ? C.troot[0] : kNone;
-      if (T == 1) C.t_ld[0] = 0u;
-      C.counters[0] = 0u;
-      C.counters[2] = 0u;
-      C.counters[3] = 0u;
-      C.counters[4] = 0u;
-      C.counters[5] = 0u;
-      C.counters[1] = 0u;
-      C.counters[7] = 0u;
-    }
-    return;
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) *C.root_out = C.N2;  // SAH node 0
-  if (T <= kMedSeg) {  // the root segment is small or medium: no cooperative level
-    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < T; p += gridDim.x * blockDim.x) C.item[0][p] = p;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-      uint32_t* st = T <= kSmallSeg ? C.small_start : C.med_start;
-      uint32_t* en = T <= kSmallSeg ? C.small_end : C.med_end;
-      uint32_t* nd = T <= kSmallSeg ? C.small_node : C.med_node;
-      st[0] = 0u;
-      en[0] = T - 1;
-      nd[0] = 0u;
-      (T <= kSmallSeg ? C.small_ld : C.med_ld)[0] = 0u;
-      C.counters[0] = 1u;
-      C.counters[2] = T <= kSmallSeg ? 1u : 0u;
-      C.counters[3] = T <= kSmallSeg ? 0u : 1u;
-      C.counters[4] = 0u;
-      C.counters[5] = 0u;
-      C.counters[1] = 0u;
-      C.counters[7] = 0u;
-    }
-    return;
-  }
+  if (sah_start(C, T)) return;
   for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < T; p += gridDim.x * blockDim.x) {
     uint32_t r = C.troot[p];
     C.item[0][p] = p;
@@ -2670,6 +2869,45 @@ wpbr_status bvh_build(wpbr_ctx* ctx) {
   return st;
 }
 
+// Grids of the SAH kernels on the current device (and the shared memory their
+// launches need), asked for once per device.
+struct BuildGrids {
+  unsigned coop, medium, small;  // coop 0: no cooperative launch
+};
+static cudaError_t build_grids(BuildGrids* out) {
+  constexpr int kDevices = 64;
+  static std::mutex mu;
+  static BuildGrids known[kDevices];
+  static bool have[kDevices];
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lock(mu);
+  if (dev >= 0 && dev < kDevices && have[dev]) {
+    *out = known[dev];
+    return cudaSuccess;
+  }
+  int sms = 0, coop = 0, per_sm = 0;
+  e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sah_levels, kCoopBlock, 0);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute((const void*)k_medium_sah, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMedSmem);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute((const void*)k_small_order, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOrderSmem);
+  if (e != cudaSuccess) return e;
+  if (per_sm > kCoopPerSM) per_sm = kCoopPerSM;
+  if (sms > 0 && (uint32_t)(per_sm * sms) > kMaxCoopGrid) per_sm = (int)(kMaxCoopGrid / (uint32_t)sms);
+  BuildGrids g{coop && per_sm > 0 ? (unsigned)(per_sm * sms) : 0u, kMedPerSM * (unsigned)sms,
+               persistent_grid((const void*)k_small_sah, kB)};
+  if (dev >= 0 && dev < kDevices) {
+    known[dev] = g;
+    have[dev] = true;
+  }
+  *out = g;
+  return cudaSuccess;
+}
+
 static wpbr_status bvh_build_tree(wpbr_ctx* ctx) {
   if (!ctx->has_scene) return set_err(ctx, WPBR_ERR_NOT_BUILT, "bvh_build: no scene uploaded");
   BvhState& B = ctx->bvh;
@@ -2773,20 +3011,30 @@ static wpbr_status bvh_build_tree(wpbr_ctx* ctx) {
   WPBR_CUDA(B.split_off.ensure(N2));
   if (!B.h_info) WPBR_CUDA(cudaMallocHost((void**)&B.h_info, sizeof(uint32_t) * kInfoWords));
 
+  BuildGrids G;
+  WPBR_CUDA(build_grids(&G));
+  if (G.coop == 0) return set_err(ctx, WPBR_ERR_CUDA, "bvh_build: cooperative launch unavailable");
+
   const unsigned g = div_up(N, kB);
-  // A3/A4: centroid bounds start empty (min words all ones, max words zero)
-  WPBR_CUDA(cudaMemsetAsync(B.cb_enc.p, 0xFF, 12, st));
-  WPBR_CUDA(cudaMemsetAsync(B.cb_enc.p + 3, 0, 12, st));
+  k_build_init<<<div_up(NU, kB), kB, 0, st>>>(BuildInit{NU, N2, N, B.visits.p, B.parent.p, B.is_int.p, B.int_kids.p,
+                                                       B.cb_enc.p, B.bar.p, B.depth_max.p, B.counters.p + 6});
+  // A3/A4
   k_prim_bounds<<<g, kB, 0, st>>>(S, B.pb_lo.p, B.pb_hi.p, B.centroid.p, B.cb_enc.p);
-  // A5
-  k_morton<<<g, kB, 0, st>>>(N, B.centroid.p, B.cb_enc.p, B.codes.p, B.k0.p, B.v0.p);
-  // A6: stable radix sort by the low 24 bits (reference order) or all 30
-  uint32_t* kin = B.k0.p;
-  uint32_t* vin = B.v0.p;
-  uint32_t* kout = B.k1.p;
-  uint32_t* vout = B.v1.p;
-  int passes = full ? 4 : 3;
-  if (N > 1) {
+  const int passes = full ? 4 : 3;
+  if (N <= kOrderMax) {
+    // A5, A6 and the treelets in one launch
+    B.skey = B.k0.p;
+    B.sprim = B.v0.p;
+    k_small_order<<<1, kOrderThreads, kOrderSmem, st>>>(N, B.centroid.p, B.cb_enc.p, passes, B.codes.p, B.skey,
+                                                         B.sprim, B.tid.p, B.tstart.p, B.dinfo.p);
+  } else {
+    // A5
+    k_morton<<<g, kB, 0, st>>>(N, B.centroid.p, B.cb_enc.p, B.codes.p, B.k0.p, B.v0.p);
+    // A6: stable radix sort by the low 24 bits (reference order) or all 30
+    uint32_t* kin = B.k0.p;
+    uint32_t* vin = B.v0.p;
+    uint32_t* kout = B.k1.p;
+    uint32_t* vout = B.v1.p;
     for (int ps = 0; ps < passes; ++ps) {
       int shift = ps * 8;
       uint32_t dmask = (ps == 3) ? 0x3Fu : 0xFFu;
@@ -2796,15 +3044,13 @@ static wpbr_status bvh_build_tree(wpbr_ctx* ctx) {
       std::swap(kin, kout);
       std::swap(vin, vout);
     }
+    B.skey = kin;
+    B.sprim = vin;
+    // treelets
+    WPBR_CUDA(scan_exclusive_in(TreeletFlagIn{B.skey}, B.tid.p, N, B.scan_tmp, st));
+    k_treelet_ids<<<g, kB, 0, st>>>(B.skey, B.tid.p, B.tstart.p, N, B.dinfo.p);
   }
-  B.skey = kin;
-  B.sprim = vin;
-  // treelets
-  WPBR_CUDA(scan_exclusive_in(TreeletFlagIn{B.skey}, B.tid.p, N, B.scan_tmp, st));
-  k_treelet_ids<<<g, kB, 0, st>>>(B.skey, B.tid.p, B.tstart.p, N, B.dinfo.p);
   // A7
-  WPBR_CUDA(cudaMemsetAsync(B.visits.p, 0, sizeof(uint32_t) * NU, st));
-  WPBR_CUDA(cudaMemsetAsync(B.parent.p, 0xFF, sizeof(uint32_t) * NU, st));
   if (N > 1)
     k_karras<<<div_up(N - 1, kB), kB, 0, st>>>(B.skey, B.tid.p, B.tstart.p, B.dinfo.p, N, B.rng_lo.p, B.rng_hi.p,
                                                B.child0.p, B.child1.p, B.parent.p);
@@ -2815,16 +3061,6 @@ static wpbr_status bvh_build_tree(wpbr_ctx* ctx) {
   // A8: the large segments' levels in one cooperative launch, then the
   // warp-local SAH of the small segments
   {
-    int dev = 0, sms = 0, coop = 0, per_sm = 0;
-    WPBR_CUDA(cudaGetDevice(&dev));
-    WPBR_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    WPBR_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-    WPBR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sah_levels, kCoopBlock, 0));
-    if (!coop || per_sm < 1) return set_err(ctx, WPBR_ERR_CUDA, "bvh_build: cooperative launch unavailable");
-    if (per_sm > kCoopPerSM) per_sm = kCoopPerSM;
-    if ((uint32_t)(per_sm * sms) > kMaxCoopGrid) per_sm = (int)(kMaxCoopGrid / (uint32_t)sms);
-    if (per_sm < 1) return set_err(ctx, WPBR_ERR_CUDA, "bvh_build: too many SMs for the cooperative grid");
-    WPBR_CUDA(cudaMemsetAsync(B.bar.p, 0, sizeof(uint32_t) * 4, st));
     CoopSah C{};
     C.N = N;
     C.N2 = N2;
@@ -2879,16 +3115,17 @@ static wpbr_status bvh_build_tree(wpbr_ctx* ctx) {
     C.bar = B.bar.p;
     C.err = ctx->d_err.p;
     void* args[] = {&C};
-    WPBR_CUDA(cudaLaunchCooperativeKernel((const void*)k_sah_levels, dim3((unsigned)(per_sm * sms)),
-                                          dim3(kCoopBlock), args, 0, st));
-    WPBR_CUDA(cudaFuncSetAttribute((const void*)k_medium_sah, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)kMedSmem));
+    if (N <= kMedSeg)
+      k_sah_start<<<div_up(N, kB), kB, 0, st>>>(C);
+    else
+      WPBR_CUDA(cudaLaunchCooperativeKernel((const void*)k_sah_levels, dim3(G.coop), dim3(kCoopBlock), args, 0, st));
     MedArgs Md{N, N2, B.troot.p, B.nb_lo.p, B.nb_hi.p, B.child0.p, B.child1.p, B.parent.p, B.sah_axis.p, B.sah_rng.p, B.cur.p,
                B.med_start.p, B.med_end.p, B.med_node.p, B.med_ld.p, B.small_start.p, B.small_end.p, B.small_node.p,
                B.small_ld.p, B.sah_ld.p, B.t_ld.p, B.counters.p, ctx->d_err.p};
-    k_medium_sah<<<kMedPerSM * (unsigned)sms, kMedBlock, kMedSmem, st>>>(Md);
+    // (a build of at most kMedSeg primitives has one such segment at most, its root)
+    k_medium_sah<<<N <= kMedSeg ? 1u : G.medium, kMedBlock, kMedSmem, st>>>(Md);
     SahArgs A{N, B.troot.p, B.nb_lo.p, B.nb_hi.p, B.sah_rng.p, B.sah_ld.p, B.t_ld.p};
-    k_small_sah<<<persistent_grid((const void*)k_small_sah, kB), kB, 0, st>>>(
+    k_small_sah<<<std::min(G.small, div_up(N, 2 * (kB / 32))), kB, 0, st>>>(
         A, B.counters.p + 2, B.small_start.p, B.small_end.p, B.small_node.p, B.small_ld.p, B.cur.p, B.counters.p,
         B.sah_axis.p,
         B.nb_lo.p, B.nb_hi.p, B.child0.p, B.child1.p, B.parent.p, N2, ctx->d_err.p);
@@ -2897,15 +3134,12 @@ static wpbr_status bvh_build_tree(wpbr_ctx* ctx) {
     k_sah_sizes<<<g, kB, 0, st>>>(B.dinfo.p, B.sah_rng.p, B.tpos.p, B.size.p, N2, ctx->d_err.p);
   }
   // A9
-  WPBR_CUDA(cudaMemsetAsync(B.is_int.p, 0, sizeof(uint32_t) * N2, st));
-  WPBR_CUDA(cudaMemsetAsync(B.depth_max.p, 0, 4, st));
   k_flatten<<<div_up((uint64_t)N2 + N, kB), kB, 0, st>>>(N, B.dinfo.p, B.skey, B.tid.p, B.tstart.p,
                                                           B.rng_lo.p, B.rng_hi.p, B.child0.p, B.parent.p, B.size.p,
                                                           B.sah_axis.p, B.nb_lo.p, B.nb_hi.p, B.sah_ld.p,
                                                           B.sah_rng.p, B.t_ld.p, B.tinv.p, B.tpos.p, B.role.p, B.lin_node.p,
                                                           B.lin_bounds.p, B.is_int.p, B.depth_max.p, ctx->d_err.p);
   WPBR_CUDA(scan_exclusive(B.is_int.p, B.int_index.p, N2, B.scan_tmp, st));
-  WPBR_CUDA(cudaMemsetAsync(B.int_kids.p, 0, sizeof(uint32_t) * N, st));
   const unsigned g2 = div_up(N2, kB);
   k_int_kids<<<g2, kB, 0, st>>>(B.dinfo.p, B.lin_node.p, B.is_int.p, B.int_index.p, B.int_kids.p);
   WPBR_CUDA(scan_exclusive(B.int_kids.p, B.int_kids.p, N, B.scan_tmp, st));
@@ -2915,7 +3149,6 @@ static wpbr_status bvh_build_tree(wpbr_ctx* ctx) {
   k_prims<<<g, kB, 0, st>>>(S, B.sprim, B.prims.p);
   // leaf-split layout (the default binary traversal); a tree whose root is a
   // leaf keeps the reference layout
-  WPBR_CUDA(cudaMemsetAsync(B.counters.p + 6, 0, 4, st));
   WPBR_CUDA(scan_exclusive_in(SplitCountIn{B.dinfo.p, B.is_int.p, B.int_index.p, B.nodes2.p, B.counters.p + 6},
                               B.split_off.p, N2, B.scan_tmp, st));
   k_split_emit<<<g2, kB, 0, st>>>(B.dinfo.p, B.is_int.p, B.int_index.p, B.nodes2.p, B.split_off.p,
