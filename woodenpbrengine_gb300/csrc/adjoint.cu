@@ -88,17 +88,19 @@ __global__ void __launch_bounds__(kTB, WPBR_ADJ_SPAWN_MIN_BLOCKS) k_adj_spawn(Pa
   uint32_t li_idx = pick_light(P, pix, pass);
   const wpbr_light& lt = P.S.lights[li_idx];
   float u0, u1;
-  sample2d(P.rs, pix, pass, wpbr_rng::DIM_LIGHT, &u0, &u1);
   V3 wi{0, 0, 0};
   RGB3 li = rgb1(0.0f);
   float lpdf = 0.0f;
-  bool ok = true;
+  bool ok = light_sample_counts(P.S, lt);
   float uvs[3] = {0.0f, 0.0f, 0.0f};
-  if (lt.type == WPBR_LIGHT_SPHERE) {
-    sphere_light_sample(P.S.sph_o2w[lt.sphere_index], P.S.sph_r[lt.sphere_index], s.p, u0, u1, &wi, &lpdf);
-    li = RGB3{lt.Le[0], lt.Le[1], lt.Le[2]};
-  } else {
-    env_li_sample(A.env_s, P.S.quirks, u0, u1, &wi, &li, &lpdf, &ok, uvs);
+  if (ok) {
+    sample2d(P.rs, pix, pass, wpbr_rng::DIM_LIGHT, &u0, &u1);
+    if (lt.type == WPBR_LIGHT_SPHERE) {
+      sphere_light_sample(P.S.sph_o2w[lt.sphere_index], P.S.sph_r[lt.sphere_index], s.p, u0, u1, &wi, &lpdf);
+      li = RGB3{lt.Le[0], lt.Le[1], lt.Le[2]};
+    } else {
+      env_li_sample(A.env_s, P.S.quirks, u0, u1, &wi, &li, &lpdf, &ok, uvs);
+    }
   }
   const bool trace_l = ok && !rblack(li);
   if (trace_l) flags |= AF_TRACE_L;

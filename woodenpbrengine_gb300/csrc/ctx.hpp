@@ -340,7 +340,7 @@ cudaError_t spectral_film_launch(wpbr_ctx* ctx, uint32_t film_slots, cudaStream_
 wpbr_status spectral_resolve(wpbr_ctx* ctx);
 // float4 per pixel of the fused pass's state buffer (RenderState::pstate);
 // the RGB and the Sampled64 spawn records both fit in it.
-constexpr int kPassStateF4 = 7;
+constexpr int kPassStateF4 = 8;
 void bvh_release(wpbr_ctx* ctx, bool keep_traversal);
 wpbr_status job_run(wpbr_ctx* ctx, uint32_t job, uint32_t pass);
 wpbr_status job_record(wpbr_ctx* ctx, uint32_t x0, uint32_t y0, uint32_t x1, uint32_t y1, wpbr_pass_record* rec);

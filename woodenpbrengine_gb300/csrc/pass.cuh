@@ -251,6 +251,15 @@ __device__ LightSample sample_light(const PassCtx& P, const wpbr_light& lt, V3 p
   return s;
 }
 
+// Whether a light sample can contribute: the reference discards the looked-up
+// radiance of an environment sample (CLightInfiniteArea.cpp:192-199), so
+// without WPBR_Q_ENV_LI_SAMPLE_FIX its value is black whatever is drawn, and
+// the fused passes leave out the draw (two CDF searches of about 20 dependent
+// loads; the staged jobs record it).
+__device__ __forceinline__ bool light_sample_counts(const SceneView& S, const wpbr_light& lt) {
+  return lt.type == WPBR_LIGHT_SPHERE || (S.quirks & WPBR_Q_ENV_LI_SAMPLE_FIX);
+}
+
 __device__ void light_compute(const PassCtx& P, const wpbr_light& lt, V3 p, V3 wi, RGB3* li, float* pdf) {
   if (lt.type == WPBR_LIGHT_SPHERE) {
     *pdf = sphere_light_pdf(P.S.sph_o2w[lt.sphere_index], P.S.sph_r[lt.sphere_index], p, P.S.quirks);

@@ -43,13 +43,13 @@ struct SpecCtx {
   float* L;             // per pixel, 64 floats
 };
 
-// Per-pixel record of k_sspawn (kSpecStateF4 float4):
+// Per-pixel record of k_sspawn (kSpecStateF4 float4, five used):
 //  [0] flags, light index (environment light on a miss), material id, w/lpdf
 //  [1] light branch: cos(wi, wh), scalar BSDF factor, |cos wi|;  w/bpdf
 //  [2] BSDF branch:  cos(wi, wh), scalar BSDF factor, |cos wi|;  -
 //  [3] environment (s, t) of the light sample (or of the camera miss), of the BSDF sample
 //  [4] textured metal: k (RGB)
-constexpr int kSpecStateF4 = 5;
+constexpr int kSpecStateF4 = kPassStateF4;  // a 128-byte line a pixel, as the RGB pass
 enum : uint32_t {
   SS_HIT = 1u,        // the camera ray hit and the scene has lights
   SS_MISS_ENV = 2u,   // the camera ray missed into the environment
@@ -182,22 +182,23 @@ __global__ void __launch_bounds__(kTB, TEX ? WPBR_SPAWN_TEX_MIN_BLOCKS : WPBR_SP
   // the environment lookup at the sampled (s, t); without the fix the
   // environment branch's Li is black and nothing is traced
   float u0, u1;
-  sample2d(P.rs, pix, pass, wpbr_rng::DIM_LIGHT, &u0, &u1);
   V3 wi{0, 0, 0};
   float lpdf = 0.0f;
-  bool ok = true, li_possible = true;
-  if (lt.type == WPBR_LIGHT_SPHERE) {
-    sphere_light_sample(P.S.sph_o2w[lt.sphere_index], P.S.sph_r[lt.sphere_index], si.p, u0, u1, &wi, &lpdf);
-  } else {
-    RGB3 li_rgb;
-    float uv[3];
-    env_li_sample(P.S.env, P.S.quirks, u0, u1, &wi, &li_rgb, &lpdf, &ok, uv);
-    li_possible = (P.S.quirks & WPBR_Q_ENV_LI_SAMPLE_FIX) != 0;
-    flags |= SS_LENV;
-    s3.x = uv[0];
-    s3.y = uv[1];
+  bool ok = light_sample_counts(P.S, lt);
+  if (ok) {
+    sample2d(P.rs, pix, pass, wpbr_rng::DIM_LIGHT, &u0, &u1);
+    if (lt.type == WPBR_LIGHT_SPHERE) {
+      sphere_light_sample(P.S.sph_o2w[lt.sphere_index], P.S.sph_r[lt.sphere_index], si.p, u0, u1, &wi, &lpdf);
+    } else {
+      RGB3 li_rgb;
+      float uv[3];
+      env_li_sample(P.S.env, P.S.quirks, u0, u1, &wi, &li_rgb, &lpdf, &ok, uv);
+      flags |= SS_LENV;
+      s3.x = uv[0];
+      s3.y = uv[1];
+    }
   }
-  if (ok && li_possible && m.type != WPBR_MAT_SPECULAR) {
+  if (ok && m.type != WPBR_MAT_SPECULAR) {
     // bsdf_eval: the specular lobe evaluates to pdf 0, which contributes nothing
     V3 wi_l = to_local(fr, wi);
     V3 wh = normalize(add(wo_l, wi_l));
