@@ -720,7 +720,7 @@ static uint64_t pass_graph_key(const wpbr_ctx* ctx) {
   const void* ptrs[] = {R.acc.p,    R.hit_prim.p, R.shadow_rays.p,     R.shadow_hit.p,      R.shadow_map.p, R.pstate.p,
                         R.Lbuf.p,   R.pfilm.p,    R.pass_dev.p,        R.counters.p,        R.pass_ptr, R.order.p,
                         R.slices.p, ctx->d_err.p, ctx->bvh.view.nodes,
-                        ctx->bvh.view.prims, R.spec_mats.p, R.spec_le.p, R.spec_L.p, R.spec_acc.p};
+                        ctx->bvh.view.prims, R.spec_mats.p, R.spec_le.p, R.spec_L.p, R.spec_acc.p, R.spec_flags.p};
   for (const void* q : ptrs) mix((uint64_t)(uintptr_t)q);
   return h;
 }

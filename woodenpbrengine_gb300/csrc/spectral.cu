@@ -8,8 +8,8 @@
 // the scalar part of shading and sampling and records, per pixel, the
 // scalar factors every spectral term needs; k_sfinish gives each pixel a
 // half-warp, 16 lanes x 4 bins, for the per-bin Fresnel terms and products;
-// k_sfilm stages 8x8-pixel tiles of sample spectra in shared memory for the
-// Mitchell film gather (4 threads x 16 bins per pixel); k_sresolve
+// k_sfilm stages film tiles' rows of sample spectra in shared memory for the
+// Mitchell film gather (4 threads x 16 bins per two pixels); k_sresolve
 // converts the film to RGB once per frame (or before a film read). Every per-bin value is
 // computed with the same operations in the same order as the one-thread
 // restatement, so the film is bit-identical to it; sums over bins (toXYZ)
@@ -41,6 +41,7 @@ struct SpecCtx {
   const SpecMat* mats;
   const S64* light_le;  // per light: sphere Le, or the environment's LEmit
   float* L;             // per pixel, 64 floats
+  uint32_t* flags;      // per pixel: a bin is not finite
 };
 
 // Per-pixel record of k_sspawn (kSpecStateF4 float4, five used):
@@ -409,136 +410,200 @@ __global__ void __launch_bounds__(128, 12) k_sfinish(PassCtx P, SpecCtx C, const
     }
   }
   st_bins(C.L + (size_t)pix * kSpecN + b0, L);
+  const bool odd = !(isfinite(L.v[0]) && isfinite(L.v[1]) && isfinite(L.v[2]) && isfinite(L.v[3]));
+  const uint32_t any = __ballot_sync(hmask, odd) & hmask;
+  if ((lane & 15u) == 0) C.flags[pix] = any != 0u;
 }
 
-// Tile-clipped Mitchell gather of k_film_tiles, 64 bins per sample. A block
-// handles an 8x8 pixel tile (inside one 32x32 film tile): it stages the
-// 12x12 halo of sample spectra (those inside the film tile's clipped window)
-// in shared memory with asynchronous copies, computes the 64 x 25 neighbour
-// weights and footprint tests meanwhile, flags black samples, then each
-// pixel's 4 threads (16
-// bins each) walk the 25 neighbours in row-major order — the reference's
-// sample order within the clipped window — with invalid or black samples
-// predicated off, so the threads of a warp never diverge.
-constexpr int kFT = 8;                    // block tile side (pixels)
-constexpr int kHalo = kFT + 4;            // staged samples per side
-constexpr int kSStride = kSpecN + 4;      // floats per staged sample (float4-aligned, bank-skewed)
-constexpr int kFilmThreads = kFT * kFT * 4;
-constexpr int kFilmBins = kSpecN / 4;
-// npass passes' samples (pass j's film positions at pf + j * W * H and
-// spectra at L + j * W * H * 64) are added in pass order, each pass's
-// neighbours in row-major order, to an accumulator held in registers: the
-// same sums as npass one-pass gathers, with one read and one write of the
+// Tile-clipped Mitchell gather of k_film_tiles, 64 bins per sample: a block
+// takes a film tile's width and four of its rows, stages the spectra of those
+// rows and of two above and below (asynchronous copies, while the Mitchell
+// factors are computed), and four threads share a column of two pixels, 16
+// bins each: every staged value is read once for both. As there, pairs outside
+// the footprint and black samples add exact zeros instead of being tested,
+// unless the block holds a sample with a non-finite bin (spec_flags, from
+// k_sfinish). npass passes' samples (pass j's film positions at pf + j * W * H,
+// spectra at L + j * W * H * 64, flags likewise) are added in pass order, each
+// pass's neighbours in row-major order, to an accumulator held in registers:
+// the same sums as npass one-pass gathers, with one read and one write of the
 // 64-bin accumulator.
-__global__ void __launch_bounds__(kFilmThreads, 4) k_sfilm(uint32_t W, uint32_t H, const float2* pf, const float* L,
-                                                        uint32_t npass, float* acc, float4* accw) {
-  __shared__ __align__(16) float S[kHalo * kHalo * kSStride];
-  __shared__ float wt[kFT * kFT * 25];
-  __shared__ uint32_t vmask[kFT * kFT];
-  __shared__ uint8_t black[kHalo * kHalo];
+//
+// What bounds it: FP32 issue (25 pairs x 64 bins of a product and a sum per
+// pixel, 230 us of it below) and the shared loads (270 us), three blocks of 76
+// KB an SM. 1001 x 563, 4 passes a launch: 893 us with 8x8 tiles (2.25 staged
+// samples a pixel, each pair tested, one pixel a thread), 560 us in this
+// layout with scalar sums, 430 us with two-lane ones and unrolled copies. An
+// 8-spp frame: 4.35 -> 3.51 ms.
+constexpr int kSRows = 4;                          // pixel rows of a block
+constexpr int kSStage = kSRows + 4;                // staged sample rows
+constexpr int kFilmThreads = kFilmTile * kSRows / 2 * 4;
+constexpr int kSSamples = kSStage * kFilmTile;
+constexpr int kSPitch = kFilmTile + 2;             // factors: two empty columns between rows,
+constexpr int kSPad = kSStage * kSPitch + 2;       // before the first and after the last
+constexpr size_t kSFilmSmem = sizeof(float) * (kSSamples * kSpecN + 10 * kSPad);
+// A sample's float4 c sits at c ^ 4 in odd columns, so that the eight lanes
+// of a shared load (two columns, four threads each) meet all banks.
+__device__ __forceinline__ int spec_slot(int col, int c) { return c ^ ((col & 1) << 2); }
+// Two bins as one two-lane value.
+__device__ __forceinline__ uint64_t two(float x, float y) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+// a + t * w, the product rounded before the sum. A two-lane product that feeds
+// a two-lane sum is contracted, so the sum is a multiply-add of the product by
+// one, which rounds once: a + p. `ones` comes from the host, unknown to the
+// compiler.
+constexpr unsigned long long kOnes = 0x3F8000003F800000ull;
+__device__ __forceinline__ void add_scaled(unsigned long long& a, unsigned long long t, unsigned long long w,
+                                           unsigned long long ones) {
+  unsigned long long p;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(p) : "l"(t), "l"(w));
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(a) : "l"(p), "l"(ones));
+}
+__global__ void __launch_bounds__(kFilmThreads, 3) k_sfilm(uint32_t W, uint32_t H, const float2* pf, const float* L,
+                                                           const uint32_t* flags, uint32_t npass, float* acc,
+                                                           float4* accw, unsigned long long ones) {
+  extern __shared__ __align__(16) float sfilm_smem[];
+  ulonglong2* S = reinterpret_cast<ulonglong2*>(sfilm_smem);   // kSSamples x 16
+  float(*s_mx)[kSPad] = reinterpret_cast<float(*)[kSPad]>(sfilm_smem + kSSamples * kSpecN);  // [5]
+  float(*s_my)[kSPad] = s_mx + 5;                              // [5]
   const int tid = (int)threadIdx.x;
-  const int bx0 = (int)blockIdx.x * kFT, by0 = (int)blockIdx.y * kFT;
-  const int tx0 = (bx0 / 32) * 32, ty0 = (by0 / 32) * 32;
-  const int tx1 = min(tx0 + 31, (int)W - 1), ty1 = min(ty0 + 31, (int)H - 1);
-  const int p = tid / 4, q = tid % 4;
-  const int lx = p % kFT, ly = p / kFT;
+  const int bx0 = (int)blockIdx.x * kFilmTile, by0 = (int)blockIdx.y * kSRows;
+  const int ty0 = by0 / 32 * 32;
+  const int tx1 = min(bx0 + 31, (int)W - 1), ty1 = min(ty0 + 31, (int)H - 1);
+  const int q = tid % 4, lx = tid / 4 % kFilmTile, ly = tid / (4 * kFilmTile) * 2;
   const int x = bx0 + lx, y = by0 + ly;
-  const bool mine = x < (int)W && y < (int)H;  // this thread's pixel is on the film
-  const size_t pix = mine ? (size_t)y * W + x : 0;
-  float* ap = acc + pix * kSpecN + kFilmBins * q;
-  float a[kFilmBins];
-  float ws = 0.0f;
-  if (mine) {
-#pragma unroll
-    for (int j = 0; j < kFilmBins / 4; ++j) {
-      float4 t = *reinterpret_cast<const float4*>(ap + 4 * j);
-      a[4 * j] = t.x; a[4 * j + 1] = t.y; a[4 * j + 2] = t.z; a[4 * j + 3] = t.w;
-    }
-    ws = accw[pix].w;
-  }
   const size_t plane = (size_t)W * H;
+  bool on[2];
+  ulonglong2 a[2][4];  // bins 4 (q + 4 j) .. + 3 of each pixel
+  float ws[2];
+#pragma unroll
+  for (int p = 0; p < 2; ++p) {
+    on[p] = x < (int)W && y + p < (int)H;
+    const size_t pix = on[p] ? (size_t)(y + p) * W + x : 0;
+    const ulonglong2* ap = reinterpret_cast<const ulonglong2*>(acc + pix * kSpecN);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) a[p][j] = on[p] ? ap[q + 4 * j] : make_ulonglong2(0, 0);
+    ws[p] = on[p] ? accw[pix].w : 0.0f;
+  }
+  const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(S);
   for (uint32_t ps = 0; ps < npass; ++ps) {
     const float2* pfp = pf + ps * plane;
     const float* Lp = L + ps * plane * kSpecN;
-    // halo spectra: asynchronous 16-byte global-to-shared copies (cp.async),
-    // zero-filled outside the film tile's clipped window; they land while
-    // the weights are computed
-    for (int i = tid; i < kHalo * kHalo * 16; i += kFilmThreads) {
-      int h = i / 16, c = i % 16;
-      int sy = by0 - 2 + h / kHalo, sx = bx0 - 2 + h % kHalo;
-      bool in = sy >= ty0 && sy <= ty1 && sx >= tx0 && sx <= tx1;
-      const float* src = in ? Lp + ((size_t)sy * W + sx) * kSpecN + 4 * c : Lp;
-      uint32_t dst = (uint32_t)__cvta_generic_to_shared(S + h * kSStride + 4 * c);
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(in ? 16 : 0) : "memory");
+    // the samples: asynchronous 16-byte copies, zero-filled outside the tile;
+    // a half-warp a sample, 16 columns a step
+    const float* Lrow = Lp + ((ptrdiff_t)(by0 - 2) * W + bx0 + tid / 16) * (ptrdiff_t)kSpecN + tid % 16 * 4;
+    const uint32_t srow = sbase + 256u * (tid / 16) + 16u * spec_slot(tid / 16, tid % 16);
+#pragma unroll
+    for (int k = 0; k < kSSamples * 16 / kFilmThreads; ++k) {
+      const int sy = by0 - 2 + k / 2;
+      const bool in = bx0 + tid / 16 + k % 2 * 16 <= tx1 && sy >= ty0 && sy <= ty1;
+      const float* src = in ? Lrow + ((ptrdiff_t)(k / 2) * W + k % 2 * 16) * (ptrdiff_t)kSpecN : Lp;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(srow + 256u * 16u * k), "l"(src),
+                   "r"(in ? 16 : 0)
+                   : "memory");
     }
     asm volatile("cp.async.commit_group;\n" ::: "memory");
-    if (tid < kFT * kFT) vmask[tid] = 0u;
-    __syncthreads();
-    // neighbour weights: entry p * 25 + k is neighbour k (row-major in the 5x5 window) of pixel p
-    for (int e = tid; e < kFT * kFT * 25; e += kFilmThreads) {
-      int pe = e / 25, k = e % 25;
-      int xe = bx0 + pe % kFT, ye = by0 + pe / kFT;
-      int sx = xe - 2 + k % 5, sy = ye - 2 + k / 5;
-      float w = 0.0f;
-      if (xe < (int)W && ye < (int)H && sx >= tx0 && sx <= tx1 && sy >= ty0 && sy <= ty1) {
-        float2 f = pfp[(size_t)sy * W + sx];
-        float dx0 = f.x - 0.5f, dy0 = f.y - 0.5f;
-        int pminx = (int)ceilf(dx0 - 2.0f), pmaxx = (int)floorf(dx0 + 2.0f);
-        int pminy = (int)ceilf(dy0 - 2.0f), pmaxy = (int)floorf(dy0 + 2.0f);
-        pminx = max(pminx, tx0);
-        pminy = max(pminy, ty0);
-        pmaxx = min(pmaxx, tx1);
-        pmaxy = min(pmaxy, ty1);
-        if (!(xe < pminx || xe > pmaxx || ye < pminy || ye > pmaxy)) {
-          w = mitchell1(((float)xe - f.x) / 2.0f) * mitchell1(((float)ye - f.y) / 2.0f);
-          atomicOr(&vmask[pe], 1u << k);
-        }
+    bool odd = false;
+    for (int i = tid; i < kSPad; i += kFilmThreads) {
+      const int sx = bx0 - 2 + i % kSPitch, sy = by0 - 2 + i / kSPitch;
+      float mx[5] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f}, my[5] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+      if (sx >= bx0 && sx <= tx1 && sy >= ty0 && sy <= ty1) {
+        const size_t sp = (size_t)sy * W + sx;
+        const float2 f = pfp[sp];
+        film_factors(f.x, sx, bx0, tx1, mx);
+        film_factors(f.y, sy, ty0, ty1, my);
+        odd |= flags[ps * plane + sp] != 0u;
       }
-      wt[e] = w;
+#pragma unroll
+      for (int k = 0; k < 5; ++k) {
+        s_mx[k][i] = mx[k];
+        s_my[k][i] = my[k];
+      }
     }
     asm volatile("cp.async.wait_all;\n" ::: "memory");
-    __syncthreads();
-    // each sample's black flag, 16 threads (a half-warp) per sample
-    for (int i = tid; i < kHalo * kHalo * 16; i += kFilmThreads) {
-      int h = i / 16, c = i % 16;
-      float4 v = *reinterpret_cast<const float4*>(S + h * kSStride + 4 * c);
-      bool nz = v.x != 0.0f || v.y != 0.0f || v.z != 0.0f || v.w != 0.0f;
-      uint32_t bal = __ballot_sync(0xFFFFFFFFu, nz);
-      if (c == 0) black[h] = ((bal >> (threadIdx.x & 16u)) & 0xFFFFu) == 0u;
-    }
-    __syncthreads();
-    if (mine) {
-      const uint32_t vm = vmask[p];
-      const float* base = S + (ly * kHalo + lx) * kSStride + kFilmBins * q;
-      const uint8_t* bl = black + ly * kHalo + lx;
-      const float* wp = wt + p * 25;
+    const bool tested = __syncthreads_or(odd);
+    if (!tested) {
+      // sample rows y - 2 .. y + 3 (outer), columns x - 2 .. x + 2 (inner);
+      // pixel p is row 4 - (r - p) of a sample's reach. The first row reaches
+      // only the upper pixel, the last only the lower.
+      auto row = [&](int r, bool up, bool down) {
 #pragma unroll
-      for (int k = 0; k < 25; ++k) {
-        const int off = (k / 5) * kHalo + k % 5;
-        const bool v = (vm >> k) & 1u;
-        const float w = wp[k];
-        const bool take = v && !bl[off];
-        const float* sp = base + off * kSStride;
-        if (take) {
+        for (int dx = 0; dx < 5; ++dx) {
+          const int i = (ly + r) * kSPitch + lx + dx;
+          const int col = min(max(lx + dx - 2, 0), kFilmTile - 1);  // beyond the tile: weight zero
+          const ulonglong2* sp = S + 16 * ((ly + r) * kFilmTile + col);
+          const float mx = s_mx[4 - dx][i];
+          const float w0 = up ? mx * s_my[4 - r][i] : 0.0f, w1 = down ? mx * s_my[5 - r][i] : 0.0f;
+          const uint64_t u = two(w0, w0), v = two(w1, w1);
 #pragma unroll
-          for (int j = 0; j < kFilmBins / 4; ++j) {
-            float4 t = *reinterpret_cast<const float4*>(sp + 4 * j);
-            a[4 * j] = a[4 * j] + t.x * w;
-            a[4 * j + 1] = a[4 * j + 1] + t.y * w;
-            a[4 * j + 2] = a[4 * j + 2] + t.z * w;
-            a[4 * j + 3] = a[4 * j + 3] + t.w * w;
+          for (int j = 0; j < 4; ++j) {
+            const ulonglong2 t = sp[spec_slot(col, q + 4 * j)];
+            if (up) {
+              add_scaled(a[0][j].x, t.x, u, ones);
+              add_scaled(a[0][j].y, t.y, u, ones);
+            }
+            if (down) {
+              add_scaled(a[1][j].x, t.x, v, ones);
+              add_scaled(a[1][j].y, t.y, v, ones);
+            }
           }
+          if (up) ws[0] = ws[0] + w0;
+          if (down) ws[1] = ws[1] + w1;
         }
-        ws = v ? ws + w : ws;
-      }
-    }
-    __syncthreads();  // the next pass restages S, wt, vmask and black
-  }
-  if (!mine) return;
+      };
+      row(0, true, false);
+#pragma unroll 1
+      for (int r = 1; r < 5; ++r) row(r, true, true);
+      row(5, false, true);
+    } else {
+      for (int p = 0; p < 2; ++p)
+        for (int k = 0; k < 25; ++k) {
+          const int sx = x - 2 + k % 5, sy = y + p - 2 + k / 5;
+          const bool in = on[p] && sx >= bx0 && sx <= tx1 && sy >= ty0 && sy <= ty1;
+          bool valid = false;
+          if (in) {
+            const float2 f = pfp[(size_t)sy * W + sx];
+            const float dx0 = f.x - 0.5f, dy0 = f.y - 0.5f;
+            valid = x >= (int)ceilf(dx0 - 2.0f) && x <= (int)floorf(dx0 + 2.0f) && y + p >= (int)ceilf(dy0 - 2.0f) &&
+                    y + p <= (int)floorf(dy0 + 2.0f);
+          }
+          const int col = min(max(sx - bx0, 0), kFilmTile - 1), row = min(max(sy - by0 + 2, 0), kSStage - 1);
+          const ulonglong2* sp = S + 16 * (row * kFilmTile + col);
+          ulonglong2 t[4];
+          bool nz = false;
 #pragma unroll
-  for (int j = 0; j < kFilmBins / 4; ++j)
-    *reinterpret_cast<float4*>(ap + 4 * j) = make_float4(a[4 * j], a[4 * j + 1], a[4 * j + 2], a[4 * j + 3]);
-  if (q == 0) accw[pix].w = ws;
+          for (int j = 0; j < 4; ++j) {
+            t[j] = sp[spec_slot(col, q + 4 * j)];
+            nz |= ((t[j].x | t[j].y) & 0x7FFFFFFF7FFFFFFFull) != 0;
+          }
+          // black in all 64 bins: the pixel's four threads
+          const uint32_t any = __ballot_sync(0xFFFFFFFFu, nz) >> (threadIdx.x & 28u) & 0xFu;
+          if (!valid) continue;
+          const int i = row * kSPitch + sx - bx0 + 2;
+          const float w = s_mx[4 - k % 5][i] * s_my[4 - k / 5][i];
+          if (any) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              add_scaled(a[p][j].x, t[j].x, two(w, w), ones);
+              add_scaled(a[p][j].y, t[j].y, two(w, w), ones);
+            }
+          }
+          ws[p] = ws[p] + w;
+        }
+    }
+    __syncthreads();  // the next pass restages the samples and factors
+  }
+#pragma unroll
+  for (int p = 0; p < 2; ++p) {
+    if (!on[p]) continue;
+    const size_t pix = (size_t)(y + p) * W + x;
+    ulonglong2* ap = reinterpret_cast<ulonglong2*>(acc + pix * kSpecN);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) ap[q + 4 * j] = a[p][j];
+    if (q == 0) accw[pix].w = ws[p];
+  }
 }
 
 // toRGB of the accumulated spectra (s64_to_rgb: per bin products, the three
@@ -613,6 +678,7 @@ wpbr_status spectral_setup(wpbr_ctx* ctx) {
                             ctx->stream));
   WPBR_CUDA(cudaMemcpyAsync(R.spec_le.p, le.data(), sizeof(S64) * le.size(), cudaMemcpyHostToDevice, ctx->stream));
   WPBR_CUDA(R.spec_L.ensure(n * kSpecN));
+  WPBR_CUDA(R.spec_flags.ensure(n));
   WPBR_CUDA(R.spec_acc.ensure(n * kSpecN));
   WPBR_CUDA(cudaMemsetAsync(R.spec_acc.p, 0, sizeof(float) * n * kSpecN, ctx->stream));
   WPBR_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -631,6 +697,7 @@ cudaError_t spectral_slots(wpbr_ctx* ctx, uint32_t slots) {
   const size_t n = (size_t)R.W * R.H;
   cudaError_t e = R.pfilm.ensure(slots * n);
   if (e == cudaSuccess) e = R.spec_L.ensure(slots * n * kSpecN);
+  if (e == cudaSuccess) e = R.spec_flags.ensure(slots * n);
   return e;
 }
 
@@ -653,7 +720,8 @@ cudaError_t spectral_finish_launch(wpbr_ctx* ctx, const PassBufs& B, const uint3
                                    cudaStream_t st) {
   RenderState& R = ctx->rs;
   uint32_t n = R.W * R.H;
-  SpecCtx C{(const SpecMat*)R.spec_mats.p, (const S64*)R.spec_le.p, R.spec_L.p + (size_t)slot * n * kSpecN};
+  SpecCtx C{(const SpecMat*)R.spec_mats.p, (const S64*)R.spec_le.p, R.spec_L.p + (size_t)slot * n * kSpecN,
+            R.spec_flags.p + (size_t)slot * n};
   k_sfinish<<<div_up((uint64_t)n * kBinLanes, 128), 128, 0, st>>>(spec_pass_ctx(ctx), C, B.pstate, B.shadow_hit,
                                                                    order);
   return cudaGetLastError();
@@ -662,8 +730,12 @@ cudaError_t spectral_finish_launch(wpbr_ctx* ctx, const PassBufs& B, const uint3
 // The film gather of sample slots 0 .. film_slots - 1 in slot order.
 cudaError_t spectral_film_launch(wpbr_ctx* ctx, uint32_t film_slots, cudaStream_t st) {
   RenderState& R = ctx->rs;
-  dim3 fg(div_up(R.W, kFT), div_up(R.H, kFT));
-  k_sfilm<<<fg, kFilmThreads, 0, st>>>(R.W, R.H, R.pfilm.p, R.spec_L.p, film_slots, R.spec_acc.p, (float4*)R.acc.p);
+  cudaError_t e = cudaFuncSetAttribute((const void*)k_sfilm, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)kSFilmSmem);
+  if (e != cudaSuccess) return e;
+  dim3 fg(div_up(R.W, kFilmTile), div_up(R.H, kSRows));
+  k_sfilm<<<fg, kFilmThreads, kSFilmSmem, st>>>(R.W, R.H, R.pfilm.p, R.spec_L.p, R.spec_flags.p, film_slots,
+                                                 R.spec_acc.p, (float4*)R.acc.p, kOnes);
   return cudaGetLastError();
 }
 
