@@ -26,11 +26,9 @@ constexpr int kTB = 128;
 #define WPBR_SPAWN_MIN_BLOCKS 12
 #endif
 // The same kernels compiled with the texture path (scenes with textured
-// metal): the EWA loops need registers, and bounding them lost (textured
-// scene at 1080p: 1535 Msamples/s unbounded, 1487 at 8 blocks, 1439 at 12)
-// while their shading waited on FP64. Without it, 16 spp, ms: unbounded (95
-// registers, 5 blocks) 10.75, 6 blocks 10.75, 7 10.53, 8 10.53. (The other
-// spawn kernel again: 6 blocks 12.06, 8 11.84, 10 11.67, 12 11.68, 14 11.80.)
+// metal), whose EWA loops need registers. Textured scene, 1080p x 16 spp, ms:
+// 5 blocks 9.47, 6 9.24, 7 9.13, 8 9.23, 10 9.30. (The other spawn kernel:
+// 6 blocks 12.06, 8 11.84, 10 11.67, 12 11.68, 14 11.80.)
 #ifndef WPBR_SPAWN_TEX_MIN_BLOCKS
 #define WPBR_SPAWN_TEX_MIN_BLOCKS 7
 #endif
