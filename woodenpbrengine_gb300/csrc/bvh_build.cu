@@ -852,11 +852,17 @@ __device__ __forceinline__ Bounds dec_bounds_cg(const uint32_t* e) {
   return dec_bounds(v);
 }
 
-// Split decision of JobBuildUpperSAH (SLBVH.cpp:504-538) by one warp: lane
-// j < 12 holds bucket j's count and bounds. One width-16 shuffle scan gives
-// lanes 0..11 the union and count of buckets 0..j (prefix) and lanes 16..27,
-// which hold the buckets in reverse order, those of buckets 11-m..11
-// (suffix); lane i < 11 costs split i from its prefix and the suffix of
+// The bucket whose count and bounds this lane gives to warp_sah_split (12 or
+// more: none): lanes 0..11 the buckets in order, lanes 16..27 in reverse.
+__device__ __forceinline__ uint32_t split_bucket() {
+  const uint32_t lane = lane_id();
+  return lane < 16 ? lane : 27u - lane;  // lanes 28..31 wrap
+}
+
+// Split decision of JobBuildUpperSAH (SLBVH.cpp:504-538) by one warp: each
+// lane holds split_bucket's count and bounds (0 and anything for none). One
+// width-16 shuffle scan gives lanes 0..11 the union and count of buckets 0..j
+// (prefix) and lanes 16..27 those of buckets 11-m..11 (suffix); lane i < 11 costs split i from its prefix and the suffix of
 // bucket i+1 (lane 26 - i): the unions of the non-empty buckets on each side,
 // as the reference's two inner loops form them. The sequential first-minimum
 // rule is a lexicographic (cost, split) reduction: a NaN never wins, and a NaN
@@ -867,15 +873,8 @@ __device__ __forceinline__ Bounds dec_bounds_cg(const uint32_t* e) {
 __device__ int warp_sah_split(uint32_t cj, const Bounds& bj, float area_all, uint32_t* k_out) {
   const uint32_t FULL = 0xFFFFFFFFu;
   const uint32_t lane = lane_id();
-  const uint32_t src = lane < 16 ? lane : 27u - lane;  // lane 16 + m takes bucket 11 - m
-  const bool holds = lane < 12 || (lane >= 16 && lane < 28);
-  const uint32_t c = __shfl_sync(FULL, cj, src & 31u);
-  const Bounds b{V3{__shfl_sync(FULL, bj.lo.x, src & 31u), __shfl_sync(FULL, bj.lo.y, src & 31u),
-                    __shfl_sync(FULL, bj.lo.z, src & 31u)},
-                 V3{__shfl_sync(FULL, bj.hi.x, src & 31u), __shfl_sync(FULL, bj.hi.y, src & 31u),
-                    __shfl_sync(FULL, bj.hi.z, src & 31u)}};
-  Bounds acc = (holds && c) ? b : bempty();
-  uint32_t nacc = holds ? c : 0u;
+  Bounds acc = cj ? bj : bempty();
+  uint32_t nacc = cj;
 #pragma unroll
   for (uint32_t o = 1; o < 16; o <<= 1) {
     const Bounds u{V3{__shfl_up_sync(FULL, acc.lo.x, o, 16), __shfl_up_sync(FULL, acc.lo.y, o, 16),
@@ -896,7 +895,9 @@ __device__ int warp_sah_split(uint32_t cj, const Bounds& bj, float area_all, uin
   if (lane < 11) {
     float l = (nacc == 0) ? 0.0f : (float)nacc * barea(acc);
     float r = (n1 == 0) ? 0.0f : (float)n1 * barea(b1);
-    cost = (float)(0.125 + (double)((l + r) / area_all));
+    // the reference adds in double and rounds: the same float (the double sum
+    // is exact unless one term is beyond the float's rounding of the other)
+    cost = 0.125f + (l + r) / area_all;
   }
   float c0 = __shfl_sync(FULL, cost, 0);
   float bc = (lane < 11 && !isnan(cost)) ? cost : __int_as_float(0x7f800000);
@@ -1198,7 +1199,7 @@ __global__ void __launch_bounds__(kCoopBlock, kCoopPerSM) k_sah_levels(CoopSah C
   __shared__ unsigned long long s_bp1[kMaxCoopGrid], s_bp2[kMaxCoopGrid];  // chunk prefixes (phase C2)
   const uint32_t FULL = 0xFFFFFFFFu;
   const uint32_t T = *C.T_p;
-  const uint32_t lane = lane_id(), wid = threadIdx.x >> 5;
+  const uint32_t lane = lane_id(), wid = threadIdx.x >> 5, sbl = split_bucket();
 
   // ---- set-up: one treelet, a small segment, or level 0 over every root ----
   if (sah_start(C, T)) return;
@@ -1436,9 +1437,9 @@ __global__ void __launch_bounds__(kCoopBlock, kCoopPerSM) k_sah_levels(CoopSah C
           const uint32_t* bk = sbk + (size_t)sv * kBucketWords;
           uint32_t cj = 0;
           Bounds bj = bempty();
-          if (lane < 12) {
-            cj = __ldcg(bk + lane * 7);
-            if (cj) bj = dec_bounds_cg(bk + lane * 7 + 1);
+          if (sbl < 12) {
+            cj = __ldcg(bk + sbl * 7);
+            if (cj) bj = dec_bounds_cg(bk + sbl * 7 + 1);
           }
           Bounds bb = dec_bounds_cg(sacc + (size_t)sv * kSegWords);
           uint32_t kv;
@@ -1857,7 +1858,7 @@ __global__ void __launch_bounds__(kMedBlock, kMedPerSM) k_medium_sah(MedArgs M) 
   uint8_t* s_bkt = (uint8_t*)(s_med + kMedOffBkt);
   uint32_t* s_misc = (uint32_t*)(s_med + kMedOffMisc);  // [0..31] warp sums, [32] active, [33] next active
   const uint32_t FULL = 0xFFFFFFFFu;
-  const uint32_t t = threadIdx.x, lane = lane_id(), wid = t >> 5;
+  const uint32_t t = threadIdx.x, lane = lane_id(), wid = t >> 5, sbl = split_bucket();
   const uint32_t nmed = M.counters[3];
   for (uint32_t pass = 0; pass < 2;) {
     // segments taken in turn from a counter, so that blocks that drew small
@@ -1978,9 +1979,9 @@ __global__ void __launch_bounds__(kMedBlock, kMedPerSM) k_medium_sah(MedArgs M) 
         const uint32_t* bk = s_bkc + j * kBucketWords;
         uint32_t cj = 0;
         Bounds bj = bempty();
-        if (lane < 12) {
-          cj = bk[lane * 7];
-          if (cj) bj = dec_bounds(bk + lane * 7 + 1);
+        if (sbl < 12) {
+          cj = bk[sbl * 7];
+          if (cj) bj = dec_bounds(bk + sbl * 7 + 1);
         }
         const Bounds bb = dec_bounds(s_acc + j * kSegWords);
         uint32_t kv;
@@ -2166,57 +2167,45 @@ __global__ void __launch_bounds__(kMedBlock, kMedPerSM) k_medium_sah(MedArgs M) 
   }
 }
 
-// An SAH node over the two roots in lanes p and p + 1 (warp-uniform call).
-// The centroid bounds' minimum along their longest axis is one root's
-// centroid, which falls in bucket 0, and the other lies at t = 1, bucket 11
-// (both in bucket 0 when the centroids coincide along that axis, or the
-// extent is not finite): every split then has the same two sides, so every
-// cost is the same float and the sequential first-minimum picks split 0 —
-// the root in bucket 0 goes left, which std::partition reaches by swapping
+// SAH nodes over two roots, all of a segment's at once: a lane whose nd is not
+// kNone holds the first of a node's roots, the next lane the second (warp-
+// uniform call). The centroid bounds' minimum along their longest axis is one
+// root's centroid, which falls in bucket 0, and the other lies at t = 1,
+// bucket 11 (both in bucket 0 when the centroids coincide along that axis, or
+// the extent is not finite): every split then has the same two sides, so
+// every cost is the same float and the sequential first-minimum picks split 0
+// — the root in bucket 0 goes left, which std::partition reaches by swapping
 // the pair when the first root is the one in bucket 11. The bounds, centroid
-// bounds, axis and buckets are computed exactly as the general step does;
-// any other bucket pair returns false and is left to the general step.
-__device__ bool sah_pair(const SahArgs& A, uint32_t base, uint32_t p, uint32_t nd, uint32_t ld, uint32_t N2, uint32_t& item, V3& lo, V3& hi,
-                         uint32_t* sah_axis, float4* nb_lo, float4* nb_hi, uint32_t* child0, uint32_t* child1,
-                         uint32_t* parent) {
+// bounds, axis and buckets are computed exactly as the general step does; a
+// lane with any other bucket pair returns false and leaves its node to the
+// general step.
+__device__ bool sah_pairs(const SahArgs& A, uint32_t base, uint32_t nd, uint32_t ld, uint32_t N2, uint32_t& item,
+                          const V3& lo, const V3& hi, uint32_t* sah_axis, float4* nb_lo, float4* nb_hi,
+                          uint32_t* child0, uint32_t* child1, uint32_t* parent) {
   const uint32_t FULL = 0xFFFFFFFFu, lane = lane_id();
-  const uint32_t it0 = __shfl_sync(FULL, item, p), it1 = __shfl_sync(FULL, item, p + 1);
-  const V3 lo0{__shfl_sync(FULL, lo.x, p), __shfl_sync(FULL, lo.y, p), __shfl_sync(FULL, lo.z, p)};
-  const V3 hi0{__shfl_sync(FULL, hi.x, p), __shfl_sync(FULL, hi.y, p), __shfl_sync(FULL, hi.z, p)};
-  const V3 lo1{__shfl_sync(FULL, lo.x, p + 1), __shfl_sync(FULL, lo.y, p + 1), __shfl_sync(FULL, lo.z, p + 1)};
-  const V3 hi1{__shfl_sync(FULL, hi.x, p + 1), __shfl_sync(FULL, hi.y, p + 1), __shfl_sync(FULL, hi.z, p + 1)};
+  const uint32_t it1 = __shfl_down_sync(FULL, item, 1);
+  const V3 lo1{__shfl_down_sync(FULL, lo.x, 1), __shfl_down_sync(FULL, lo.y, 1), __shfl_down_sync(FULL, lo.z, 1)};
+  const V3 hi1{__shfl_down_sync(FULL, hi.x, 1), __shfl_down_sync(FULL, hi.y, 1), __shfl_down_sync(FULL, hi.z, 1)};
   auto emin = [](float a, float b) { return fdec(min(fenc(a), fenc(b))); };
   auto emax = [](float a, float b) { return fdec(max(fenc(a), fenc(b))); };
-  const Bounds bb{V3{emin(lo0.x, lo1.x), emin(lo0.y, lo1.y), emin(lo0.z, lo1.z)},
-                  V3{emax(hi0.x, hi1.x), emax(hi0.y, hi1.y), emax(hi0.z, hi1.z)}};
-  const V3 c0 = mul(add(lo0, hi0), 0.5f), c1 = mul(add(lo1, hi1), 0.5f);
+  const Bounds bb{V3{emin(lo.x, lo1.x), emin(lo.y, lo1.y), emin(lo.z, lo1.z)},
+                  V3{emax(hi.x, hi1.x), emax(hi.y, hi1.y), emax(hi.z, hi1.z)}};
+  const V3 c0 = mul(add(lo, hi), 0.5f), c1 = mul(add(lo1, hi1), 0.5f);
   const Bounds cb{V3{emin(c0.x, c1.x), emin(c0.y, c1.y), emin(c0.z, c1.z)},
                   V3{emax(c0.x, c1.x), emax(c0.y, c1.y), emax(c0.z, c1.z)}};
   const int dim = bmax_extent(cb);
-  const uint32_t b0 = sah_bucket(lo0, hi0, cb, dim), b1 = sah_bucket(lo1, hi1, cb, dim);
-  bool swap;
-  if (b0 == 0u && (b1 == 11u || b1 == 0u))
-    swap = false;
-  else if (b0 == 11u && b1 == 0u)
-    swap = true;
-  else
-    return false;
-  if (swap) {
-    if (lane == p) {
-      item = it1;
-      lo = lo1;
-      hi = hi1;
-    } else if (lane == p + 1) {
-      item = it0;
-      lo = lo0;
-      hi = hi0;
-    }
-  }
-  if (lane == 0) {
+  const uint32_t b0 = sah_bucket(lo, hi, cb, dim), b1 = sah_bucket(lo1, hi1, cb, dim);
+  const bool keep = b0 == 0u && (b1 == 11u || b1 == 0u), swap = b0 == 11u && b1 == 0u;
+  const bool done = nd != kNone && (keep || swap);
+  const uint32_t it0 = item;
+  const uint32_t sw = __ballot_sync(FULL, done && swap), below = __shfl_up_sync(FULL, item, 1);
+  if (sw >> lane & 1u) item = it1;
+  if (lane > 0 && (sw >> (lane - 1u) & 1u)) item = below;
+  if (done) {
     const uint32_t me = N2 + nd;
     sah_axis[nd] = (uint32_t)dim;
-    A.sah_rng[2 * nd] = base + p;
-    A.sah_rng[2 * nd + 1] = base + p + 2;
+    A.sah_rng[2 * nd] = base + lane;
+    A.sah_rng[2 * nd + 1] = base + lane + 2;
     A.sah_ld[nd] = ld;
     A.t_ld[swap ? it1 : it0] = ld_child(ld, 0);
     A.t_ld[swap ? it0 : it1] = ld_child(ld, 1);
@@ -2228,27 +2217,31 @@ __device__ bool sah_pair(const SahArgs& A, uint32_t base, uint32_t p, uint32_t n
     child1[me] = r1;
     parent[r1] = (me << 1) | 1u;
   }
-  return true;
+  return done;
 }
 
 // Segments of 2..32 roots: the whole SAH recursion inside one warp. Bounds
 // by warp reductions, buckets by shared-memory atomics, the split decision by
-// warp_sah_split, the two-pointer partition by ballots. Each segment's n - 2
-// new SAH node ids are reserved with one atomic. Nodes over two roots (about
-// half of them) are finished by sah_pair within the step that creates them
-// instead of a step of their own. A persistent grid of warps walks the
-// queue, whose length it reads from *nsmall_p (the cooperative and
-// block-local levels fill the queue on the device), each warp taking the
-// next segment from counters[5] (then counters[1]).
+// warp_sah_split, the two-pointer partition by ballots and a table of the
+// moving lanes. Each segment's n - 2 new SAH node ids are reserved with one
+// atomic. Nodes over two roots (about half of them) wait in their first
+// root's lane and are finished together by sah_pairs, a lane each: inside the
+// step that makes them each took the whole warp's instructions. What bounds
+// it is instruction issue (75 %). 1.31M triangles: 291 us with a warp a pair,
+// FP64 costs and bit-by-bit selection of the partition's partners, now 193 us.
+// A persistent grid of warps walks the queue, whose length it reads from
+// *nsmall_p (the cooperative and block-local levels fill the queue on the
+// device), each warp taking the next segment from counters[5] (then
+// counters[1]).
 __global__ void k_small_sah(SahArgs A, const uint32_t* nsmall_p, const uint32_t* sm_start, const uint32_t* sm_end,
                             const uint32_t* sm_node, const uint32_t* sm_ld, uint32_t* cur, uint32_t* counters, uint32_t* sah_axis,
                             float4* nb_lo, float4* nb_hi, uint32_t* child0, uint32_t* child1, uint32_t* parent,
                             uint32_t N2, uint32_t* err) {
-  __shared__ uint32_t sh_bcnt[kB / 32][12];
-  __shared__ uint32_t sh_benc[kB / 32][12 * 6];
+  __shared__ uint4 sh_bk[kB / 32][12 * 2];  // per bucket: lo xyz, count; hi xyz
+  __shared__ uint32_t sh_sel[kB / 32][2 * 32];
   __shared__ uint32_t sh_stack[kB / 32][4 * 64];
   const uint32_t FULL = 0xFFFFFFFFu;
-  const uint32_t w = threadIdx.x >> 5, lane = lane_id();
+  const uint32_t w = threadIdx.x >> 5, lane = lane_id(), sbl = split_bucket();
   const uint32_t nsmall = *nsmall_p;
   for (uint32_t pass = 0; pass < 2;) {
     // segments (2 to 32 roots) taken in turn from a counter, which keeps the
@@ -2276,23 +2269,42 @@ __global__ void k_small_sah(SahArgs A, const uint32_t* nsmall_p, const uint32_t*
     id_base = __shfl_sync(FULL, id_base, 0);
     uint32_t* stk = sh_stack[w];
     __syncwarp();
-    int sp = 1;
-    const uint32_t ld0 = sm_ld[seg];
-    if (n == 2 &&
-        sah_pair(A, base, 0, sm_node[seg], ld0, N2, item, lo, hi, sah_axis, nb_lo, nb_hi, child0, child1, parent)) {
-      sp = 0;
-    } else if (lane == 0) {
-      stk[0] = 0;
-      stk[1] = n - 1;
-      stk[2] = sm_node[seg];
-      stk[3] = ld0;
+    int sp = 0;
+    // a node over this lane's root and the next one's
+    uint32_t pair_nd = kNone, pair_ld = 0;
+    if (lane == 0) {
+      if (n == 2) {
+        pair_nd = sm_node[seg];
+        pair_ld = sm_ld[seg];
+      } else {
+        stk[0] = 0;
+        stk[1] = n - 1;
+        stk[2] = sm_node[seg];
+        stk[3] = sm_ld[seg];
+      }
     }
+    if (n > 2) sp = 1;
     __syncwarp();
     uint32_t guard = 0;
-    while (sp > 0) {
+    for (;;) {
       if (++guard > 64) {
         if (lane == 0) atomicOr(err, kErrLoopLimit);
         break;
+      }
+      if (sp == 0) {  // the waiting pairs
+        const uint32_t wait = __ballot_sync(FULL, pair_nd != kNone);
+        if (!wait) break;
+        const bool done =
+            sah_pairs(A, base, pair_nd, pair_ld, N2, item, lo, hi, sah_axis, nb_lo, nb_hi, child0, child1, parent);
+        const uint32_t left = wait & ~__ballot_sync(FULL, done);
+        if (!left) break;
+        if (left >> lane & 1u) {  // to the general step
+          uint32_t* e = stk + 4 * __popc(left & ((1u << lane) - 1u));
+          e[0] = lane; e[1] = lane + 1; e[2] = pair_nd; e[3] = pair_ld;
+        }
+        pair_nd = kNone;
+        sp = __popc(left);
+        __syncwarp();
       }
       --sp;
       uint32_t a = stk[4 * sp], b = stk[4 * sp + 1], nd = stk[4 * sp + 2], ld = stk[4 * sp + 3];
@@ -2315,26 +2327,27 @@ __global__ void k_small_sah(SahArgs A, const uint32_t* nsmall_p, const uint32_t*
       int dim = bmax_extent(cb);
       uint32_t ib = act ? sah_bucket(lo, hi, cb, dim) : 0u;
       // per-bucket counts and bounds
-      uint32_t* bcnt = sh_bcnt[w];
-      uint32_t* benc = sh_benc[w];
-      if (lane < 12) {
-        bcnt[lane] = 0;
-        for (int k = 0; k < 6; ++k) benc[lane * 6 + k] = k < 3 ? 0xFFFFFFFFu : 0u;
-      }
+      uint4* bk = sh_bk[w];
+      if (lane < 24) bk[lane] = lane & 1u ? uint4{0u, 0u, 0u, 0u} : uint4{0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0u};
       __syncwarp();
       if (act) {
-        atomicAdd(&bcnt[ib], 1u);
-        uint32_t* be = benc + ib * 6;
+        uint32_t* be = (uint32_t*)(bk + 2 * ib);
         atomicMin(be + 0, fenc(lo.x));
         atomicMin(be + 1, fenc(lo.y));
         atomicMin(be + 2, fenc(lo.z));
-        atomicMax(be + 3, fenc(hi.x));
-        atomicMax(be + 4, fenc(hi.y));
-        atomicMax(be + 5, fenc(hi.z));
+        atomicAdd(be + 3, 1u);
+        atomicMax(be + 4, fenc(hi.x));
+        atomicMax(be + 5, fenc(hi.y));
+        atomicMax(be + 6, fenc(hi.z));
       }
       __syncwarp();
-      uint32_t cj = lane < 12 ? bcnt[lane] : 0u;
-      Bounds bj = (lane < 12 && cj) ? dec_bounds(benc + lane * 6) : bempty();
+      uint32_t cj = 0;
+      Bounds bj = bempty();
+      if (sbl < 12) {
+        const uint4 l = bk[2 * sbl], h = bk[2 * sbl + 1];
+        cj = l.w;
+        if (cj) bj = Bounds{V3{fdec(l.x), fdec(l.y), fdec(l.z)}, V3{fdec(h.x), fdec(h.y), fdec(h.z)}};
+      }
       uint32_t k;
       int best = warp_sah_split(cj, bj, barea(bb), &k);
       // two-pointer partition of [a, b] by ib <= best
@@ -2343,17 +2356,15 @@ __global__ void k_small_sah(SahArgs A, const uint32_t* nsmall_p, const uint32_t*
       uint32_t fmask = __ballot_sync(FULL, act && lane < spt && !pred);
       uint32_t tmask = __ballot_sync(FULL, act && lane >= spt && pred);
       uint32_t src = lane;
-      if (act && lane < spt && !pred) {
-        uint32_t r = __popc(fmask & ((1u << lane) - 1u));
-        uint32_t m = __brev(tmask);  // r-th highest set bit of tmask
-        for (uint32_t q = 0; q < r; ++q) m &= m - 1u;
-        src = 31u - (uint32_t)(__ffs(m) - 1);
-      } else if (act && lane >= spt && pred) {
-        uint32_t r = __popc(tmask & ~((2u << lane) - 1u));  // trues above this lane
-        if (lane == 31) r = 0;
-        uint32_t m = fmask;
-        for (uint32_t q = 0; q < r; ++q) m &= m - 1u;
-        src = (uint32_t)(__ffs(m) - 1);
+      const bool mf = fmask >> lane & 1u, mt = tmask >> lane & 1u;
+      if (fmask) {  // the r-th false from the left and the r-th true from the right
+        uint32_t* sel = sh_sel[w];
+        const uint32_t r =
+            mf ? __popc(fmask & ((1u << lane) - 1u)) : __popc(tmask >> lane) - 1;  // trues above this lane
+        if (mf || mt) sel[(mt ? 32u : 0u) + r] = lane;
+        __syncwarp();
+        if (mf || mt) src = sel[(mf ? 32u : 0u) + r] & 31u;
+        __syncwarp();
       }
       item = __shfl_sync(FULL, item, src);
       lo.x = __shfl_sync(FULL, lo.x, src); lo.y = __shfl_sync(FULL, lo.y, src);
@@ -2373,7 +2384,7 @@ __global__ void k_small_sah(SahArgs A, const uint32_t* nsmall_p, const uint32_t*
       uint32_t litem = __shfl_sync(FULL, item, a);
       uint32_t ritem = __shfl_sync(FULL, item, b);
       // the children's node ids (lane 0 keeps the running count); children of
-      // two roots are finished here
+      // two roots wait
       uint32_t cl = 0, cr = 0;
       if (lane == 0) {
         if (ln > 1) cl = id_base + id_next++;
@@ -2381,10 +2392,14 @@ __global__ void k_small_sah(SahArgs A, const uint32_t* nsmall_p, const uint32_t*
       }
       cl = __shfl_sync(FULL, cl, 0);
       cr = __shfl_sync(FULL, cr, 0);
-      const bool lpair =
-          ln == 2 && sah_pair(A, base, a, cl, ld_child(ld, 0), N2, item, lo, hi, sah_axis, nb_lo, nb_hi, child0, child1, parent);
-      const bool rpair =
-          rn == 2 && sah_pair(A, base, mid, cr, ld_child(ld, 1), N2, item, lo, hi, sah_axis, nb_lo, nb_hi, child0, child1, parent);
+      if (ln == 2 && lane == a) {
+        pair_nd = cl;
+        pair_ld = ld_child(ld, 0);
+      }
+      if (rn == 2 && lane == mid) {
+        pair_nd = cr;
+        pair_ld = ld_child(ld, 1);
+      }
       if (lane == 0) {
         if (ln == 1) {
           uint32_t r = A.troot[litem];
@@ -2394,7 +2409,7 @@ __global__ void k_small_sah(SahArgs A, const uint32_t* nsmall_p, const uint32_t*
         } else {
           child0[me] = N2 + cl;
           parent[N2 + cl] = (me << 1) | 0u;
-          if (!lpair) {
+          if (ln > 2) {
             stk[4 * sp] = a; stk[4 * sp + 1] = mid - 1; stk[4 * sp + 2] = cl; stk[4 * sp + 3] = ld_child(ld, 0);
             ++sp;
           }
@@ -2407,7 +2422,7 @@ __global__ void k_small_sah(SahArgs A, const uint32_t* nsmall_p, const uint32_t*
         } else {
           child1[me] = N2 + cr;
           parent[N2 + cr] = (me << 1) | 1u;
-          if (!rpair) {
+          if (rn > 2) {
             stk[4 * sp] = mid; stk[4 * sp + 1] = b; stk[4 * sp + 2] = cr; stk[4 * sp + 3] = ld_child(ld, 1);
             ++sp;
           }
