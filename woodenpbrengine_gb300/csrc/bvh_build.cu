@@ -957,8 +957,12 @@ __device__ __forceinline__ uint32_t sah_bucket(const V3& lo, const V3& hi, const
 // leaves at its next barrier. Indices derived from scanned values are checked
 // before use.
 // ---------------------------------------------------------------------------
-// 1.31M-triangle build, device ms: 512 threads (2 blocks per SM) 1.588,
-// 1024 (1 per SM, half the grid barrier's arrivals) 1.575.
+// What bounds it: the chain of dependent loads and barriers of a phase (a
+// quarter of the issue slots used; eight levels of 4 phases at 8 to 12 us each).
+// 1.31M triangles: 398 us with a barrier of two words and fences, prefixes of
+// the flags by 64-bit shuffles and buckets reduced one at a time, now 334 us.
+// 512 threads (2 blocks per SM) instead of 1024 (1, half the grid barrier's
+// arrivals): the build 1.588 against 1.575 ms.
 #ifndef WPBR_COOP_BLOCK
 #define WPBR_COOP_BLOCK 1024
 #endif
@@ -967,7 +971,8 @@ constexpr int kCoopPerSM = 1024 / kCoopBlock;  // resident blocks per SM (64 reg
 constexpr int kCoopWarps = kCoopBlock / 32;
 constexpr uint32_t kMaxCoopGrid = 1024;  // blocks of the cooperative grid (chunk prefixes in shared memory)
 static_assert(kMaxCoopGrid <= 2 * kCoopBlock, "block_scan_pairs scans two entries a thread");
-constexpr uint32_t kSpinLimit = 1u << 24;   // barrier polls (100 ns apart) before giving up
+constexpr uint32_t kSpinLimit = 1u << 22;   // barrier polls (about half a microsecond each) before giving up
+constexpr unsigned long long kBarAbort = 1ull << 63;
 constexpr uint32_t kSegWords = 12;          // bounds lo/hi, centroid bounds lo/hi (encoded)
 constexpr uint32_t kBucketWords = 12 * 7;   // per bucket: count, lo xyz, hi xyz (encoded)
 
@@ -1019,44 +1024,37 @@ struct CoopSah {
   uint32_t* small_ld;
   uint32_t* counters;  // [0] SAH nodes allocated, [2] small segments queued, [3] medium segments queued
   uint32_t* root_out;  // unified id of the tree's root
-  uint32_t* bar;       // grid barrier: [0] arrivals, [1] generation, [2] abort
+  unsigned long long* bar;  // grid barrier: arrivals and abort flag
   uint32_t* err;
 };
 
-__device__ __forceinline__ uint32_t ld_vol(const uint32_t* p) { return *(const volatile uint32_t*)p; }
-
-// Grid-wide barrier of the cooperative launch. false: some block gave up
-// waiting (abort set), and the caller leaves the kernel.
-__device__ bool coop_sync(uint32_t* bar, uint32_t* err) {
+// Grid-wide barrier of the cooperative launch: one arrival count, never reset
+// within a launch (barrier r is passed at r * gridDim.x arrivals), whose top
+// bit is the abort flag, so that a block makes one release-acquire addition
+// and polls one word. false: some block gave up waiting, and the caller
+// leaves the kernel. (With a generation word next to the count, fences around
+// both and a 100 ns sleep between polls a barrier took 2.8 us, 33 of them 90 us
+// of a 1.31M-triangle build.)
+__device__ bool coop_sync(unsigned long long* bar, uint32_t* err, uint32_t& round) {
   __shared__ uint32_t s_ok;
+  ++round;
   __syncthreads();
   if (threadIdx.x == 0) {
-    const uint32_t gen = ld_vol(bar + 1);
-    __threadfence();
-    bool ok = true;
-    if (atomicAdd(bar, 1u) == gridDim.x - 1) {
-      atomicExch(bar, 0u);
-      __threadfence();
-      atomicAdd(bar + 1, 1u);
-    } else {
-      uint32_t spins = 0;
-      while (ld_vol(bar + 1) == gen) {
-        if (ld_vol(bar + 2)) {
-          ok = false;
-          break;
-        }
-        if (++spins > kSpinLimit) {
-          atomicOr(bar + 2, 1u);
-          atomicOr(err, kErrLoopLimit);
-          ok = false;
-          break;
-        }
-        __nanosleep(100);
+    const unsigned long long want = (unsigned long long)round * gridDim.x;
+    unsigned long long v;
+    asm volatile("atom.add.acq_rel.gpu.global.u64 %0, [%1], 1;" : "=l"(v) : "l"(bar) : "memory");
+    ++v;
+    uint32_t spins = 0;
+    while (!(v & kBarAbort) && v < want) {
+      if (++spins > kSpinLimit) {
+        atomicOr(bar, kBarAbort);
+        atomicOr(err, kErrLoopLimit);
+        v = kBarAbort;
+        break;
       }
+      asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(bar) : "memory");
     }
-    __threadfence();
-    if (ld_vol(bar + 2)) ok = false;
-    s_ok = ok ? 1u : 0u;
+    s_ok = (v & kBarAbort) ? 0u : 1u;
   }
   __syncthreads();
   return s_ok != 0;
@@ -1201,6 +1199,8 @@ __global__ void __launch_bounds__(kCoopBlock, kCoopPerSM) k_sah_levels(CoopSah C
   const uint32_t T = *C.T_p;
   const uint32_t lane = lane_id(), wid = threadIdx.x >> 5, sbl = split_bucket();
 
+  uint32_t round = 0;  // grid barriers passed
+
   // ---- set-up: one treelet, a small segment, or level 0 over every root ----
   if (sah_start(C, T)) return;
   for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < T; p += gridDim.x * blockDim.x) {
@@ -1225,7 +1225,7 @@ __global__ void __launch_bounds__(kCoopBlock, kCoopPerSM) k_sah_levels(CoopSah C
     C.counters[1] = 0u;
     C.counters[7] = 0u;
   }
-  if (!coop_sync(C.bar, C.err)) return;
+  if (!coop_sync(C.bar, C.err, round)) return;
 
   // every phase walks the block's chunk of consecutive positions in batches
   const uint32_t ntiles = div_up_d(T, kCoopBlock);
@@ -1338,7 +1338,7 @@ __global__ void __launch_bounds__(kCoopBlock, kCoopPerSM) k_sah_levels(CoopSah C
         }
         __syncthreads();
       }
-      if (!coop_sync(C.bar, C.err)) return;
+      if (!coop_sync(C.bar, C.err, round)) return;
     }
 
     // ---- B: buckets ----
@@ -1373,33 +1373,9 @@ __global__ void __launch_bounds__(kCoopBlock, kCoopPerSM) k_sah_levels(CoopSah C
           ib = sah_bucket(lo, hi, cb, bmax_extent(cb));
           C.bucket[p[k]] = (uint8_t)ib;
         }
-        const uint32_t s0 = __shfl_sync(FULL, sk, 0);
-        if (s0 != kNone && __all_sync(FULL, sk == s0)) {  // one segment: reduce per present bucket
-          uint32_t present = __reduce_or_sync(FULL, 1u << ib);
-          uint32_t* base_bk = s_bk + (s0 & (kSlots - 1)) * kBucketWords;
-          while (present) {
-            const uint32_t j = __ffs(present) - 1;
-            present &= present - 1;
-            const bool in = ib == j;
-            const uint32_t cnt = __popc(__ballot_sync(FULL, in));
-            uint32_t v0 = __reduce_min_sync(FULL, in ? fenc(lo.x) : 0xFFFFFFFFu);
-            uint32_t v1 = __reduce_min_sync(FULL, in ? fenc(lo.y) : 0xFFFFFFFFu);
-            uint32_t v2 = __reduce_min_sync(FULL, in ? fenc(lo.z) : 0xFFFFFFFFu);
-            uint32_t v3 = __reduce_max_sync(FULL, in ? fenc(hi.x) : 0u);
-            uint32_t v4 = __reduce_max_sync(FULL, in ? fenc(hi.y) : 0u);
-            uint32_t v5 = __reduce_max_sync(FULL, in ? fenc(hi.z) : 0u);
-            if (lane == 0) {
-              uint32_t* d = base_bk + j * 7;
-              atomicAdd(d, cnt);
-              atomicMin(d + 1, v0);
-              atomicMin(d + 2, v1);
-              atomicMin(d + 3, v2);
-              atomicMax(d + 4, v3);
-              atomicMax(d + 5, v4);
-              atomicMax(d + 6, v5);
-            }
-          }
-        } else if (sk != kNone) {
+        // (a reduction per bucket that the warp's roots meet, six to twelve of
+        // them, takes longer than the atomics' conflicts: 398 -> 388 us)
+        if (sk != kNone) {
           uint32_t* d = s_bk + (sk & (kSlots - 1)) * kBucketWords + ib * 7;
           atomicAdd(d, 1u);
           atomicMin(d + 1, fenc(lo.x));
@@ -1423,7 +1399,7 @@ __global__ void __launch_bounds__(kCoopBlock, kCoopPerSM) k_sah_levels(CoopSah C
       }
       __syncthreads();
     }
-    if (!coop_sync(C.bar, C.err)) return;
+    if (!coop_sync(C.bar, C.err, round)) return;
 
     // ---- C1: decisions, partition flags, scans within each block's chunk ----
     {
@@ -1456,7 +1432,13 @@ __global__ void __launch_bounds__(kCoopBlock, kCoopPerSM) k_sah_levels(CoopSah C
           }
         }
         __syncthreads();
-        unsigned long long v1[kBatchTiles], v2[kBatchTiles], i1[kBatchTiles], i2[kBatchTiles];
+        // exclusive prefixes within the warp by ballots: the flags are single
+        // bits, the children counts of a segment's first position 0, 1 or 2
+        unsigned long long e1[kBatchTiles], e2[kBatchTiles];
+        const uint32_t below = (1u << lane) - 1u;
+        auto counts = [&](uint32_t hi, uint32_t lo, uint32_t m) {
+          return ((unsigned long long)__popc(hi & m) << 32) | (unsigned long long)__popc(lo & m);
+        };
         uint8_t bkt[kBatchTiles];
 #pragma unroll
         for (int k = 0; k < kBatchTiles; ++k) bkt[k] = s[k] != kNone ? __ldcg(C.bucket + p[k]) : (uint8_t)0;
@@ -1475,13 +1457,19 @@ __global__ void __launch_bounds__(kCoopBlock, kCoopPerSM) k_sah_levels(CoopSah C
               nl = (uint32_t)(ln > kMedSeg) + (uint32_t)(rn > kMedSeg);
             }
           }
-          v1[k] = ((unsigned long long)fT << 32) | (unsigned long long)fF;
-          v2[k] = ((unsigned long long)nl << 32) | (unsigned long long)nn;
-          i1[k] = warp_incl_scan64(v1[k]);
-          i2[k] = warp_incl_scan64(v2[k]);
-          if (lane == 31) {
-            s_w1[k][wid] = i1[k];
-            s_w2[k][wid] = i2[k];
+          const uint32_t bF = __ballot_sync(FULL, fF), bT = __ballot_sync(FULL, fT);
+          e1[k] = counts(bT, bF, below);
+          e2[k] = 0ull;
+          unsigned long long t2 = 0ull;
+          if (__any_sync(FULL, nn != 0u)) {
+            const uint32_t n1 = __ballot_sync(FULL, nn >= 1u), n2 = __ballot_sync(FULL, nn >= 2u);
+            const uint32_t l1 = __ballot_sync(FULL, nl >= 1u), l2 = __ballot_sync(FULL, nl >= 2u);
+            e2[k] = counts(l1, n1, below) + counts(l2, n2, below);
+            t2 = counts(l1, n1, FULL) + counts(l2, n2, FULL);
+          }
+          if (lane == 0) {
+            s_w1[k][wid] = counts(bT, bF, FULL);
+            s_w2[k][wid] = t2;
           }
         }
         __syncthreads();
@@ -1503,11 +1491,11 @@ __global__ void __launch_bounds__(kCoopBlock, kCoopPerSM) k_sah_levels(CoopSah C
         unsigned long long o1 = carry1, o2 = carry2;
 #pragma unroll
         for (int k = 0; k < kBatchTiles; ++k) {
-          if (p[k] < c1) C.ftl[p[k]] = o1 + s_w1[k][wid] + (i1[k] - v1[k]);
+          if (p[k] < c1) C.ftl[p[k]] = o1 + s_w1[k][wid] + e1[k];
           if (s[k] != kNone) {
             const SlotSeg& g = sl[s[k] & (kSlots - 1)];
             if (p[k] == g.a) {
-              C.segpre[s[k]] = o2 + s_w2[k][wid] + (i2[k] - v2[k]);
+              C.segpre[s[k]] = o2 + s_w2[k][wid] + e2[k];
               C.sdec[s[k]] = make_uint4(g.spt, g.mid, kNone, kNone);
               C.sbest[s[k]] = g.best;
             }
@@ -1524,7 +1512,7 @@ __global__ void __launch_bounds__(kCoopBlock, kCoopPerSM) k_sah_levels(CoopSah C
         C.btot[2 * blockIdx.x + 1] = carry2;
       }
     }
-    if (!coop_sync(C.bar, C.err)) return;
+    if (!coop_sync(C.bar, C.err, round)) return;
 
     // ---- C2: prefixes over the chunks, select tables, SAH nodes, children ----
     block_scan_pairs(C.btot, gridDim.x, s_bp1, s_bp2, &s_w1[0][0], &s_w2[0][0], s_tot);
@@ -1632,7 +1620,7 @@ __global__ void __launch_bounds__(kCoopBlock, kCoopPerSM) k_sah_levels(CoopSah C
         __syncthreads();
       }
     }
-    if (!coop_sync(C.bar, C.err)) return;
+    if (!coop_sync(C.bar, C.err, round)) return;
 
     // ---- E: swap pairs, next level's position arrays, single-root children ----
     {
@@ -1757,7 +1745,7 @@ __global__ void __launch_bounds__(kCoopBlock, kCoopPerSM) k_sah_levels(CoopSah C
         __syncthreads();
       }
     }
-    if (!coop_sync(C.bar, C.err)) return;
+    if (!coop_sync(C.bar, C.err, round)) return;
     par = nx;
     if (__ldcg(C.lvl + 8 * par) == 0u) break;
   }
@@ -3127,7 +3115,7 @@ static wpbr_status bvh_build_tree(wpbr_ctx* ctx) {
     C.med_node = B.med_node.p;
     C.counters = B.counters.p;
     C.root_out = B.dinfo.p + kInfoRoot;
-    C.bar = B.bar.p;
+    C.bar = (unsigned long long*)B.bar.p;
     C.err = ctx->d_err.p;
     void* args[] = {&C};
     if (N <= kMedSeg)
