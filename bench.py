@@ -59,13 +59,13 @@ SAMPLE_BYTES_SAMPLED64 = SAMPLE_BYTES_ENV - 256.0 + 16 * (64 * 4 + 4)
 # refit 120 B (codes 12, node 12, leaf bounds 24, child bounds 48, write 24).
 BUILD_BYTES_PER_PRIM = 56.0 + 64.0 + 120.0
 # kernels of one fused sample pass: camera traversal, spawn, shadow traversal,
-# finish, film; films of 2^17 pixels and more add the two kernels that order
-# the pixels by material category
+# finish, film; films of 2^17 pixels and more add the kernel that orders the
+# pixels by material category
 SORT_MIN_PIXELS = 1 << 17
 
 
 def pass_launches(pixels):
-    return 5 + (2 if pixels >= SORT_MIN_PIXELS else 0)
+    return 5 + (1 if pixels >= SORT_MIN_PIXELS else 0)
 
 
 STAGES = ["CAMERA_RAYS", "COLLIDE_PRIMARY", "EMITTED_LIGHT", "BSDF_SETUP", "SAMPLE_LIGHT", "SHADOW_LIGHT",

@@ -97,8 +97,8 @@ struct BvhState {
 };
 
 // Words of RenderState::counters (zeroed at the start of every pass).
-constexpr uint32_t kQueueCounter = 24;
-constexpr uint32_t kPassCounters = 25;
+constexpr uint32_t kQueueCounter = 2;
+constexpr uint32_t kPassCounters = 3;
 
 struct RenderState {
   bool ready = false;
@@ -121,9 +121,8 @@ struct RenderState {
   uint64_t graph_key = 0;
   DevBuf<uint32_t> pass_dev;  // pass index read by the captured kernels
   DevBuf<uint32_t> counters;  // kPassCounters words: ray-fetch counters of the pass's two traversal
-                              // launches, the per-category pixel counts and cursors of the
-                              // material-sorted order, and (kQueueCounter) the queued shadow rays
-  DevBuf<uint32_t> order;     // the pass's pixels grouped by material category (k_cat_scatter)
+                              // launches and (kQueueCounter) the queued shadow rays
+  DevBuf<uint32_t> order;     // the pass's pixels, each tile's grouped by material category (k_cat_order)
   // Sampled64 mode: material / light spectra, per-pixel sample spectra, film spectra
   DevBuf<float> spec_mats, spec_le, spec_L, spec_acc;
   DevBuf<uint32_t> spec_flags;  // per sample: a bin is not finite

@@ -79,69 +79,94 @@ __device__ __forceinline__ uint32_t prim_material(const SceneView& S, uint32_t p
 // (CBSDFConductorMicroface.cpp:84-115, CBSDFDielectricMicroface.cpp:84-115,
 // CBSDFSpecularReflectance.cpp:63-93) after the sphere or the triangle
 // surface-interaction job (CSSphere.cpp:122-186, CSTriangle.cpp:149-319).
-// The wavefront shades the pixels of a pass in that grouping: after the
-// camera traversal the pixels are ordered by category = primitive kind x
-// material type (2 x 5), camera misses (and scenes without lights) last, so
-// the spawn and finish kernels' warps mostly run one code path. Within a
-// category pixels keep their film order in runs of a block (one atomic per
-// block and category claims a run).
+// The wavefront shades the pixels of a pass in that grouping, tile by tile:
+// after the camera traversal the pixels of every run of kCatTile are ordered
+// by category = primitive kind x material type (2 x 5), camera misses (and
+// scenes without lights) last, so the spawn and finish kernels' warps mostly
+// run one code path. Within a category pixels keep their film order.
+//
+// One launch, a block a tile, no global atomics: at most ten of a tile's 256
+// warps hold two categories, and a tile's pixels stay near each other. Over
+// the whole film (a counting launch, then one that claimed runs by atomics)
+// the order took 36 us of a 1080p pass. 1080p x 16 spp, ms: whole film full
+// 10.70 / textured 9.19, tiles of 2,048 10.52 / 9.43, 8,192 10.20 / 9.02,
+// 16,384 10.35 / 8.89, 32,768 10.32 / 8.87; 1001 x 563 Sampled64 3.44, 3.54,
+// 3.45, 3.50, 3.52 (large tiles leave SMs idle).
 constexpr uint32_t kMatTypes = 5;                  // WPBR_MAT_CONDUCTOR .. WPBR_MAT_METAL_ISOTROPIC
 constexpr uint32_t kPixCats = 2 * kMatTypes + 1;   // last: misses
-constexpr uint32_t kCatBlock = 256;
-// Films of fewer pixels are shaded in film order: the two ordering launches
-// cost more than they save there (256x256 x 4 spp: 647 Msamples/s in film
-// order, 614 sorted; 1920x1080 x 64 spp: 1,276 in film order, 1,364 sorted).
+constexpr uint32_t kCatBlock = 512, kCatItems = 16;  // pixels per thread
+constexpr uint32_t kCatTile = kCatBlock * kCatItems;
+// Films of fewer pixels are shaded in film order: four passes of 256 x 256 in
+// film order / sorted, us: spheres 177 / 177, mesh 353 / 355, textured 396 /
+// 384, of 200 x 180 151 / 148, 311 / 316, 346 / 338.
 constexpr uint32_t kSortMinPixels = 1u << 17;
 
-__device__ __forceinline__ uint32_t pixel_category(const SceneView& S, uint32_t prim) {
-  if (prim == kNoHit || S.nlights == 0) return kPixCats - 1;
-  uint32_t t = S.mats[prim_material(S, prim)].type;
-  return (prim < S.ns ? 0u : kMatTypes) + (t < kMatTypes ? t : kMatTypes - 1);
-}
-
-// counts[0..kPixCats): pixels per category (zeroed before the pass)
-__global__ void __launch_bounds__(kCatBlock) k_cat_count(SceneView S, uint32_t n, const uint32_t* hit_prim,
-                                                         uint32_t* counts) {
-  __shared__ uint32_t s_cnt[kPixCats];
-  if (threadIdx.x < kPixCats) s_cnt[threadIdx.x] = 0;
+// order[]: the pixels of each tile grouped by category.
+__global__ void __launch_bounds__(kCatBlock) k_cat_order(SceneView S, uint32_t n, const uint32_t* hit_prim,
+                                                         uint32_t* order) {
+  constexpr uint32_t kWarps = kCatBlock / 32, kRuns = kCatItems * kWarps;  // a run: 32 pixels
+  constexpr uint32_t kPer = (kPixCats * kRuns + kCatBlock - 1) / kCatBlock;
+  __shared__ uint32_t s_at[kPer * kCatBlock];  // per category and run: pixels, then their start
+  __shared__ uint32_t s_sum[kWarps];
+  const uint32_t base = blockIdx.x * kCatTile, lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+  // a thread's loads go out together, level by level: hit, material, its type
+  uint32_t prim[kCatItems], m[kCatItems], c[kCatItems];
+#pragma unroll
+  for (uint32_t k = 0; k < kCatItems; ++k) {
+    const uint32_t i = base + k * kCatBlock + threadIdx.x;
+    prim[k] = i < n && S.nlights ? hit_prim[i] : kNoHit;
+  }
+#pragma unroll
+  for (uint32_t k = 0; k < kCatItems; ++k) {
+    const bool sph = prim[k] < S.ns;
+    const uint32_t* id = sph ? S.sph_mat + prim[k] : S.tri_mat + (prim[k] - S.ns);
+    m[k] = prim[k] != kNoHit ? *id : 0u;
+  }
+#pragma unroll
+  for (uint32_t k = 0; k < kCatItems; ++k) {
+    const uint32_t t = prim[k] != kNoHit ? S.mats[m[k]].type : 0u;
+    c[k] = (prim[k] < S.ns ? 0u : kMatTypes) + (t < kMatTypes ? t : kMatTypes - 1);
+    if (prim[k] == kNoHit) c[k] = kPixCats - 1;
+    if (base + k * kCatBlock + threadIdx.x >= n) c[k] = kPixCats;  // no pixel
+  }
+#pragma unroll
+  for (uint32_t q = 0; q < kPer; ++q) s_at[q * kCatBlock + threadIdx.x] = 0;
   __syncthreads();
-  uint32_t i = blockIdx.x * kCatBlock + threadIdx.x;
-  if (i < n) atomicAdd(&s_cnt[pixel_category(S, hit_prim[i])], 1u);
-  __syncthreads();
-  if (threadIdx.x < kPixCats && s_cnt[threadIdx.x]) atomicAdd(&counts[threadIdx.x], s_cnt[threadIdx.x]);
-}
-
-// order[]: the pixels grouped by category (category c starts at the sum of
-// the counts before it); cursor[0..kPixCats) zeroed before the pass.
-__global__ void __launch_bounds__(kCatBlock) k_cat_scatter(SceneView S, uint32_t n, const uint32_t* hit_prim,
-                                                           const uint32_t* counts, uint32_t* cursor,
-                                                           uint32_t* order, uint32_t* err) {
-  __shared__ uint32_t s_cnt[kPixCats], s_base[kPixCats];
-  if (threadIdx.x < kPixCats) s_cnt[threadIdx.x] = 0;
-  __syncthreads();
-  const uint32_t i = blockIdx.x * kCatBlock + threadIdx.x;
-  const uint32_t lane = threadIdx.x & 31u;
-  uint32_t c = i < n ? pixel_category(S, hit_prim[i]) : kPixCats;  // kPixCats: no pixel
-  uint32_t peers = __match_any_sync(0xFFFFFFFFu, c);
-  uint32_t leader = __ffs(peers) - 1u;
-  uint32_t wbase = 0;
-  if (lane == leader && c < kPixCats) wbase = atomicAdd(&s_cnt[c], (uint32_t)__popc(peers));
-  wbase = __shfl_sync(0xFFFFFFFFu, wbase, leader);
-  uint32_t rank = wbase + __popc(peers & ((1u << lane) - 1u));
-  __syncthreads();
-  if (threadIdx.x < kPixCats) {
-    uint32_t start = 0;
-    for (uint32_t k = 0; k < threadIdx.x; ++k) start += counts[k];
-    s_base[threadIdx.x] = s_cnt[threadIdx.x] ? start + atomicAdd(&cursor[threadIdx.x], s_cnt[threadIdx.x]) : 0u;
+  uint32_t rank[kCatItems];
+#pragma unroll
+  for (uint32_t k = 0; k < kCatItems; ++k) {
+    const uint32_t peers = __match_any_sync(0xFFFFFFFFu, c[k]);
+    rank[k] = __popc(peers & ((1u << lane) - 1u));
+    if (rank[k] == 0 && c[k] < kPixCats) s_at[c[k] * kRuns + k * kWarps + w] = __popc(peers);
   }
   __syncthreads();
-  if (c < kPixCats) {
-    uint32_t pos = s_base[c] + rank;  // < n when the counts are this pass's
-    if (pos < n)
-      order[pos] = i;
-    else
-      atomicOr(err, kErrBuild);
+  uint32_t v[kPer], sum = 0;
+#pragma unroll
+  for (uint32_t q = 0; q < kPer; ++q) {
+    v[q] = s_at[threadIdx.x * kPer + q];
+    sum += v[q];
   }
+  uint32_t x = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+    if (lane >= (uint32_t)o) x += y;
+  }
+  if (lane == 31) s_sum[w] = x;
+  __syncthreads();
+  uint32_t run = x - sum;
+#pragma unroll
+  for (uint32_t q = 0; q < kWarps; ++q) run += q < w ? s_sum[q] : 0u;
+#pragma unroll
+  for (uint32_t q = 0; q < kPer; ++q) {
+    s_at[threadIdx.x * kPer + q] = run;
+    run += v[q];
+  }
+  __syncthreads();
+#pragma unroll
+  for (uint32_t k = 0; k < kCatItems; ++k)
+    if (c[k] < kPixCats)
+      order[base + s_at[c[k] * kRuns + k * kWarps + w] + rank[k]] = base + k * kCatBlock + threadIdx.x;
 }
 
 // Full interaction for the winning primitive: re-runs its intersection test

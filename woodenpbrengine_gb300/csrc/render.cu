@@ -552,8 +552,6 @@ wpbr_status env_preprocess(wpbr_ctx* ctx) {
   return env_distribution_build(ctx, ctx->env_rgb.p, d, &ctx->env_marg_int);
 }
 
-static_assert(kQueueCounter == 2 + 2 * kPixCats, "pass counters: fetches, categories, then the queue");
-
 wpbr_status render_setup(wpbr_ctx* ctx, uint32_t spp, uint32_t seed, uint32_t stream) {
   if (!ctx->has_scene) return set_err(ctx, WPBR_ERR_NOT_BUILT, "render_setup: no scene");
   if (!ctx->bvh.built) return set_err(ctx, WPBR_ERR_NOT_BUILT, "render_setup: BVH not built");
@@ -645,10 +643,7 @@ wpbr_status pass_kernels(wpbr_ctx* ctx, const PassBufs& B, const uint32_t* pass_
   // the pixels in material-sorted order for the spawn and finish kernels
   const uint32_t* order = nullptr;
   if (n >= kSortMinPixels) {
-    uint32_t* cat_counts = counters + 2;
-    k_cat_count<<<div_up(n, kCatBlock), kCatBlock, 0, st>>>(P.S, n, B.hit_prim, cat_counts);
-    k_cat_scatter<<<div_up(n, kCatBlock), kCatBlock, 0, st>>>(P.S, n, B.hit_prim, cat_counts, cat_counts + kPixCats,
-                                                              B.order, P.err);
+    k_cat_order<<<div_up(n, kCatTile), kCatBlock, 0, st>>>(P.S, n, B.hit_prim, B.order);
     order = B.order;
   }
   if (spectral)
