@@ -3,7 +3,7 @@
 // A batch owns one wpbr_ctx per scene (scene buffers, per-pixel render state,
 // film) and one pooled device arena holding every scene's traversal layout
 // (Node2 array and primitive records, each block 256-byte aligned). A sample pass of all scenes is one CUDA graph: a fork event on the
-// batch stream, one branch per scene with the five kernels of the fused pass
+// batch stream, one branch per scene with the kernels of the fused pass
 // (render_pass_launch) on that scene's stream, and a join back. All branches
 // read the pass index from one device word, so a pass costs one 4-byte copy and
 // one graph launch whatever the number of scenes.

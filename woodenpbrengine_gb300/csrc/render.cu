@@ -6,7 +6,7 @@
 //    per-pixel state buffers, each recordable for stage-by-stage parity;
 //  * the fused path (wpbr_render_pass): camera+primary traversal, shading +
 //    sample generation (spawn), one traversal launch for both shadow rays,
-//    MIS finish, film gather — five kernels per sample pass, captured once as
+//    MIS finish, film gather — five kernels per sample pass (six on large films), captured once as
 //    a CUDA graph that reads the pass index from device memory.
 #include <algorithm>
 #include <cstring>
@@ -671,7 +671,7 @@ wpbr_status pass_kernels(wpbr_ctx* ctx, const PassBufs& B, const uint32_t* pass_
 }
 }  // namespace
 
-// Launches the five kernels of one sample pass on the context's stream. The
+// Launches the kernels of one sample pass on the context's stream. The
 // pass index is read from device memory (R.pass_ptr, shared across the scenes
 // of a batch, else R.pass_dev); R.trace_grid caps the persistent traversal
 // grids (0: one full wave of resident blocks).
@@ -695,7 +695,7 @@ wpbr_status render_pass_launch(wpbr_ctx* ctx) {
 
 // Everything the captured pass graph bakes into its kernel arguments: the
 // scene/BVH epoch, the sample-stream parameters, the film size and every
-// device pointer the five kernels receive.
+// device pointer the kernels receive.
 static uint64_t pass_graph_key(const wpbr_ctx* ctx) {
   const RenderState& R = ctx->rs;
   uint64_t h = 0xCBF29CE484222325ull;
@@ -735,7 +735,7 @@ wpbr_status render_pass_fused(wpbr_ctx* ctx, uint32_t pass) {
   }
   if (!R.graph_ok) {
     R.graph_key = key;
-    // capture the five kernels once; later passes replay the graph
+    // capture the kernels once; later passes replay the graph
     cudaGraph_t g = nullptr;
     if (cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
       wpbr_status s = render_pass_launch(ctx);
@@ -937,7 +937,7 @@ wpbr_status job_record(wpbr_ctx* ctx, uint32_t x0, uint32_t y0, uint32_t x1, uin
 
 // The accumulators as separate radiance and weight arrays, as the caller
 // receives them. Films are read through the pass state's memory, which every
-// pass writes before it reads (112 bytes a pixel), so a read allocates nothing
+// pass writes before it reads (128 bytes a pixel), so a read allocates nothing
 // and the host only receives the copies, into pages touched while the last
 // passes still run: splitting 1920 x 1080 float4s on the host, through a
 // vector of its own, took 3.4 ms, the copies alone take 0.24.
