@@ -344,12 +344,11 @@ constexpr int kPassStateF4 = 8;
 void bvh_release(wpbr_ctx* ctx, bool keep_traversal);
 wpbr_status job_run(wpbr_ctx* ctx, uint32_t job, uint32_t pass);
 wpbr_status job_record(wpbr_ctx* ctx, uint32_t x0, uint32_t y0, uint32_t x1, uint32_t y1, wpbr_pass_record* rec);
-// Write-touches every page of a caller's pageable host buffer that a copy will
-// fill, leaving its contents: called while the GPU still works on the result.
-// A copy into pages that were never touched takes their faults one by one on
-// the copy's side: 33 MB of a 1080p film 0.8 ms, and 8 to 40 ms while the
-// process's heap still grows, against 0.24 ms into touched pages (and 0.6 to
-// 1.1 ms to touch them).
+// Faults in for writing every page of a caller's pageable host buffer that a
+// copy will fill, leaving its contents: called while the GPU still works on
+// the result. A copy into pages that were never touched takes their faults one
+// by one on the copy's side: 33 MB of a 1080p film 12 ms, against 0.24 ms into
+// pages that are there (and 0.8 to 1.1 ms to fault them in).
 void touch_pages(void* host, size_t bytes);
 wpbr_status film_read(wpbr_ctx* ctx, float* acc_L, float* acc_w);
 wpbr_status film_tonemap(wpbr_ctx* ctx, uint8_t* out);
