@@ -91,7 +91,9 @@ __device__ __forceinline__ uint32_t prim_material(const SceneView& S, uint32_t p
 // the order took 36 us of a 1080p pass. 1080p x 16 spp, ms: whole film full
 // 10.70 / textured 9.19, tiles of 2,048 10.52 / 9.43, 8,192 10.20 / 9.02,
 // 16,384 10.35 / 8.89, 32,768 10.32 / 8.87; 1001 x 563 Sampled64 3.44, 3.54,
-// 3.45, 3.50, 3.52 (large tiles leave SMs idle).
+// 3.45, 3.50, 3.52 (large tiles leave SMs idle). (The spawn kernel alone is
+// slower for it, 91 -> 100 us: a tile's categories run side by side and its
+// warps wait more for instructions.)
 constexpr uint32_t kMatTypes = 5;                  // WPBR_MAT_CONDUCTOR .. WPBR_MAT_METAL_ISOTROPIC
 constexpr uint32_t kPixCats = 2 * kMatTypes + 1;   // last: misses
 constexpr uint32_t kCatBlock = 512, kCatItems = 16;  // pixels per thread
