@@ -60,3 +60,21 @@ def test_groups_without_capture_or_memory(W, spectral):
         ctx.set_stream(None)
         got = frame(W, ctx, res, spp)
         assert np.array_equal(got[0], one[0]) and np.array_equal(got[1], one[1])
+
+
+@pytest.mark.parametrize("spectral", [False, True])
+def test_each_group_allocation_may_fail(W, spectral):
+    # whichever of the group's buffers cannot be had, the frame renders one
+    # pass at a time in the buffers of render_setup, which stay usable
+    res, spp = (70, 41), 5
+    for budget in range(5):
+        with context(W, 2, res, spectral) as ctx:
+            ctx.render_setup(spp, seed=3, stream=1)
+            W.debug_fail_allocations(budget)
+            try:
+                ctx.render()
+            finally:
+                W.debug_fail_allocations(-1)
+            got = [a.view(np.uint32) for a in ctx.film(*res)]
+            one = frame(W, ctx, res, spp, one_by_one=True)
+            assert np.array_equal(got[0], one[0]) and np.array_equal(got[1], one[1]), budget

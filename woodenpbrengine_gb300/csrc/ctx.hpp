@@ -42,6 +42,17 @@ struct DevBuf {
     if (e == cudaSuccess) n = count;
     return e;
   }
+  // ensure, leaving the buffer as it was when the larger one cannot be had
+  // (both exist for a moment; contents are not carried over).
+  cudaError_t grow(size_t count) {
+    if (count <= n && p) return cudaSuccess;
+    DevBuf larger;
+    cudaError_t e = larger.ensure(count);
+    if (e != cudaSuccess) return e;
+    release();
+    *this = larger;
+    return e;
+  }
   void release() {
     if (p) cudaFree(p);
     p = nullptr;

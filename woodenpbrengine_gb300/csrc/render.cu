@@ -574,7 +574,7 @@ wpbr_status render_setup(wpbr_ctx* ctx, uint32_t spp, uint32_t seed, uint32_t st
   WPBR_CUDA(R.pstate.ensure(n * kStateF4));
   WPBR_CUDA(R.Lbuf.ensure(n));
   WPBR_CUDA(R.pfilm.ensure(n));
-  WPBR_CUDA(R.pass_dev.ensure(1));
+  WPBR_CUDA(R.pass_dev.ensure(RenderState::kMaxGroup));
   WPBR_CUDA(R.counters.ensure(kPassCounters));  // allocated before any graph capture
   WPBR_CUDA(R.order.ensure(n));
   WPBR_CUDA(cudaMemsetAsync(R.acc.p, 0, n * 4 * sizeof(float), ctx->stream));
@@ -835,16 +835,13 @@ wpbr_status render_frame(wpbr_ctx* ctx) {
   uint32_t K = R.pass_ptr ? 1u : group_size(R, spectral);
   if (K > 1) {
     // the group's buffers; a device without room for them renders one pass at
-    // a time, in the buffers render_setup made
+    // a time, in the buffers render_setup made (which a failure here leaves)
     cudaError_t e = R.slices.ensure((K - 1) * slice_bytes(n));
-    if (e == cudaSuccess) e = R.pass_dev.ensure(RenderState::kMaxGroup);
     if (e == cudaSuccess && spectral) e = spectral_slots(ctx, K);
     if (e == cudaErrorMemoryAllocation) {
       cudaGetLastError();
       R.slices.release();
       K = 1;
-      WPBR_CUDA(R.pass_dev.ensure(1));
-      if (spectral) WPBR_CUDA(spectral_slots(ctx, 1));
     } else {
       WPBR_CUDA(e);
     }

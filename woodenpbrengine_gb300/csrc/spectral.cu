@@ -691,13 +691,14 @@ static PassCtx spec_pass_ctx(wpbr_ctx* ctx) {
                   ctx->rs.W, ctx->rs.H, ctx->d_err.p);
 }
 
-// Room for `slots` passes' film positions and sample spectra.
+// Room for `slots` passes' film positions and sample spectra; without it the
+// slots that are there stay.
 cudaError_t spectral_slots(wpbr_ctx* ctx, uint32_t slots) {
   RenderState& R = ctx->rs;
   const size_t n = (size_t)R.W * R.H;
-  cudaError_t e = R.pfilm.ensure(slots * n);
-  if (e == cudaSuccess) e = R.spec_L.ensure(slots * n * kSpecN);
-  if (e == cudaSuccess) e = R.spec_flags.ensure(slots * n);
+  cudaError_t e = R.pfilm.grow(slots * n);
+  if (e == cudaSuccess) e = R.spec_L.grow(slots * n * kSpecN);
+  if (e == cudaSuccess) e = R.spec_flags.grow(slots * n);
   return e;
 }
 
