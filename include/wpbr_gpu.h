@@ -59,6 +59,10 @@ typedef struct wpbr_ctx wpbr_ctx;
 WPBR_API wpbr_status wpbr_create(int device, wpbr_ctx** out);
 WPBR_API void wpbr_destroy(wpbr_ctx* ctx);
 WPBR_API const char* wpbr_last_error(const wpbr_ctx* ctx);
+/* Later calls work on cuda_stream. A stream of the caller's is not ordered
+ * with the one set before it: work still queued there (an asynchronous render,
+ * say) is to be waited for, by an event or on the host, before calls that
+ * depend on it. */
 WPBR_API wpbr_status wpbr_set_stream(wpbr_ctx* ctx, void* cuda_stream);
 WPBR_API void* wpbr_get_stream(const wpbr_ctx* ctx);
 /* wpbr_quirk bits (wpbr_scene.h); applies to later builds and renders. */

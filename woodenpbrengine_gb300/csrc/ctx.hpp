@@ -137,6 +137,7 @@ struct RenderState {
   // Sampled64 mode: material / light spectra, per-pixel sample spectra, film spectra
   DevBuf<float> spec_mats, spec_le, spec_L, spec_acc;
   DevBuf<uint32_t> spec_flags;  // per sample: a bin is not finite
+  DevBuf<float> film_out;   // what film_read and film_tonemap copy to the host
   bool spec_dirty = false;  // Sampled64 passes ran since the last toRGB of the film
   const uint32_t* pass_ptr = nullptr;  // shared pass index (batches); null: pass_dev
   uint32_t trace_grid = 0;             // persistent traversal grid cap (0: full)

@@ -933,15 +933,17 @@ wpbr_status job_record(wpbr_ctx* ctx, uint32_t x0, uint32_t y0, uint32_t x1, uin
 }
 
 // The accumulators as separate radiance and weight arrays, as the caller
-// receives them. Films are read through the pass state's memory, which every
-// pass writes before it reads (128 bytes a pixel), so a read allocates nothing
-// and the host only receives the copies, into pages touched while the last
-// passes still run: splitting 1920 x 1080 float4s on the host, through a
-// vector of its own, took 3.4 ms, the copies alone take 0.24.
+// receives them. Larger films are split on the device into a buffer that reads
+// alone use (the pass state's memory would do, but a caller may read on one
+// stream while passes still run on another), so the host only receives the
+// copies, into pages touched while the last passes still run: splitting 1920 x
+// 1080 float4s on the host, through a vector of its own, took 3.4 ms, the
+// copies alone take 0.24.
 //
-// Films of at most kFilmHostSplit pixels are copied as they are and split on
-// the host: one copy instead of a launch and two. us a read, host / device
-// split: 64 x 64 28 / 42, 96 x 96 38 / 44, 128 x 128 51 / 49, 256 x 256 120 / 68.
+// Films of at most kFilmHostSplit pixels, and films that there is no device
+// memory to split, are copied as they are and split on the host: one copy
+// instead of a launch and two. us a read, host / device split: 64 x 64 28 / 42,
+// 96 x 96 38 / 44, 128 x 128 51 / 49, 256 x 256 120 / 68.
 constexpr uint32_t kFilmHostSplit = 12288;
 wpbr_status film_read(wpbr_ctx* ctx, float* acc_L, float* acc_w) {
   RenderState& R = ctx->rs;
@@ -949,10 +951,9 @@ wpbr_status film_read(wpbr_ctx* ctx, float* acc_L, float* acc_w) {
   wpbr_status rs = spectral_resolve(ctx);
   if (rs != WPBR_OK) return rs;
   const uint32_t n = R.W * R.H;
-  static_assert(kStateF4 >= 1, "four floats a pixel of scratch");
-  float* L = (float*)R.pstate.p;
-  float* w = L + 3 * (size_t)n;
-  if (n <= kFilmHostSplit) {
+  cudaError_t e = n > kFilmHostSplit ? R.film_out.ensure(4 * (size_t)n) : cudaErrorMemoryAllocation;
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
     std::vector<float4> a(n);
     WPBR_CUDA(cudaMemcpyAsync(a.data(), R.acc.p, (size_t)n * 16, cudaMemcpyDeviceToHost, ctx->stream));
     WPBR_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -966,6 +967,9 @@ wpbr_status film_read(wpbr_ctx* ctx, float* acc_L, float* acc_w) {
     }
     return WPBR_OK;
   }
+  WPBR_CUDA(e);
+  float* L = R.film_out.p;
+  float* w = L + 3 * (size_t)n;
   k_film_split<<<div_up(n, 256), 256, 0, ctx->stream>>>(n, (const float4*)R.acc.p, L, w);
   WPBR_CUDA(cudaGetLastError());
   touch_pages(acc_L, (size_t)n * 12);
@@ -982,7 +986,8 @@ wpbr_status film_tonemap(wpbr_ctx* ctx, uint8_t* out) {
   wpbr_status rs = spectral_resolve(ctx);
   if (rs != WPBR_OK) return rs;
   uint32_t n = R.W * R.H;
-  uint8_t* rgb8 = (uint8_t*)R.pstate.p;  // as film_read
+  WPBR_CUDA(R.film_out.ensure(((size_t)n * 3 + 3) / 4));  // as film_read
+  uint8_t* rgb8 = (uint8_t*)R.film_out.p;
   k_tonemap<<<div_up(n, 256), 256, 0, ctx->stream>>>(n, (const float4*)R.acc.p, rgb8);
   WPBR_CUDA(cudaGetLastError());
   touch_pages(out, (size_t)n * 3);
