@@ -45,3 +45,8 @@ def test_non_finite_samples(W, O, ctx, spp):
         assert not np.isfinite(L).all() and np.isfinite(L).any()
     finally:
         rgb[:] = keep
+
+
+def test_more_rows_than_a_grid_dimension_of_blocks(W, O, ctx):
+    # 4 pixel rows a block: more than 65,535 rows of blocks
+    _film(W, O, ctx, W.SceneGen(0, 6, (1, 262150)), (1, 262150), 1, 8)

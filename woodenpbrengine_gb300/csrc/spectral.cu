@@ -469,7 +469,9 @@ __global__ void __launch_bounds__(kFilmThreads, 3) k_sfilm(uint32_t W, uint32_t 
   float(*s_mx)[kSPad] = reinterpret_cast<float(*)[kSPad]>(sfilm_smem + kSSamples * kSpecN);  // [5]
   float(*s_my)[kSPad] = s_mx + 5;                              // [5]
   const int tid = (int)threadIdx.x;
-  const int bx0 = (int)blockIdx.x * kFilmTile, by0 = (int)blockIdx.y * kSRows;
+  // blocks in one dimension, row by row: a grid's second one ends at 65,535
+  const uint32_t nx = (W + kFilmTile - 1) / kFilmTile;
+  const int bx0 = (int)(blockIdx.x % nx) * kFilmTile, by0 = (int)(blockIdx.x / nx) * kSRows;
   const int ty0 = by0 / 32 * 32;
   const int tx1 = min(bx0 + 31, (int)W - 1), ty1 = min(ty0 + 31, (int)H - 1);
   const int q = tid % 4, lx = tid / 4 % kFilmTile, ly = tid / (4 * kFilmTile) * 2;
@@ -734,8 +736,8 @@ cudaError_t spectral_film_launch(wpbr_ctx* ctx, uint32_t film_slots, cudaStream_
   cudaError_t e = cudaFuncSetAttribute((const void*)k_sfilm, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)kSFilmSmem);
   if (e != cudaSuccess) return e;
-  dim3 fg(div_up(R.W, kFilmTile), div_up(R.H, kSRows));
-  k_sfilm<<<fg, kFilmThreads, kSFilmSmem, st>>>(R.W, R.H, R.pfilm.p, R.spec_L.p, R.spec_flags.p, film_slots,
+  const unsigned blocks = div_up(R.W, kFilmTile) * div_up(R.H, kSRows);
+  k_sfilm<<<blocks, kFilmThreads, kSFilmSmem, st>>>(R.W, R.H, R.pfilm.p, R.spec_L.p, R.spec_flags.p, film_slots,
                                                  R.spec_acc.p, (float4*)R.acc.p, kOnes);
   return cudaGetLastError();
 }
