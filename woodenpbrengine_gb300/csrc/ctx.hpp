@@ -345,7 +345,7 @@ struct PassBufs {
 // spectra side by side and gathers them into the film at once.
 cudaError_t spectral_slots(wpbr_ctx* ctx, uint32_t slots);
 cudaError_t spectral_spawn_launch(wpbr_ctx* ctx, const PassBufs& B, const uint32_t* pass_ptr, const uint32_t* order,
-                                  uint32_t slot, cudaStream_t st);
+                                  uint32_t slot, int tex, cudaStream_t st);
 cudaError_t spectral_finish_launch(wpbr_ctx* ctx, const PassBufs& B, const uint32_t* order, uint32_t slot,
                                    cudaStream_t st);
 cudaError_t spectral_film_launch(wpbr_ctx* ctx, uint32_t film_slots, cudaStream_t st);

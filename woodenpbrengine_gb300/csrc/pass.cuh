@@ -32,6 +32,23 @@ constexpr int kTB = 128;
 #ifndef WPBR_SPAWN_TEX_MIN_BLOCKS
 #define WPBR_SPAWN_TEX_MIN_BLOCKS 7
 #endif
+// Textured spawns come in two builds. With few pixels in flight a launch lasts
+// as long as its slowest warps: the wide one has a copy of every lookup and as
+// many registers as it likes (95, none spilled). With many the compact one
+// wins, at 7 blocks and with the lookups in loops (texture.cuh). Compact /
+// wide, us: one RGB pass of 256 x 256 320 / 198, 512 x 512 374 / 269, 1080p 823 /
+// 733; frames of 2 passes of 1080p 1,276 / 1,247, 4 of 1280 x 800 1,501 /
+// 1,359, 16 (8 at a time) of 1001 x 563 3,082 / 3,076, of 1280 x 800 4,848 /
+// 5,199, 4 of 1080p 2,232 / 2,373; Sampled64, one of 512 x 512 483 / 381, 4 of
+// 1001 x 563 1,685 / 1,656, of 1280 x 800 2,838 / 2,905, of 1080p 5,489 / 5,622.
+enum : int { kTexNone, kTexWide, kTexCompact };
+constexpr uint64_t kTexWideMax = 1ull << 22, kTexWideMaxSpectral = 3ull << 20;  // pixels in flight
+inline int tex_build(bool textured, bool spectral, uint64_t pixels) {
+  return !textured ? kTexNone : (pixels <= (spectral ? kTexWideMaxSpectral : kTexWideMax) ? kTexWide : kTexCompact);
+}
+constexpr int spawn_min_blocks(int tex) {
+  return tex == kTexNone ? WPBR_SPAWN_MIN_BLOCKS : (tex == kTexWide ? 1 : WPBR_SPAWN_TEX_MIN_BLOCKS);
+}
 // The differentiable estimator's spawn: forward 4.06 -> 3.84 ms at 12 blocks
 // (512x512 x 16 spp).
 #ifndef WPBR_ADJ_SPAWN_MIN_BLOCKS
@@ -200,16 +217,17 @@ __device__ SurfInt make_si(const SceneView& S, uint32_t prim, V3 o, V3 d) {
 // The material of a hit: the scene's, or for textured metal the conductor
 // built from its textures at the hit's footprint (camera-ray differentials,
 // sphere or uv mapping).
-// TEX = false compiles the texture path out, for scenes without textured
+// TEX = kTexNone compiles the texture path out, for scenes without textured
 // materials (the context knows: has_metal).
-template <bool TEX = true>
+template <int TEX>
 __device__ wpbr_material hit_material(const SceneView& S, uint32_t prim, uint32_t mid, const SurfInt& s,
                                       const RayD& r) {
   wpbr_material m = S.mats[mid];
-  if (!TEX || !WPBR_MAT_TEXTURED(m.type)) return m;
+  if (TEX == kTexNone || !WPBR_MAT_TEXTURED(m.type)) return m;
   SurfDiff D = surf_differentials(s, r);
-  TexFootprint fp = prim < S.ns ? sphere_footprint(S.sph_w2o[prim], s, D) : uv_footprint(s, D);
-  return metal_material(S.tex, m, fp);
+  constexpr bool kCompact = TEX == kTexCompact;
+  TexFootprint fp = prim < S.ns ? sphere_footprint<kCompact>(S.sph_w2o[prim], s, D) : uv_footprint(s, D);
+  return metal_material<kCompact>(S.tex, m, fp);
 }
 // The part of a textured-metal material that varies per hit, packed in a
 // float4 (alpha, k.rgb), and its inverse.

@@ -113,7 +113,7 @@ __global__ void kj_bsdf_setup(PassCtx P, Staged G) {
     // JobGenerateBSDFMaterialMetal (MEngine.cpp:399-403)
     RayD r = camera_ray(P.S.cam, G.f[F_PFILM][2 * pix], G.f[F_PFILM][2 * pix + 1]);
     SurfInt hs = make_si(P.S, prim, r.o, r.d);
-    float4 v = metal_pack(hit_material(P.S, prim, mid, hs, r));
+    float4 v = metal_pack(hit_material<kTexWide>(P.S, prim, mid, hs, r));
     float* q = G.f[F_MAT] + 4 * (size_t)pix;
     q[0] = v.x; q[1] = v.y; q[2] = v.z; q[3] = v.w;
   }
@@ -255,8 +255,8 @@ enum : int { ST_BWI, ST_P, ST_BF, ST_METAL, ST_LI, ST_WI, ST_WO };  // float4 of
 static_assert(kStateF4 == 8, "a 128-byte line");
 enum : uint32_t { SF_TRACE_L = 2u, SF_TRACE_B = 4u, SF_METAL = 16u };
 
-template <bool TEX>
-__global__ void __launch_bounds__(kTB, TEX ? WPBR_SPAWN_TEX_MIN_BLOCKS : WPBR_SPAWN_MIN_BLOCKS) k_spawn(PassCtx P, const uint32_t* pass_dev, const uint32_t* hit_prim,
+template <int TEX>
+__global__ void __launch_bounds__(kTB, spawn_min_blocks(TEX)) k_spawn(PassCtx P, const uint32_t* pass_dev, const uint32_t* hit_prim,
                                                float4* state, ShadowQueue sq, float4* Lb, float2* pf,
                                                const uint32_t* order) {
   uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(kTB, TEX ? WPBR_SPAWN_TEX_MIN_BLOCKS : WPBR_SP
   Frame fr = bsdf_frame(s);
   uint32_t mid = prim_material(P.S, prim);
   const wpbr_material m = hit_material<TEX>(P.S, prim, mid, s, r);
-  if (TEX && WPBR_MAT_TEXTURED(P.S.mats[mid].type)) {
+  if (TEX != kTexNone && WPBR_MAT_TEXTURED(P.S.mats[mid].type)) {
     flags |= SF_METAL;
     st[ST_METAL] = metal_pack(m);
   }
@@ -646,11 +646,12 @@ wpbr_status pass_kernels(wpbr_ctx* ctx, const PassBufs& B, const uint32_t* pass_
     k_cat_order<<<div_up(n, kCatTile), kCatBlock, 0, st>>>(P.S, n, B.hit_prim, B.order);
     order = B.order;
   }
+  const int tex = tex_build(ctx->has_metal, spectral, (uint64_t)n * share);
   if (spectral)
-    WPBR_CUDA(spectral_spawn_launch(ctx, B, pass_ptr, order, spec_slot, st));
+    WPBR_CUDA(spectral_spawn_launch(ctx, B, pass_ptr, order, spec_slot, tex, st));
   else
-    (ctx->has_metal ? k_spawn<true> : k_spawn<false>)<<<div_up(n, kTB), kTB, 0, st>>>(
-        P, pass_ptr, B.hit_prim, B.pstate, sq, B.Lbuf, B.pfilm, order);
+    (tex == kTexNone ? k_spawn<kTexNone> : tex == kTexWide ? k_spawn<kTexWide> : k_spawn<kTexCompact>)
+        <<<div_up(n, kTB), kTB, 0, st>>>(P, pass_ptr, B.hit_prim, B.pstate, sq, B.Lbuf, B.pfilm, order);
   // shadow rays: unoccluded iff no hit or the closest hit is the sampled
   // light's primitive; with environment lights only that is "no hit", which
   // the any-hit traversal decides with the same primitive tests, stopping at

@@ -135,8 +135,8 @@ __device__ __forceinline__ FScalars f_scalars(const wpbr_material& m, float d_wh
   return F;
 }
 
-template <bool TEX>
-__global__ void __launch_bounds__(kTB, TEX ? WPBR_SPAWN_TEX_MIN_BLOCKS : WPBR_SPAWN_MIN_BLOCKS) k_sspawn(PassCtx P, const uint32_t* pass_dev, const uint32_t* hit_prim,
+template <int TEX>
+__global__ void __launch_bounds__(kTB, spawn_min_blocks(TEX)) k_sspawn(PassCtx P, const uint32_t* pass_dev, const uint32_t* hit_prim,
                                                 float4* state, ShadowQueue sq, float2* pf, const uint32_t* order) {
   uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
   if (slot >= P.W * P.H) return;
@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(kTB, TEX ? WPBR_SPAWN_TEX_MIN_BLOCKS : WPBR_SP
   Frame fr = bsdf_frame(si);
   uint32_t mid = prim_material(P.S, prim);
   const wpbr_material m = hit_material<TEX>(P.S, prim, mid, si, r);
-  if (TEX && WPBR_MAT_TEXTURED(P.S.mats[mid].type)) {
+  if (TEX != kTexNone && WPBR_MAT_TEXTURED(P.S.mats[mid].type)) {
     flags |= SS_TEX;
     st[4] = make_float4(m.k[0], m.k[1], m.k[2], 0.0f);
   }
@@ -706,14 +706,15 @@ cudaError_t spectral_slots(wpbr_ctx* ctx, uint32_t slots) {
 
 // The scalar spawn of the Sampled64 pass, between the camera traversal and
 // the shadow-ray traversal (render_pass_launch); the pass's film positions go
-// to sample slot `slot`.
+// to sample slot `slot`; tex: tex_build of the pass.
 cudaError_t spectral_spawn_launch(wpbr_ctx* ctx, const PassBufs& B, const uint32_t* pass_ptr, const uint32_t* order,
-                                  uint32_t slot, cudaStream_t st) {
+                                  uint32_t slot, int tex, cudaStream_t st) {
   RenderState& R = ctx->rs;
   uint32_t n = R.W * R.H;
   const ShadowQueue sq{B.shadow_rays, B.shadow_map, B.counters + kQueueCounter};
-  (ctx->has_metal ? k_sspawn<true> : k_sspawn<false>)<<<div_up(n, kTB), kTB, 0, st>>>(
-      spec_pass_ctx(ctx), pass_ptr, B.hit_prim, B.pstate, sq, R.pfilm.p + (size_t)slot * n, order);
+  (tex == kTexNone ? k_sspawn<kTexNone> : tex == kTexWide ? k_sspawn<kTexWide> : k_sspawn<kTexCompact>)
+      <<<div_up(n, kTB), kTB, 0, st>>>(spec_pass_ctx(ctx), pass_ptr, B.hit_prim, B.pstate, sq,
+                                       R.pfilm.p + (size_t)slot * n, order);
   return cudaGetLastError();
 }
 

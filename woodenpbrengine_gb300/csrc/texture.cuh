@@ -66,6 +66,7 @@ WPBR_HD RGB3 tex_triangle(const TexView& T, const TexInfo& ti, V2 st, uint32_t m
 }
 
 // Elliptically weighted average over one level with the Gaussian table.
+template <bool COMPACT>
 WPBR_HD RGB3 tex_ewa(const TexView& T, const TexInfo& ti, const TexFootprint& fp, uint32_t mip) {
   const TexLevel& L = T.levels[ti.first_level + mip];
   float rx = (float)L.w, ry = (float)L.h;
@@ -94,9 +95,25 @@ WPBR_HD RGB3 tex_ewa(const TexView& T, const TexInfo& ti, const TexFootprint& fp
   }
   RGB3 sum = rgb1(0.0f);
   float sw = 0.0f;
+  // The weight's index needs no upper clamp: r2 < 1.
+  if constexpr (!COMPACT) {
+    for (int it = it0; it <= it1; ++it) {
+      const float tt = (float)it - sy;
+      for (int is = is0; is <= is1; ++is) {
+        const float ss = (float)is - sx;
+        const float r2 = ((A * ss) * ss + (B * ss) * tt) + (C * tt) * tt;
+        if (r2 < 1.0f) {
+          const float w = T.gauss[(int)(r2 * (float)kGaussTable)];
+          sum = radd(sum, rmuls(tex_texel(T, L, is, it), w));
+          sw = sw + w;
+        }
+      }
+    }
+    return RGB3{sum.r / sw, sum.g / sw, sum.b / sw};
+  }
   // Two texels of a row at a time, their loads together; a texel outside the
   // ellipse adds zeros, which change no sum (one that starts at +0 never
-  // becomes -0). The weight's index needs no upper clamp: r2 < 1.
+  // becomes -0).
 #pragma unroll 1
   for (int it = it0; it <= it1; ++it) {
     const float tt = (float)it - sy;
@@ -146,13 +163,15 @@ WPBR_HD float log2_(float x) { return mul_const(logf_(x), kLog2eMul); }
 // finest level, a level at or past the coarsest reads texel (0, 0) of the
 // coarsest level, otherwise two levels are blended.
 //
-// The lookups stand in a loop, as do the two textures of a material and the
-// three points of a spherical footprint: with a copy of each at every use (4
-// EWA with their inner loops unrolled, 8 bilinear, 6 inverse trigonometric, 4
-// logarithms) the textured spawn kernel's warps spent 44 % of their time
-// waiting for instructions, now 27 %. A 1080p frame of 16 spp: 10.0 -> 9.68 ms
-// with the loops, 9.22 with the EWA loops not unrolled, 9.13 with two texels a
-// step.
+// COMPACT: the lookups stand in a loop, as do the two textures of a material
+// and the three points of a spherical footprint, and the EWA loops are not
+// unrolled: with a copy of each at every use (4 EWA with their inner loops
+// unrolled, 8 bilinear, 6 inverse trigonometric, 4 logarithms) the textured
+// spawn kernel's warps spent 44 % of their time waiting for instructions, now
+// 27 %. A 1080p frame of 16 spp: 10.0 -> 9.68 ms with the loops, 9.22 with the
+// EWA loops not unrolled, 9.13 with two texels a step. Where few pixels are in
+// flight the copies' shorter chains count instead (kTexWideMax).
+template <bool COMPACT>
 WPBR_HD RGB3 tex_eval(const TexView& T, uint32_t texid, const TexFootprint& fp, bool iso) {
   const TexInfo& ti = T.tex[texid];
   const uint32_t n = ti.n_levels;
@@ -196,10 +215,18 @@ WPBR_HD RGB3 tex_eval(const TexView& T, uint32_t texid, const TexFootprint& fp, 
       lookups = 2;
     }
   }
+  if constexpr (!COMPACT) {
+    if (!ewa) {
+      const RGB3 v = tex_triangle(T, ti, fp.p, mip);
+      return lookups == 1 ? v : rlerp(t, v, tex_triangle(T, ti, fp.p, mip + 1));
+    }
+    const RGB3 v = tex_ewa<COMPACT>(T, ti, fp, mip);
+    return lookups == 1 ? v : rlerp(t, v, tex_ewa<COMPACT>(T, ti, fp, mip + 1));
+  }
   RGB3 c = rgb1(0.0f);
 #pragma unroll 1
   for (uint32_t k = 0; k < lookups; ++k) {
-    const RGB3 v = ewa ? tex_ewa(T, ti, fp, mip + k) : tex_triangle(T, ti, fp.p, mip + k);
+    const RGB3 v = ewa ? tex_ewa<COMPACT>(T, ti, fp, mip + k) : tex_triangle(T, ti, fp.p, mip + k);
     c = k ? rlerp(t, c, v) : v;
   }
   return c;
@@ -263,11 +290,12 @@ WPBR_HD float sphere_wrap(float x) {
   return x;
 }
 
+template <bool COMPACT>
 WPBR_HD TexFootprint sphere_footprint(const Xf& w2o, const SurfInt& s, const SurfDiff& D) {
   TexFootprint fp;
   const float dt = 0.1f;
   V2 st = V2{0.0f, 0.0f}, stdx = st, stdy = st;
-#pragma unroll 1
+#pragma unroll (COMPACT ? 1 : 3)
   for (int k = 0; k < 3; ++k) {
     const V3 off = mul(k == 1 ? D.dpdx : D.dpdy, dt);
     const V2 v = sphere_st(w2o, k == 0 ? s.p : add(s.p, off));
@@ -301,13 +329,14 @@ WPBR_HD float roughness_to_alpha(float r) {
 }
 
 // JobGenerateBSDFMaterialMetal: the conductor of one hit.
+template <bool COMPACT>
 WPBR_HD wpbr_material metal_material(const TexView& T, const wpbr_material& m, const TexFootprint& fp) {
   bool iso = m.type == WPBR_MAT_METAL_ISOTROPIC;
   RGB3 metallic = rgb1(0.0f), rough = metallic;
-#pragma unroll 1
+#pragma unroll (COMPACT ? 1 : 2)
   for (int k = 0; k < 2; ++k) {
     metallic = rough;
-    rough = tex_eval(T, k ? m.tex[1] : m.tex[0], fp, iso);
+    rough = tex_eval<COMPACT>(T, k ? m.tex[1] : m.tex[0], fp, iso);
   }
   float sv = clampf(rough.r * 90.0f, 0.0f, 90.0f);
   float alpha = roughness_to_alpha(sv);
