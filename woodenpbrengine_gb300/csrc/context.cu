@@ -668,7 +668,6 @@ static wpbr_status collide_pipelined(wpbr_ctx* ctx, const float* rays, uint64_t 
   // copies already queued read `rays` and write `hits`, so all four streams
   // are drained before the call returns, whatever happened.
   wpbr_status s = WPBR_OK;
-  bool touched = false;
   cudaError_t ce = cudaSuccess;
   const char* what = "collide";
   for (int i = 0; i < 4; ++i) {
@@ -686,8 +685,9 @@ static wpbr_status collide_pipelined(wpbr_ctx* ctx, const float* rays, uint64_t 
     if (s != WPBR_OK) break;
     ce = cudaEventRecord(ctx->io_ev[1], cs);
     if (ce == cudaSuccess) ce = cudaStreamWaitEvent(ctx->io_d2h, ctx->io_ev[1], 0);
-    if (!touched) touch_pages(hits, 16 * n);  // while the first chunk is traced
-    touched = true;
+    // the chunk's pages alone, while it is traced: all pages at the first chunk
+    // left the device waiting (6 M rays into new memory 8.45 ms, 6.3 so)
+    touch_pages(hits + 4 * off, 16 * c);
     if (ce == cudaSuccess)
       ce = cudaMemcpyAsync(hits + 4 * off, ctx->io_hits.p + off, 16 * c, cudaMemcpyDeviceToHost, ctx->io_d2h);
     if (ce != cudaSuccess) {
