@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "camera.cuh"
+#include "pass_groups.hpp"
 #include "views.cuh"
 #include "wpbr_gpu.h"
 
@@ -146,7 +147,7 @@ struct RenderState {
   // graph, each on its own stream, state slice and pass index word. Slice 0
   // is the buffers above, the others lie in `slices`; a frame has at most two
   // graphs, one for its whole groups and one for the passes left over.
-  static constexpr uint32_t kMaxGroup = 8;
+  static constexpr uint32_t kMaxGroup = kMaxGroupPasses;
   struct GroupGraph {
     cudaGraphExec_t exec = nullptr;
     uint64_t key = 0;
@@ -343,6 +344,7 @@ struct PassBufs {
 // `order`: the material-sorted pixel order (null: film order).
 // Sample slots: a Sampled64 frame writes `slots` passes' film positions and
 // spectra side by side and gathers them into the film at once.
+size_t spectral_slot_bytes(size_t pixels);
 cudaError_t spectral_slots(wpbr_ctx* ctx, uint32_t slots);
 cudaError_t spectral_spawn_launch(wpbr_ctx* ctx, const PassBufs& B, const uint32_t* pass_ptr, const uint32_t* order,
                                   uint32_t slot, int tex, cudaStream_t st);

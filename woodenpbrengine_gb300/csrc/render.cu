@@ -14,6 +14,7 @@
 #include "common.cuh"
 #include "ctx.hpp"
 #include "pass.cuh"
+#include "pass_groups.hpp"
 #include "traverse.cuh"
 #include "traverse_persistent.cuh"
 
@@ -755,21 +756,6 @@ wpbr_status render_pass_fused(wpbr_ctx* ctx, uint32_t pass) {
   return WPBR_OK;
 }
 
-// Passes per group of a frame. A traversal launch ends with a tail in which
-// most of its warps have no ray left (1080p full frame: 31 to 41 % of the warp
-// slots active over the launch), and a small film never fills the GPU at all,
-// so the passes of a group run as concurrent branches and fill one another's
-// tails. 1080p x 16 spp, full frame / textured, groups of 1: 19.9 / 14.6 ms;
-// 2: 16.0 / 14.1; 4: 15.2 / 13.8; 8: 14.8 / 13.6. A Sampled64 pass also keeps a
-// slot of 64-bin samples per pixel until the group's film gather, so those
-// groups stop at 4. Groups are bounded to 2^24 pixels of state (3.8 GB);
-// larger films render fewer passes at a time.
-uint32_t group_size(const RenderState& R, bool spectral) {
-  const uint64_t n = (uint64_t)R.W * R.H;
-  const uint64_t k = std::max<uint64_t>(1u, (1ull << 24) / n);
-  return (uint32_t)std::min<uint64_t>({k, R.spp, spectral ? 4u : RenderState::kMaxGroup});
-}
-
 // Captures (or reuses) the graph of a group of K passes. RGB: K branches, each
 // pass in its own state slice, and the film gathers in pass order on the
 // context's stream, each as soon as its branch is done. Sampled64: K branches
@@ -833,7 +819,13 @@ wpbr_status render_frame(wpbr_ctx* ctx) {
   if (!R.ready) return set_err(ctx, WPBR_ERR_NOT_BUILT, "render: render_setup not called");
   const size_t n = (size_t)R.W * R.H;
   const bool spectral = ctx->spectrum == WPBR_SPECTRUM_SAMPLED64;
-  uint32_t K = R.pass_ptr ? 1u : group_size(R, spectral);
+  uint32_t K = R.pass_ptr ? 1u : group_passes(n, R.spp, spectral);
+  const size_t slot_bytes = spectral ? spectral_slot_bytes(n) : 0;
+  if (K > 1 && (R.slices.n < (K - 1) * slice_bytes(n) || (spectral && R.spec_flags.n < K * n))) {
+    size_t room = 0, total = 0;
+    WPBR_CUDA(cudaMemGetInfo(&room, &total));
+    K = group_passes_within(K, slice_bytes(n) + slot_bytes, room + R.slices.n);  // the old slices go first
+  }
   if (K > 1) {
     // the group's buffers; a device without room for them renders one pass at
     // a time, in the buffers render_setup made (which a failure here leaves)

@@ -693,6 +693,8 @@ static PassCtx spec_pass_ctx(wpbr_ctx* ctx) {
                   ctx->rs.W, ctx->rs.H, ctx->d_err.p);
 }
 
+size_t spectral_slot_bytes(size_t pixels) { return pixels * (sizeof(float2) + kSpecN * sizeof(float) + sizeof(uint32_t)); }
+
 // Room for `slots` passes' film positions and sample spectra; without it the
 // slots that are there stay.
 cudaError_t spectral_slots(wpbr_ctx* ctx, uint32_t slots) {
