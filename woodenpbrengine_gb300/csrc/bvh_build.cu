@@ -971,7 +971,10 @@ constexpr int kCoopPerSM = 1024 / kCoopBlock;  // resident blocks per SM (64 reg
 constexpr int kCoopWarps = kCoopBlock / 32;
 constexpr uint32_t kMaxCoopGrid = 1024;  // blocks of the cooperative grid (chunk prefixes in shared memory)
 static_assert(kMaxCoopGrid <= 2 * kCoopBlock, "block_scan_pairs scans two entries a thread");
-constexpr uint32_t kSpinLimit = 1u << 22;   // barrier polls (about half a microsecond each) before giving up
+// Barrier polls (a load from L2 each, half a microsecond and more) before
+// giving up: some ten seconds. Blocks may have to wait for other streams'
+// kernels to leave their SMs, so the bound is one of time, not of work.
+constexpr uint32_t kSpinLimit = 1u << 24;
 constexpr unsigned long long kBarAbort = 1ull << 63;
 constexpr uint32_t kSegWords = 12;          // bounds lo/hi, centroid bounds lo/hi (encoded)
 constexpr uint32_t kBucketWords = 12 * 7;   // per bucket: count, lo xyz, hi xyz (encoded)
