@@ -36,3 +36,27 @@ def test_scene_kinds(W, O, ctx, config, level, extent, n):
     assert np.array_equal(hg[at].view(np.uint32), ho.view(np.uint32))
     assert np.array_equal(np.isfinite(ag[:, 0]), np.isfinite(hg[:, 0]))
     ctx.check_device_errors()
+
+
+@pytest.mark.parametrize("row", [0, 1, 2])
+def test_bounds_that_hold_a_nan(W, row):
+    # a finite transform that overflows to inf - inf gives one sphere's bounds,
+    # and those of nodes above it, a NaN: boxes are still decided as the
+    # statistics kernel decides them, over the same leaves (the sphere itself
+    # is where no ray meets it: its hits would lie outside such a box)
+    g = W.SceneGen(2, 3, (32, 32), level=2)
+    s = g.desc.contents.spheres[5]
+    s.radius = 2.0
+    for c, v in enumerate([3e38, -3e38, 0.0, 0.0]):
+        s.object_to_world.m[4 * row + c] = v
+    s.world_to_object.m[3] = 1e6
+    rays = random_rays(20000, 12.0, 5)
+    with W.Context(0) as c:
+        c.upload(g.desc)
+        c.build()
+        assert np.isnan(c.bvh_export()["node_bounds"]).any()
+        c.set_traversal(W.TRAVERSAL_BINARY_FULL_LEAVES)
+        hits = c.collide(rays)
+        want, _ = c.collide(rays, stats=True)
+        c.check_device_errors()
+    assert np.array_equal(hits.view(np.uint32), want.view(np.uint32))

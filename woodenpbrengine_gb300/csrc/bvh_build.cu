@@ -61,6 +61,7 @@ enum : uint32_t {
   kInfoT = 0,      // treelets
   kInfoRoot = 1,   // unified id of the root
   kInfoM = 2,      // nodes of the flattened tree
+  kInfoNaN = 3,    // some primitive's bounds hold a NaN
   kInfoSum = 16,   // summary block copied to the host (k_build_summary)
   kInfoWords = 40
 };
@@ -294,7 +295,8 @@ namespace {
 // ---------------------------------------------------------------------------
 // A3/A4: primitive bounds, centroids, centroid bounds
 // ---------------------------------------------------------------------------
-__global__ void k_prim_bounds(SceneView S, float4* pb_lo, float4* pb_hi, float4* cen, uint32_t* cb_enc) {
+__global__ void k_prim_bounds(SceneView S, float4* pb_lo, float4* pb_hi, float4* cen, uint32_t* cb_enc,
+                              uint32_t* info) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   uint32_t e[6] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u, 0u};
   if (i < S.N) {
@@ -316,6 +318,9 @@ __global__ void k_prim_bounds(SceneView S, float4* pb_lo, float4* pb_hi, float4*
       b = Bounds{vmin(a, bb), vmax(a, bb)};
       b = bunionp(b, c);
     }
+    // (an overflowing or projective sphere transform; unions of other bounds hold none)
+    if (isnan(b.lo.x) || isnan(b.lo.y) || isnan(b.lo.z) || isnan(b.hi.x) || isnan(b.hi.y) || isnan(b.hi.z))
+      info[kInfoNaN] = 1u;
     V3 ce = bcentroid(b);
     pb_lo[i] = make_float4(b.lo.x, b.lo.y, b.lo.z, 0.0f);
     pb_hi[i] = make_float4(b.hi.x, b.hi.y, b.hi.z, 0.0f);
@@ -651,7 +656,7 @@ __global__ void __launch_bounds__(kOrderThreads) k_small_order(uint32_t N, const
 // Every buffer that a build's kernels expect cleared.
 struct BuildInit {
   uint32_t NU, N2, N;
-  uint32_t *visits, *parent, *is_int, *int_kids, *cb_enc, *bar, *depth_max, *split_depth;
+  uint32_t *visits, *parent, *is_int, *int_kids, *cb_enc, *bar, *depth_max, *split_depth, *info;
 };
 __global__ void k_build_init(BuildInit B) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -666,6 +671,7 @@ __global__ void k_build_init(BuildInit B) {
   if (i == 0) {
     *B.depth_max = 0u;
     *B.split_depth = 0u;
+    B.info[kInfoNaN] = 0u;
   }
 }
 
@@ -2798,7 +2804,7 @@ __global__ void k_split_emit(const uint32_t* info, const uint32_t* is_int, const
 // What the host needs once the tree is built, gathered for one copy:
 // treelets, flattened nodes, interior nodes, leaf-split records and depth,
 // tree depth, SAH nodes, the error word, the root's record and bounds.
-constexpr uint32_t kSumWords = 17;
+constexpr uint32_t kSumWords = 18;
 __global__ void k_build_summary(uint32_t* info, const uint32_t* is_int, const uint32_t* int_index,
                                 const Node2* nodes, const uint32_t* split_off, const uint32_t* counters,
                                 const uint32_t* depth_max, const uint32_t* lin_node, const float* lin_bounds,
@@ -2816,6 +2822,7 @@ __global__ void k_build_summary(uint32_t* info, const uint32_t* is_int, const ui
   o[7] = *err;
   for (int k = 0; k < 3; ++k) o[8 + k] = lin_node[k];
   for (int k = 0; k < 6; ++k) o[11 + k] = __float_as_uint(lin_bounds[k]);
+  o[17] = info[kInfoNaN];
 }
 static_assert(kInfoSum + kSumWords <= kInfoWords, "summary block fits the info words");
 
@@ -3023,9 +3030,9 @@ static wpbr_status bvh_build_tree(wpbr_ctx* ctx) {
 
   const unsigned g = div_up(N, kB);
   k_build_init<<<div_up(NU, kB), kB, 0, st>>>(BuildInit{NU, N2, N, B.visits.p, B.parent.p, B.is_int.p, B.int_kids.p,
-                                                       B.cb_enc.p, B.bar.p, B.depth_max.p, B.counters.p + 6});
+                                                       B.cb_enc.p, B.bar.p, B.depth_max.p, B.counters.p + 6, B.dinfo.p});
   // A3/A4
-  k_prim_bounds<<<g, kB, 0, st>>>(S, B.pb_lo.p, B.pb_hi.p, B.centroid.p, B.cb_enc.p);
+  k_prim_bounds<<<g, kB, 0, st>>>(S, B.pb_lo.p, B.pb_hi.p, B.centroid.p, B.cb_enc.p, B.dinfo.p);
   const int passes = full ? 4 : 3;
   if (N <= kOrderMax) {
     // A5, A6 and the treelets in one launch
@@ -3201,6 +3208,7 @@ static wpbr_status bvh_build_tree(wpbr_ctx* ctx) {
   v.stack_cap = kDefaultStackCap;
   v.step_cap = kDefaultStepCap;
   v.n_prims = N;
+  v.nan_bounds = o[17];
   v.n_int = n_int + n_split;
   B.view = v;
   B.built = true;

@@ -96,7 +96,7 @@ __device__ __forceinline__ float prim_test_shared(const SceneView& S, const floa
 // ---- box tests of one node ---------------------------------------------------
 // slab_test's decision for both children with fewer instructions, for rays
 // whose plane distances cannot be NaN (origin and reciprocal direction finite,
-// |origin| <= 2^100, no reciprocal zero). Then, per axis, the smaller product
+// |origin| <= 2^100, no reciprocal zero; no NaN in the tree's bounds). Then, per axis, the smaller product
 // is the one slab_test selects by the direction's sign; slab_test's comparisons
 // amount to max(entries) <= min(exits), because an axis's own entry and exit
 // are in order wherever the scaled exit is positive; scaling the smallest exit
@@ -364,7 +364,7 @@ __global__ void __launch_bounds__(kPersistBlock, Sink::kMinBlocks) k_trace_persi
           const V3 inv{1.0f / d.x, 1.0f / d.y, 1.0f / d.z};
           const int neg[3] = {inv.x < 0.0f, inv.y < 0.0f, inv.z < 0.0f};
           near1 = (neg[0] ? 1u : 0u) | (neg[1] ? 2u : 0u) | (neg[2] ? 4u : 0u);
-          plain = box_pair_ok(o, inv);
+          plain = box_pair_ok(o, inv) && !Bv.nan_bounds;
           rb = RayBox{pack2(o.x, o.x),     pack2(o.y, o.y),     pack2(o.z, o.z),
                       pack2(inv.x, inv.x), pack2(inv.y, inv.y), pack2(inv.z, inv.z)};
           L = entry_limit(tmax);

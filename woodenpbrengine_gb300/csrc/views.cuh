@@ -71,6 +71,7 @@ struct BvhView {
   uint32_t ref_depth;       // depth of the reference's tree (max_depth adds the split levels)
   uint32_t stack_cap;       // stack entries a lane may use (launches clamp it to the kernel's array)
   uint32_t step_cap;        // iterations of a traversal loop before the traversal gives up
+  uint32_t nan_bounds;      // some node's bounds hold a NaN: every box test is slab_test's own
 };
 
 // Bounds of a well-formed traversal: the stack never holds more entries than
