@@ -1387,12 +1387,12 @@ __global__ void __launch_bounds__(kCoopBlock, kCoopPerSM) k_sah_levels(CoopSah C
         if (sk != kNone) {
           uint32_t* d = s_bk + (sk & (kSlots - 1)) * kBucketWords + ib * 7;
           atomicAdd(d, 1u);
-          atomicMin(d + 1, fenc(lo.x));
-          atomicMin(d + 2, fenc(lo.y));
-          atomicMin(d + 3, fenc(lo.z));
-          atomicMax(d + 4, fenc(hi.x));
-          atomicMax(d + 5, fenc(hi.y));
-          atomicMax(d + 6, fenc(hi.z));
+          atomicMin(d + 1, fenc_bits(lo.x));
+          atomicMin(d + 2, fenc_bits(lo.y));
+          atomicMin(d + 3, fenc_bits(lo.z));
+          atomicMax(d + 4, fenc_bits(hi.x));
+          atomicMax(d + 5, fenc_bits(hi.y));
+          atomicMax(d + 6, fenc_bits(hi.z));
         }
       }
       __syncthreads();
@@ -2183,10 +2183,13 @@ __device__ bool sah_pairs(const SahArgs& A, uint32_t base, uint32_t nd, uint32_t
   const uint32_t it1 = __shfl_down_sync(FULL, item, 1);
   const V3 lo1{__shfl_down_sync(FULL, lo.x, 1), __shfl_down_sync(FULL, lo.y, 1), __shfl_down_sync(FULL, lo.z, 1)};
   const V3 hi1{__shfl_down_sync(FULL, hi.x, 1), __shfl_down_sync(FULL, hi.y, 1), __shfl_down_sync(FULL, hi.z, 1)};
+  // (bounds by fenc_bits, as by words that came through shuffles: a NaN stays)
+  auto omin = [](float a, float b) { return fenc_bits(b) < fenc_bits(a) ? b : a; };
+  auto omax = [](float a, float b) { return fenc_bits(b) > fenc_bits(a) ? b : a; };
   auto emin = [](float a, float b) { return fdec(min(fenc(a), fenc(b))); };
   auto emax = [](float a, float b) { return fdec(max(fenc(a), fenc(b))); };
-  const Bounds bb{V3{emin(lo.x, lo1.x), emin(lo.y, lo1.y), emin(lo.z, lo1.z)},
-                  V3{emax(hi.x, hi1.x), emax(hi.y, hi1.y), emax(hi.z, hi1.z)}};
+  const Bounds bb{V3{omin(lo.x, lo1.x), omin(lo.y, lo1.y), omin(lo.z, lo1.z)},
+                  V3{omax(hi.x, hi1.x), omax(hi.y, hi1.y), omax(hi.z, hi1.z)}};
   const V3 c0 = mul(add(lo, hi), 0.5f), c1 = mul(add(lo1, hi1), 0.5f);
   const Bounds cb{V3{emin(c0.x, c1.x), emin(c0.y, c1.y), emin(c0.z, c1.z)},
                   V3{emax(c0.x, c1.x), emax(c0.y, c1.y), emax(c0.z, c1.z)}};

@@ -22,6 +22,12 @@ __device__ __forceinline__ uint32_t fenc(float f) {
   uint32_t u = __float_as_uint(f);
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
+// The same map in integer arithmetic throughout: fenc of a float at hand may be
+// compiled to a floating-point absolute value, which takes a NaN to -0.
+__device__ __forceinline__ uint32_t fenc_bits(float f) {
+  const uint32_t u = __float_as_uint(f);
+  return u ^ ((uint32_t)((int32_t)u >> 31) | 0x80000000u);
+}
 __device__ __forceinline__ float fdec(uint32_t u) {
   return __uint_as_float((u & 0x80000000u) ? (u & 0x7FFFFFFFu) : ~u);
 }
