@@ -341,7 +341,8 @@ constexpr int kFilmPix = 2;                  // pixels (one column) per thread
 constexpr uint64_t kFilmFewBlocks = 608;     // 4 a SM
 constexpr int kFilmPitch = kFilmTile + 4;    // staged columns, two empty ones either side
 
-// mitchell1 at the distance |x| <= 2.5 itself: both branches as one polynomial
+// One dimension of the MitchellFilter of radius 2, B = C = 1/3 (CSFilm.h:20-44),
+// at a distance of t <= 2.5 pixels: both branches as one polynomial
 // (the inner one adds a zero linear term).
 __device__ __forceinline__ float mitchell_at(float t) {
   const float B = (float)(1.0 / 3.0f), C = (float)(1.0 / 3.0f);
@@ -352,7 +353,7 @@ __device__ __forceinline__ float mitchell_at(float t) {
   const float d = outer ? 8.0f * B + 24.0f * C : 6.0f - 2.0f * B;
   return (((((a * t) * t) * t + ((b * t) * t)) + (c * t)) + d) * (1.0f / 6.0f);
 }
-// mitchell1's inner branch, |x| <= 1.
+// Its inner branch, t <= 1.
 __device__ __forceinline__ float mitchell_inner(float t) {
   const float B = (float)(1.0 / 3.0f), C = (float)(1.0 / 3.0f);
   return (((((12.0f - 9.0f * B - 6.0f * C) * t) * t) * t + (((-18.0f + 12.0f * B + 6.0f * C) * t) * t)) +

@@ -458,17 +458,4 @@ WPBR_HD void env_li_compute(const EnvView& e, V3 wi, RGB3* li, float* pdf) {
   }
 }
 
-// ---- film: MitchellFilter r=2, B=C=1/3 (CSFilm.h:20-44) -------------------------
-WPBR_HD float mitchell1(float x) {
-  const float B = (float)(1.0 / 3.0f), C = (float)(1.0 / 3.0f);
-  x = fabs_(2.0f * x);
-  if (x > 1.0f)
-    return ((((((-B - 6.0f * C) * x) * x) * x + (((6.0f * B + 30.0f * C) * x) * x)) + ((-12.0f * B - 48.0f * C) * x)) +
-            (8.0f * B + 24.0f * C)) *
-           (1.0f / 6.0f);
-  return (((((12.0f - 9.0f * B - 6.0f * C) * x) * x) * x + (((-18.0f + 12.0f * B + 6.0f * C) * x) * x)) +
-          (6.0f - 2.0f * B)) *
-         (1.0f / 6.0f);
-}
-
 }  // namespace wpbr
