@@ -435,6 +435,7 @@ __global__ void __launch_bounds__(128, 12) k_sfinish(PassCtx P, SpecCtx C, const
 // layout with scalar sums, 430 us with two-lane ones and unrolled copies. An
 // 8-spp frame: 4.35 -> 3.51 ms.
 constexpr int kSRows = 4;                          // pixel rows of a block
+constexpr unsigned kMaxGridRows = 65535;
 constexpr int kSStage = kSRows + 4;                // staged sample rows
 constexpr int kFilmThreads = kFilmTile * kSRows / 2 * 4;
 constexpr int kSSamples = kSStage * kFilmTile;
@@ -469,9 +470,9 @@ __global__ void __launch_bounds__(kFilmThreads, 3) k_sfilm(uint32_t W, uint32_t 
   float(*s_mx)[kSPad] = reinterpret_cast<float(*)[kSPad]>(sfilm_smem + kSSamples * kSpecN);  // [5]
   float(*s_my)[kSPad] = s_mx + 5;                              // [5]
   const int tid = (int)threadIdx.x;
-  // blocks in one dimension, row by row: a grid's second one ends at 65,535
-  const uint32_t nx = (W + kFilmTile - 1) / kFilmTile;
-  const int bx0 = (int)(blockIdx.x % nx) * kFilmTile, by0 = (int)(blockIdx.x / nx) * kSRows;
+  // (rows of blocks beyond the second grid dimension's 65,535 in the third)
+  const int bx0 = (int)blockIdx.x * kFilmTile, by0 = (int)(blockIdx.z * kMaxGridRows + blockIdx.y) * kSRows;
+  if (by0 >= (int)H) return;
   const int ty0 = by0 / 32 * 32;
   const int tx1 = min(bx0 + 31, (int)W - 1), ty1 = min(ty0 + 31, (int)H - 1);
   const int q = tid % 4, lx = tid / 4 % kFilmTile, ly = tid / (4 * kFilmTile) * 2;
@@ -739,8 +740,9 @@ cudaError_t spectral_film_launch(wpbr_ctx* ctx, uint32_t film_slots, cudaStream_
   cudaError_t e = cudaFuncSetAttribute((const void*)k_sfilm, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)kSFilmSmem);
   if (e != cudaSuccess) return e;
-  const unsigned blocks = div_up(R.W, kFilmTile) * div_up(R.H, kSRows);
-  k_sfilm<<<blocks, kFilmThreads, kSFilmSmem, st>>>(R.W, R.H, R.pfilm.p, R.spec_L.p, R.spec_flags.p, film_slots,
+  const unsigned rows = div_up(R.H, kSRows);
+  const dim3 fg(div_up(R.W, kFilmTile), std::min(rows, kMaxGridRows), div_up(rows, kMaxGridRows));
+  k_sfilm<<<fg, kFilmThreads, kSFilmSmem, st>>>(R.W, R.H, R.pfilm.p, R.spec_L.p, R.spec_flags.p, film_slots,
                                                  R.spec_acc.p, (float4*)R.acc.p, kOnes);
   return cudaGetLastError();
 }
