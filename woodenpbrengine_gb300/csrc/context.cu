@@ -270,7 +270,6 @@ WPBR_API void wpbr_destroy(wpbr_ctx* ctx) {
   R.pstate.release();
   R.Lbuf.release(); R.pfilm.release(); R.pass_dev.release(); R.counters.release(); R.order.release(); R.slices.release();
   R.spec_mats.release(); R.spec_le.release(); R.spec_L.release(); R.spec_flags.release(); R.spec_acc.release();
-  R.film_out.release();
   ctx->io_rays.release(); ctx->io_hits.release(); ctx->io_stats.release();
   ctx->tscr[0].release(); ctx->tscr[1].release();
   for (cudaEvent_t& ev : ctx->io_ev)

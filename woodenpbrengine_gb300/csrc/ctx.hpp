@@ -116,7 +116,7 @@ struct RenderState {
   bool ready = false;
   uint32_t spp = 0, seed = 0, stream = 0;
   uint32_t W = 0, H = 0;
-  DevBuf<float> acc;  // W*H*4 (L rgb, weight)
+  DevBuf<float> acc;  // W*H*4 (L rgb, weight), then W*H*4 that reads copy to the host from
   // fused-path per-pixel state
   DevBuf<uint32_t> hit_prim;
   DevBuf<float4> shadow_rays;   // the pass's queued shadow rays (2 float4 each), at most 2 per pixel
@@ -138,7 +138,6 @@ struct RenderState {
   // Sampled64 mode: material / light spectra, per-pixel sample spectra, film spectra
   DevBuf<float> spec_mats, spec_le, spec_L, spec_acc;
   DevBuf<uint32_t> spec_flags;  // per sample: a bin is not finite
-  DevBuf<float> film_out;   // what film_read and film_tonemap copy to the host
   bool spec_dirty = false;  // Sampled64 passes ran since the last toRGB of the film
   const uint32_t* pass_ptr = nullptr;  // shared pass index (batches); null: pass_dev
   uint32_t trace_grid = 0;             // persistent traversal grid cap (0: full)

@@ -567,7 +567,7 @@ wpbr_status render_setup(wpbr_ctx* ctx, uint32_t spp, uint32_t seed, uint32_t st
   R.W = ctx->cam.W;
   R.H = ctx->cam.H;
   size_t n = (size_t)R.W * R.H;
-  WPBR_CUDA(R.acc.ensure(n * 4));
+  WPBR_CUDA(R.acc.ensure(n * 4 + n * 4));  // the accumulators, then what reads copy to the host
   WPBR_CUDA(R.hit_prim.ensure(n));
   WPBR_CUDA(R.shadow_rays.ensure(n * 4));
   WPBR_CUDA(R.shadow_map.ensure(n * 2));
@@ -820,11 +820,12 @@ wpbr_status render_frame(wpbr_ctx* ctx) {
   const size_t n = (size_t)R.W * R.H;
   const bool spectral = ctx->spectrum == WPBR_SPECTRUM_SAMPLED64;
   uint32_t K = R.pass_ptr ? 1u : group_passes(n, R.spp, spectral);
-  const size_t slot_bytes = spectral ? spectral_slot_bytes(n) : 0;
-  if (K > 1 && (R.slices.n < (K - 1) * slice_bytes(n) || (spectral && R.spec_flags.n < K * n))) {
+  const size_t pass_bytes = slice_bytes(n) + (spectral ? spectral_slot_bytes(n) : 0);
+  if ((K - 1) * pass_bytes > kGroupUnasked &&
+      (R.slices.n < (K - 1) * slice_bytes(n) || (spectral && R.spec_flags.n < K * n))) {
     size_t room = 0, total = 0;
     WPBR_CUDA(cudaMemGetInfo(&room, &total));
-    K = group_passes_within(K, slice_bytes(n) + slot_bytes, room + R.slices.n);  // the old slices go first
+    K = group_passes_within(K, pass_bytes, room + R.slices.n);  // the old slices go first
   }
   if (K > 1) {
     // the group's buffers; a device without room for them renders one pass at
@@ -926,16 +927,15 @@ wpbr_status job_record(wpbr_ctx* ctx, uint32_t x0, uint32_t y0, uint32_t x1, uin
 }
 
 // The accumulators as separate radiance and weight arrays, as the caller
-// receives them. Larger films are split on the device into a buffer that reads
-// alone use (the pass state's memory would do, but a caller may read on one
-// stream while passes still run on another), so the host only receives the
-// copies, into pages touched while the last passes still run: splitting 1920 x
-// 1080 float4s on the host, through a vector of its own, took 3.4 ms, the
-// copies alone take 0.24.
+// receives them. Larger films are split on the device into memory that reads
+// alone use, behind the accumulators (the pass state's would do, but a caller
+// may read on one stream while passes still run on another), so the host only
+// receives the copies, into pages touched while the last passes still run:
+// splitting 1920 x 1080 float4s on the host, through a vector of its own, took
+// 3.4 ms, the copies alone take 0.24.
 //
-// Films of at most kFilmHostSplit pixels, and films that there is no device
-// memory to split, are copied as they are and split on the host: one copy
-// instead of a launch and two. us a read into kept / new arrays, host and
+// Films of at most kFilmHostSplit pixels are copied as they are and split on
+// the host: one copy instead of a launch and two. us a read into kept / new arrays, host and
 // device split: 100 x 100 26.0 / 28.2 on the host; 110 x 111 29.1 / 31.7; 110 x
 // 112 28.5 / 31.6 and 28.8 / 35.5; 128 x 128 33.5 / 37.0 and 29.3 / 37.6;
 // 160 x 160 45.0 / 49.5 and 30.0 / 41.0. (A vector of float4s, which is
@@ -947,9 +947,7 @@ wpbr_status film_read(wpbr_ctx* ctx, float* acc_L, float* acc_w) {
   wpbr_status rs = spectral_resolve(ctx);
   if (rs != WPBR_OK) return rs;
   const uint32_t n = R.W * R.H;
-  cudaError_t e = n > kFilmHostSplit ? R.film_out.ensure(4 * (size_t)n) : cudaErrorMemoryAllocation;
-  if (e == cudaErrorMemoryAllocation) {
-    cudaGetLastError();
+  if (n <= kFilmHostSplit) {
     std::vector<float> a((size_t)n * 4);
     WPBR_CUDA(cudaMemcpyAsync(a.data(), R.acc.p, (size_t)n * 16, cudaMemcpyDeviceToHost, ctx->stream));
     WPBR_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -963,8 +961,7 @@ wpbr_status film_read(wpbr_ctx* ctx, float* acc_L, float* acc_w) {
     }
     return WPBR_OK;
   }
-  WPBR_CUDA(e);
-  float* L = R.film_out.p;
+  float* L = R.acc.p + 4 * (size_t)n;
   float* w = L + 3 * (size_t)n;
   k_film_split<<<div_up(n, 256), 256, 0, ctx->stream>>>(n, (const float4*)R.acc.p, L, w);
   WPBR_CUDA(cudaGetLastError());
@@ -982,8 +979,7 @@ wpbr_status film_tonemap(wpbr_ctx* ctx, uint8_t* out) {
   wpbr_status rs = spectral_resolve(ctx);
   if (rs != WPBR_OK) return rs;
   uint32_t n = R.W * R.H;
-  WPBR_CUDA(R.film_out.ensure(((size_t)n * 3 + 3) / 4));  // as film_read
-  uint8_t* rgb8 = (uint8_t*)R.film_out.p;
+  uint8_t* rgb8 = (uint8_t*)(R.acc.p + 4 * (size_t)n);  // as film_read
   k_tonemap<<<div_up(n, 256), 256, 0, ctx->stream>>>(n, (const float4*)R.acc.p, rgb8);
   WPBR_CUDA(cudaGetLastError());
   touch_pages(out, (size_t)n * 3);
