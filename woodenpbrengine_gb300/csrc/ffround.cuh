@@ -13,8 +13,8 @@
 // available precision", Numer. Math. 18, 1971) with a relative error below
 // 2^-43, and the float result is taken only if every number within 2^-42 of
 // hi + lo rounds to the same float (Ziv's rounding test). The double
-// expression lies within 2^-51 of the exact value, so it then rounds to that
-// float too: the result is the double expression's, bit for bit. Everything
+// expressions lie within 2^-50 of the exact value (tr_rcp, of six roundings,
+// within 2^-50.4), so they then round to that float too: the result is the double expression's, bit for bit. Everything
 // else (about one operand in 10^5, and operands so large, small or special
 // that an error term could leave the float range) takes the double expression
 // itself, out of line.

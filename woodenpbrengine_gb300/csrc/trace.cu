@@ -14,7 +14,9 @@ namespace {
 // benchmark rays on 1.31 M triangles 395 / 359, any-hit segments 390 / 354,
 // rays aimed from outside 385 / 318. At 524,288 it is still 6 to 15 % behind, at
 // 4 M even, and at 8.4 M ahead for rays off the surface (segments 4.11 / 4.40
-// ms, benchmark rays 3.93 / 4.00).
+// ms, benchmark rays 3.93 / 4.00). The line is no higher because the header
+// promises the order from 512k rays on, and a caller's wpbr_set_ray_sort asks
+// for it there.
 constexpr uint64_t kRaySortMin = 1u << 19;
 
 template <bool ANY, bool STATS, int STACK>

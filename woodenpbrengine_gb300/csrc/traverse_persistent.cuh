@@ -706,9 +706,9 @@ inline void launch_traversal_kernel(const SceneView& S, BvhView Bv, const Src& s
 // of 250 and more) the 256-entry kernel of the reference's nodesToVisit[256]
 // (SLBVH.cpp:101); grid_cap limits the persistent grid (0: one full wave of
 // resident blocks), share is the number of launches of this size that run at
-// the same time (the branches of a pass group or a batch). n > 0. The counter must be zero when the kernel starts and
-// is used by batches larger than the grid's first rays only; zero_counter
-// clears it here when it is.
+// the same time (the branches of a pass group or a batch). n > 0. The counter
+// must be zero when the kernel starts and is used by batches larger than the
+// grid's first rays only; zero_counter clears it here when it is.
 //
 // The collide kernels are compiled without the sphere test for scenes that
 // have no spheres: its transform and quadratic beside the traversal's state
