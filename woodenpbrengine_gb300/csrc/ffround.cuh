@@ -13,11 +13,12 @@
 // available precision", Numer. Math. 18, 1971) with a relative error below
 // 2^-43, and the float result is taken only if every number within 2^-42 of
 // hi + lo rounds to the same float (Ziv's rounding test). The double
-// expressions lie within 2^-50 of the exact value (tr_rcp, of six roundings,
-// within 2^-50.4), so they then round to that float too: the result is the double expression's, bit for bit. Everything
-// else (about one operand in 10^5, and operands so large, small or special
-// that an error term could leave the float range) takes the double expression
-// itself, out of line.
+// expressions lie within 2^-50 of the exact value (tr_rcp's, of six roundings,
+// within 2^-50.4; the others within 2^-51), so they then round to that float
+// too: the result is the double expression's, bit for bit. Everything else
+// (about one operand in 10^5, and operands so large, small or special that an
+// error term could leave the float range) takes the double expression itself,
+// out of line.
 //
 // Per pass, before -> after: 1080p full frame, spawn 171 -> 143 us, finish 70
 // -> 57 us; textured spheres at 1080p, shadow rays 144 -> 112 us; 512 x 512
